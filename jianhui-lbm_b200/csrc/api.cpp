@@ -125,7 +125,7 @@ struct lbm_handle {
   // beside the step kernel (ev_fork: the step's start, ev_bc: faces done)
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_bc = nullptr;
-  DevBuf pop[2], table, ref_of, window, rho_given, u_given, rho_prev, u_prev, partials, result;
+  DevBuf pop, table, ref_of, window, rho_given, u_given, rho_prev, u_prev, partials, result;
   // pressure/velocity faces: plan, per-step records (ping-pong like pop),
   // operations, M^-1 for the moment rule, post-rule populations of the state
   BcPlan bc;
@@ -139,9 +139,17 @@ struct lbm_handle {
   bool ct_ok = false;
   bool ct_on = false;  // the int32 table unless chosen (lbm_set_table_mode, lbm_autotune)
   double ct_wide_frac = 1.0;
+  // row form of the pull table, built with every layout of a solve that is
+  // large enough; read instead of the int32 table when few enough nodes are
+  // marked
+  DevBuf rows, rows_marked;
+  int marked = 0;
+  bool rows_on() const { return rows.p != nullptr && rows_pay(marked, geo.count); }
   // field export: device buffers kept between calls
   DevBuf x_rint, x_uint, x_rref, x_uref;
-  int cur = 0;
+  // phase of the populations (kPull / kLocal); with faces also the record of
+  // the state, snap[cur]
+  int cur = kPull;
   long long step = 0;
   bool given_macro = true;  // next step / reduce takes rho, u from rho_given / u_given
   bool uprev_valid = false;
@@ -152,7 +160,7 @@ struct lbm_handle {
   int last_p = -1;
   double fp16_scale = 1.0;
   double last_ms = 0.0;
-  // captured step chains, one per starting buffer
+  // captured step chains, one per starting phase
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   int graph_steps = 0;
   // false when the layout was built on the device and the host copies of the
@@ -212,10 +220,33 @@ lbm_status build_compact_table(lbm_handle* h) {
   return LBM_OK;
 }
 
-// Table bytes the step kernel reads per node.
+// Builds the row form of the table; h->marked is set when the stream has
+// been waited for.
+lbm_status build_rows(lbm_handle* h) {
+  if (!rows_large(h->geo.count, kQ * (long long)store_bytes(h->kind))) return LBM_OK;
+  if (!h->rows.p) {
+    LBM_CUDA_TRY(h->rows.alloc((size_t)9 * h->geo.npad * sizeof(int32_t)));
+    LBM_CUDA_TRY(h->rows_marked.alloc(sizeof(int)));
+  }
+  LBM_CUDA_TRY(cudaMemsetAsync(h->rows_marked.p, 0, sizeof(int), h->stream));
+  LBM_CUDA_TRY(launch_row_table(h->table.as<int32_t>(), h->geo.npad, 0, h->geo.count, h->rows.as<int32_t>(),
+                                h->rows_marked.as<int>(), h->stream));
+  LBM_CUDA_TRY(cudaMemcpyAsync(&h->marked, h->rows_marked.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  return LBM_OK;
+}
+
+// Bytes per node of the pull table in the chosen mode.
 double table_bytes_per_node(const lbm_handle* h) {
   if (!(h->ct_ok && h->ct_on)) return 18.0 * 4.0;
   return 18.0 * 2.0 + 18.0 * 4.0 / 32.0 + h->ct_wide_frac * 18.0 * 4.0;
+}
+
+// Table bytes a step reads per node: those of the row form where the int32
+// mode reads it, by every second step (the others read none).
+double step_table_bytes(const lbm_handle* h) {
+  if (!(h->ct_ok && h->ct_on) && h->rows_on())
+    return 0.5 * (9.0 * 4.0 + 5.0 * 4.0 * h->marked / std::max(h->geo.count, 1));
+  return 0.5 * table_bytes_per_node(h);
 }
 
 lbm_status upload_layout(lbm_handle* h) {
@@ -230,6 +261,9 @@ lbm_status upload_layout(lbm_handle* h) {
     LBM_CUDA_TRY(cudaMemcpyAsync(h->window.p, g.in_window.data(), (size_t)g.count, cudaMemcpyHostToDevice, h->stream));
   }
   h->last_p = g.count > 0 ? g.int_of[g.count] : -1;
+  lbm_status rst = build_rows(h);
+  if (rst != LBM_OK) return rst;
+  LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));  // h->marked
   h->drop_graphs();
   h->cell_idx_valid = false;
   // the compact form is built when it is first chosen (lbm_set_table_mode,
@@ -299,7 +333,7 @@ lbm_status layout(lbm_handle* h, int ordering) {
 lbm_status alloc_device(lbm_handle* h) {
   const size_t npad = (size_t)h->geo.npad;
   const size_t s = store_bytes(h->kind);
-  for (auto& b : h->pop) LBM_CUDA_TRY(b.alloc(kQ * npad * s));
+  LBM_CUDA_TRY(h->pop.alloc(kQ * npad * s));
   LBM_CUDA_TRY(h->table.alloc(18 * npad * sizeof(int32_t)));
   LBM_CUDA_TRY(h->ref_of.alloc(std::max<size_t>(h->geo.count, 1) * sizeof(int32_t)));
   LBM_CUDA_TRY(h->rho_given.alloc(npad * h->mac_bytes()));
@@ -314,11 +348,11 @@ lbm_status alloc_device(lbm_handle* h) {
 lbm_status init_state(lbm_handle* h) {
   double feq[kQ];
   for (int q = 0; q < kQ; q++) feq[q] = feq_ref(q, 1.0, h->prm.u_init, h->lat);
-  LBM_CUDA_TRY(launch_init_uniform(h->kind, h->pop[0].p, h->table.as<int32_t>(), h->geo.count, h->geo.npad,
+  LBM_CUDA_TRY(launch_init_uniform(h->kind, h->pop.p, h->table.as<int32_t>(), h->geo.count, h->geo.npad,
                                    h->fp16_scale, feq, h->stream));
   LBM_CUDA_TRY(launch_fill_macro(h->kind, h->rho_given.p, h->u_given.p, h->geo.count, h->geo.npad, 1.0,
                                  h->prm.u_init, h->stream));
-  h->cur = 0;
+  h->cur = kPull;
   h->step = 0;
   h->given_macro = true;
   h->uprev_valid = false;
@@ -339,8 +373,8 @@ void kernel_force(const lbm_handle* h, double* gx, double* gy, double* gz) {
 
 StepArgs step_args(lbm_handle* h, bool write) {
   StepArgs a{};
-  a.src_pop = h->pop[h->cur].p;
-  a.dst_pop = h->pop[1 - h->cur].p;
+  a.pop = h->pop.p;
+  a.phase = h->cur;
   a.table = h->table.as<int32_t>();
   a.n = h->geo.count;
   a.npad = h->geo.npad;
@@ -360,6 +394,8 @@ StepArgs step_args(lbm_handle* h, bool write) {
     a.ct_off = h->ct_off.as<uint16_t>();
     a.nwarps = h->geo.npad / 32;
   }
+  if (h->rows_on()) a.rows = h->rows.as<int32_t>();
+  a.ahead = prefetch_ahead(n, kQ * (long long)store_bytes(h->kind), a.rows ? 36 : 72);
   a.snap_begin = h->bc.active ? h->bc.snap_begin : n;
   a.nsnap = std::max(n - a.snap_begin, 1);
   a.snap_dst = h->bc.active ? h->snap[1 - h->cur].as<double>() : nullptr;
@@ -367,7 +403,7 @@ StepArgs step_args(lbm_handle* h, bool write) {
 }
 
 // Arguments of the face-node kernel for a step whose step arguments are s and
-// whose source buffers have parity c.
+// whose state has phase c.
 BcArgs bc_args(lbm_handle* h, const StepArgs& s, int c) {
   BcArgs b{};
   b.s = s;
@@ -388,10 +424,11 @@ BcArgs bc_args(lbm_handle* h, const StepArgs& s, int c) {
 }
 
 // One step: the step kernel over [0, n_main) and, with faces, the face kernel
-// over [n_main, n).  The two write disjoint nodes of the new state and of the
-// record (the step kernel the nodes below n_main, the face kernel the rest)
-// and read only the previous step's, so the face kernel runs on the side
-// stream beside the step kernel and the step ends when both have.
+// over [n_main, n).  Each reads and writes only the slots of its own nodes and
+// their part of the new record (the step kernel the nodes below n_main, the
+// face kernel the rest), and the previous step's record, so the face kernel
+// runs on the side stream beside the step kernel and the step ends when both
+// have.
 cudaError_t launch_full_step(lbm_handle* h, const StepArgs& a, int c) {
   if (!h->bc.active) return launch_step(h->kind, a, h->block, h->stream);
   cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
@@ -429,7 +466,7 @@ lbm_status one_step(lbm_handle* h, bool write) {
   return LBM_OK;
 }
 
-constexpr int kGraphSteps = 16;  // even: a replay leaves the buffer parity unchanged
+constexpr int kGraphSteps = 16;  // even: a replay leaves the phase unchanged
 
 lbm_status ensure_graph(lbm_handle* h) {
   if (h->graph[h->cur]) return LBM_OK;
@@ -440,8 +477,7 @@ lbm_status ensure_graph(lbm_handle* h) {
   cudaError_t err = cudaSuccess;
   for (int s = 0; s < kGraphSteps && err == cudaSuccess; s++) {
     StepArgs a = step_args(h, false);
-    a.src_pop = h->pop[c].p;
-    a.dst_pop = h->pop[1 - c].p;
+    a.phase = c;
     a.rho_in = a.u_in = nullptr;
     if (h->bc.active) a.snap_dst = h->snap[1 - c].as<double>();
     err = launch_full_step(h, a, c);
@@ -506,7 +542,8 @@ lbm_status run_steps(lbm_handle* h, int nsteps) {
 // Error + Comput_Perm on the device; optional macro fields (internal order).
 lbm_status reduce_raw(lbm_handle* h, double r[8], double* rho_out_int, double* u_out_int) {
   ReduceArgs a{};
-  a.pop = h->pop[h->cur].p;
+  a.pop = h->pop.p;
+  a.phase = h->cur;
   a.table = h->table.as<int32_t>();
   a.n = h->geo.count;
   a.npad = h->geo.npad;
@@ -681,15 +718,16 @@ lbm_status lbm_create(const lbm_params* p, const uint8_t* mask, int nx, int ny, 
   lbm_status st;
   if ((st = alloc_device(h.get())) != LBM_OK) return st;
   if (on_device) {
-    // the indexing's scratch (5 bytes per cell) lives in the second
-    // population array, which nothing reads before the first step writes it
+    // the indexing's scratch (5 bytes per cell) lives in the population array,
+    // which the initial state overwrites
     SetupScratch scratch;
-    scratch.borrow(h->pop[1].p, h->pop[1].bytes, (long long)nx * ny * nz, h->geo.count);
+    scratch.borrow(h->pop.p, h->pop.bytes, (long long)nx * ny * nz, h->geo.count);
     if ((st = device_index_reference(h->mask.data(), nx, ny, nz, h->geo.count, h->table.as<int32_t>(), h->geo.npad,
                                      0, h->ref_of.as<int32_t>(), scratch, h->stream)) != LBM_OK)
       return st;
     h->ordering = LBM_ORDER_REFERENCE;
     h->last_p = h->geo.count - 1;
+    if ((st = build_rows(h.get())) != LBM_OK) return st;
     LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));  // before the scratch is freed
   } else if ((st = layout(h.get(), ord)) != LBM_OK) {
     return st;
@@ -880,7 +918,7 @@ lbm_status lbm_get_populations(lbm_handle* h, double* f) {
   int n_main;
   const double* bnd_f;
   if ((st = finalize_faces(h, &n_main, &bnd_f)) != LBM_OK) return st;
-  LBM_CUDA_TRY(launch_export_pop(h->kind, h->pop[h->cur].p, h->table.as<int32_t>(), h->ref_of.as<int32_t>(), n,
+  LBM_CUDA_TRY(launch_export_pop(h->kind, h->pop.p, h->cur, h->table.as<int32_t>(), h->ref_of.as<int32_t>(), n,
                                  h->geo.npad, h->fp16_scale, out.as<double>(), h->stream, n_main, bnd_f));
   LBM_CUDA_TRY(d2h_staged(f, out.p, out.bytes, h->stream));
   return LBM_OK;
@@ -898,11 +936,12 @@ lbm_status lbm_set_state(lbm_handle* h, const double* rho, const double* u, cons
   LBM_CUDA_TRY(cudaMemcpyAsync(fin.p, f, fin.bytes, cudaMemcpyHostToDevice, h->stream));
   LBM_CUDA_TRY(cudaMemcpyAsync(rin.p, rho, rin.bytes, cudaMemcpyHostToDevice, h->stream));
   LBM_CUDA_TRY(cudaMemcpyAsync(uin.p, u, uin.bytes, cudaMemcpyHostToDevice, h->stream));
-  LBM_CUDA_TRY(launch_import_pop(h->kind, h->pop[h->cur].p, h->table.as<int32_t>(), h->ref_of.as<int32_t>(), n,
+  LBM_CUDA_TRY(launch_import_pop(h->kind, h->pop.p, h->table.as<int32_t>(), h->ref_of.as<int32_t>(), n,
                                  h->geo.npad, h->fp16_scale, fin.as<double>(), h->stream));
   LBM_CUDA_TRY(launch_import_macro(h->kind, h->rho_given.p, h->u_given.p, h->ref_of.as<int32_t>(), n, h->geo.npad,
                                    rin.as<double>(), uin.as<double>(), h->stream));
   LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+  h->cur = kPull;
   h->given_macro = true;
   h->uprev_valid = false;
   return LBM_OK;
@@ -945,13 +984,13 @@ lbm_status lbm_memory(lbm_handle* h, size_t* device_bytes, double* bytes_per_lu)
   if (!h) return fail(LBM_ERR_ARG, "null handle");
   if (device_bytes) {
     size_t b = 0;
-    for (const DevBuf* d : {&h->pop[0], &h->pop[1], &h->table, &h->ref_of, &h->window, &h->rho_given, &h->u_given,
+    for (const DevBuf* d : {&h->pop, &h->table, &h->ref_of, &h->window, &h->rho_given, &h->u_given,
                             &h->rho_prev, &h->u_prev, &h->partials, &h->result, &h->snap[0], &h->snap[1],
-                            &h->bc_ops, &h->bc_off, &h->bc_mi, &h->bnd_f, &h->ct_base, &h->ct_off})
+                            &h->bc_ops, &h->bc_off, &h->bc_mi, &h->bnd_f, &h->ct_base, &h->ct_off, &h->rows})
       b += d->bytes;
     *device_bytes = b;
   }
-  if (bytes_per_lu) *bytes_per_lu = 2.0 * kQ * (double)store_bytes(h->kind) + table_bytes_per_node(h);
+  if (bytes_per_lu) *bytes_per_lu = 2.0 * kQ * (double)store_bytes(h->kind) + step_table_bytes(h);
   return LBM_OK;
 }
 
@@ -993,7 +1032,7 @@ lbm_status lbm_autotune(lbm_handle* h, int trial_steps, int* ordering_out, int* 
     int n_main;
     const double* bnd_f;
     if ((st = finalize_faces(h, &n_main, &bnd_f)) != LBM_OK) return st;
-    LBM_CUDA_TRY(launch_export_pop(h->kind, h->pop[h->cur].p, h->table.as<int32_t>(), h->ref_of.as<int32_t>(), n,
+    LBM_CUDA_TRY(launch_export_pop(h->kind, h->pop.p, h->cur, h->table.as<int32_t>(), h->ref_of.as<int32_t>(), n,
                                    h->geo.npad, h->fp16_scale, fsave.as<double>(), h->stream, n_main, bnd_f));
   }
   DevBuf rref, uref;
@@ -1013,7 +1052,6 @@ lbm_status lbm_autotune(lbm_handle* h, int trial_steps, int* ordering_out, int* 
                                      rref.as<double>(), uref.as<double>(), h->stream));
   }
   const long long step0 = h->step;
-  const int cur0 = h->cur;
   const bool uprev0 = h->uprev_valid;
   const int orders[4] = {LBM_ORDER_REFERENCE, LBM_ORDER_MORTON, LBM_ORDER_HILBERT, LBM_ORDER_BRICK};
   const int blocks[4] = {128, 256, 512, 64};
@@ -1030,7 +1068,7 @@ lbm_status lbm_autotune(lbm_handle* h, int trial_steps, int* ordering_out, int* 
     h->ct_on = c.ct == 1;
     h->drop_graphs();
     h->given_macro = false;  // timing only; the state is restored below
-    h->cur = 0;
+    h->cur = kPull;
     lbm_status s2;
     if ((s2 = run_steps(h, 2)) != LBM_OK) return s2;  // warm-up
     if ((s2 = run_steps(h, steps)) != LBM_OK) return s2;
@@ -1068,8 +1106,8 @@ lbm_status lbm_autotune(lbm_handle* h, int trial_steps, int* ordering_out, int* 
   h->block = best_b;
   h->ct_on = best_ct && h->ct_ok;
   h->drop_graphs();
-  h->cur = cur0;
-  LBM_CUDA_TRY(launch_import_pop(h->kind, h->pop[h->cur].p, h->table.as<int32_t>(), h->ref_of.as<int32_t>(), n,
+  h->cur = kPull;
+  LBM_CUDA_TRY(launch_import_pop(h->kind, h->pop.p, h->table.as<int32_t>(), h->ref_of.as<int32_t>(), n,
                                  h->geo.npad, h->fp16_scale, fsave.as<double>(), h->stream));
   if (given)
     LBM_CUDA_TRY(launch_import_macro(h->kind, h->rho_given.p, h->u_given.p, h->ref_of.as<int32_t>(), n, h->geo.npad,

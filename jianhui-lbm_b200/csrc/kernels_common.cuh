@@ -1,12 +1,25 @@
 // Device code shared by the kernel translation units.
 //
 // Data layout in HBM (one solver instance):
-//   pop   [19][npad]  post-collision populations of the last step, structure
-//                     of arrays, one row per direction (storage type per Store)
+//   pop   [19][npad]  populations, structure of arrays, one row per direction
+//                     (storage type per Store), updated in place
 //   table [18][npad]  int32 pull sources for q = 1..18: flat index into pop
 //   rho   [npad], u [3][npad]  macro arrays (double for FP64 kinds, float else)
-// A node p of step n pulls f_q(p) = pop[table[q-1][p]] (q >= 1) and
-// pop[0*npad + p] (q = 0), relaxes in moment space and writes pop'[q][p].
+//
+// In-place streaming (the A-A pattern of Bailey et al. 2009, on the sparse
+// table).  The table is a permutation of the 18 npad slots of the moving
+// directions: slot s_q(p) = table[q-1][p] holds the f_q that node p pulls.
+// A state is in one of two phases:
+//   kPull   pop holds the post-collision f*_q(p) at (q, p): the
+//           post-streaming f_q(p) is at s_q(p)
+//   kLocal  the post-streaming f_q(p) is at (opp q, p), the node's own slots
+// A step from kPull reads f_q(p) at s_q(p) and writes f*_opp(q)(p) into that
+// same slot.  By the table's definition s_q(p) is (q, p - e_q), or (opp q, p)
+// behind a wall, so what node m = p - e_q finds in its own slot (q, m) is
+// f*_opp(q)(m + e_q), its post-streaming f_opp(q): a kLocal state.  A step
+// from kLocal reads (opp q, p) and writes f*_q(p) to (q, p): a kPull state.
+// Every slot is read and written by the one thread of its node, so a step
+// needs one array; every second step reads no table and gathers nothing.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -46,8 +59,8 @@ struct Traits<Store::F16> {
   static constexpr bool kDev = true;
 };
 
-// Read-only (non-coherent) loads: the source population array and the table
-// are never written during a launch.
+// Read-only (non-coherent) loads, for the table and for populations that the
+// launch does not write.
 __device__ __forceinline__ double ldg_(const double* p) { return __ldg(p); }
 __device__ __forceinline__ float ldg_(const float* p) { return __ldg(p); }
 __device__ __forceinline__ float ldg_(const __half* p) {
@@ -60,6 +73,62 @@ __device__ __forceinline__ typename Traits<K>::A load_pop(const typename Traits<
     return ldg_(p) * inv_scale;
   else
     return ldg_(p);
+}
+// Load of a population in a launch that updates the array in place.
+template <Store K>
+__device__ __forceinline__ typename Traits<K>::A load_pop_rw(const typename Traits<K>::T* p, float inv_scale) {
+  if constexpr (K == Store::F16)
+    return __half2float(*p) * inv_scale;
+  else
+    return *p;
+}
+// The 18 slots a thread reads, kept in shared memory until it stores into
+// them: held in registers across the collision they would cost the step a
+// resident block or spills.  Written and read by the same thread only, so no
+// barrier; 16 bytes per lane and access.
+template <int BS>
+struct SlotKeep {
+  int4 a[4][BS];
+  int2 b[BS];
+};
+template <int BS, typename F>
+__device__ __forceinline__ void keep_slots(SlotKeep<BS>& k, int t, F&& slot) {
+#pragma unroll
+  for (int i = 0; i < 4; i++) k.a[i][t] = make_int4(slot(4 * i + 1), slot(4 * i + 2), slot(4 * i + 3), slot(4 * i + 4));
+  k.b[t] = make_int2(slot(17), slot(18));
+}
+template <int BS, typename F>
+__device__ __forceinline__ void for_kept_slots(const SlotKeep<BS>& k, int t, F&& use) {
+  asm volatile("" ::: "memory");  // else the compiler carries the stored values in registers
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int4 v = k.a[i][t];
+    use(4 * i + 1, v.x);
+    use(4 * i + 2, v.y);
+    use(4 * i + 3, v.z);
+    use(4 * i + 4, v.w);
+  }
+  const int2 w = k.b[t];
+  use(17, w.x);
+  use(18, w.y);
+}
+// Prefetches into L2 the population rows, and the table rows if any, of the BS
+// nodes `ahead` nodes after the block's: one 128-byte line per thread.
+template <int BS, int TABLE_ROWS, typename T>
+__device__ __forceinline__ void prefetch_block(const T* pop, const int32_t* table, int npad, int ahead) {
+  const int p = blockIdx.x * BS + ahead;
+  if (ahead == 0 || p + BS > npad) return;
+  constexpr int kPopLines = BS * (int)sizeof(T) / 128, kTableLines = BS * 4 / 128;
+  for (int i = threadIdx.x; i < kQ * kPopLines + TABLE_ROWS * kTableLines; i += BS) {
+    const int j = i - kQ * kPopLines;
+    const char* line = j < 0 ? reinterpret_cast<const char*>(pop + (size_t)(i / kPopLines) * npad + p) + (i % kPopLines) * 128
+                             : reinterpret_cast<const char*>(table + (size_t)(j / kTableLines) * npad + p) + (j % kTableLines) * 128;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
+  }
+}
+// Slot of the post-streaming f_q(p), q >= 1, of a state in either phase.
+__device__ __forceinline__ int32_t state_slot(int phase, const int32_t* __restrict__ table, int npad, int p, int q) {
+  return phase == kLocal ? opp(q) * npad + p : __ldg(table + (size_t)(q - 1) * npad + p);
 }
 template <Store K>
 __device__ __forceinline__ void store_pop(typename Traits<K>::T* p, typename Traits<K>::A v, float scale) {
@@ -361,7 +430,7 @@ __global__ void __launch_bounds__(kReduceThreads) reduce_kernel(ReduceArgs a) {
         f[0] = load_pop<K>(pop + p, inv_scale);
 #pragma unroll
         for (int q = 1; q < kQ; q++)
-          f[q] = load_pop<K>(pop + __ldg(a.table + (size_t)(q - 1) * a.npad + p), inv_scale);
+          f[q] = load_pop<K>(pop + state_slot(a.phase, a.table, a.npad, p, q), inv_scale);
       }
       if constexpr (K == Store::F64) {
         if (a.lat.on)
@@ -414,7 +483,8 @@ __global__ void __launch_bounds__(kReduceThreads) reduce_kernel(ReduceArgs a) {
 // Reference-layout export: out[ref_of[p]*19 + q] = f_q(p) (post-streaming, full f).
 // Face nodes [n_main, n) take their populations from bnd_f when it is set.
 template <Store K>
-__global__ void export_pop_kernel(const typename Traits<K>::T* __restrict__ pop, const int32_t* __restrict__ table,
+__global__ void export_pop_kernel(const typename Traits<K>::T* __restrict__ pop, int phase,
+                                  const int32_t* __restrict__ table,
                                   const int32_t* __restrict__ ref_of, int n, int npad, float inv_scale,
                                   double* __restrict__ out, int n_main, const double* __restrict__ bnd_f) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -429,7 +499,7 @@ __global__ void export_pop_kernel(const typename Traits<K>::T* __restrict__ pop,
   row[0] = to_full<K>(load_pop<K>(pop + p, inv_scale), 0);
 #pragma unroll
   for (int q = 1; q < kQ; q++)
-    row[q] = to_full<K>(load_pop<K>(pop + table[(size_t)(q - 1) * npad + p], inv_scale), q);
+    row[q] = to_full<K>(load_pop<K>(pop + state_slot(phase, table, npad, p, q), inv_scale), q);
 }
 
 // Inverse of the pull: pop[table(q,p)] = f_q(p), so that the next step pulls
@@ -468,11 +538,11 @@ cudaError_t reduce_dispatch(const ReduceArgs& a, cudaStream_t st) {
 }
 
 template <Store K>
-cudaError_t export_dispatch(const void* pop, const int32_t* table, const int32_t* ref_of, int n, int npad,
+cudaError_t export_dispatch(const void* pop, int phase, const int32_t* table, const int32_t* ref_of, int n, int npad,
                             double fp16_scale, double* out, cudaStream_t st, int n_main = 0,
                             const double* bnd_f = nullptr) {
   if (n == 0) return cudaSuccess;
-  export_pop_kernel<K><<<(n + 255) / 256, 256, 0, st>>>(static_cast<const typename Traits<K>::T*>(pop), table,
+  export_pop_kernel<K><<<(n + 255) / 256, 256, 0, st>>>(static_cast<const typename Traits<K>::T*>(pop), phase, table,
                                                         ref_of, n, npad, (float)(1.0 / fp16_scale), out, n_main,
                                                         bnd_f);
   return cudaGetLastError();

@@ -229,10 +229,17 @@ lbm_status fail(lbm_status s, const std::string& msg);
 // Storage kinds of the population arrays.
 enum class Store { F64 = 0, F32 = 1, F16 = 2, F64D = 3 };
 
+// Phase of an in-place population array (kernels_common.cuh): where the
+// post-streaming f_q(p) of the state lies, and where a step leaves the next
+// state's.
+enum Phase { kPull = 0, kLocal = 1 };
+
 struct StepArgs {
-  const void* src_pop;   // [19][npad] post-collision of the previous step
-  void* dst_pop;         // [19][npad] this step's post-collision
+  void* pop;             // [19][npad] populations, updated in place
+  int phase;             // Phase of the state the step starts from
   const int32_t* table;  // [18][npad]
+  const int32_t* rows;   // [9][npad] row form of the table (row_table.cuh), or null
+  int ahead;             // nodes ahead that a block prefetches into L2, 0 = none
   int n;                 // fluid nodes
   int npad;
   // macro input for a step that must use given rho/u (first step after init
@@ -274,6 +281,35 @@ cudaError_t launch_step(Store kind, const StepArgs& a, int block, cudaStream_t s
 cudaError_t launch_compact_table(const int32_t* table, int n, int npad, int32_t* ct_base, uint16_t* ct_off,
                                  unsigned long long* wide, cudaStream_t st);
 
+// Row form of the table entries of nodes [begin, begin + n) of a table of row
+// stride `stride`, at rows + i * stride + begin; adds the marked nodes to
+// *marked (device) when it is not null.
+cudaError_t launch_row_table(const int32_t* table, int stride, int begin, int n, int32_t* rows, int* marked,
+                             cudaStream_t st);
+// Whether the row form is the better one to read, for n nodes with pop_bytes
+// of populations per node (rows_large: whether to build it), `marked` of
+// them marked (rows_pay: whether to read it).
+//  * It reads 36 bytes per node against 72, and each marked node up to five
+//    table entries in 32-byte sectors of their own: the two meet where 160
+//    bytes x the marked share are 36, at 0.22.  Reference order marks 2 / nx
+//    of the nodes, the curve orders most of them.
+//  * Its arithmetic costs more than the bytes it saves while the solve lives
+//    in the 126 MB L2 with either form: FP32 steps of cubes at porosity 0.35
+//    took (int32 | rows) 4.28 | 4.62 us at 64^3, 9.12 | 9.51 at 96^3 and
+//    12.8 | 13.4 at 112^3 (73 MB with the int32 table), 21.1 | 19.4 at 128^3
+//    (109 MB); the line is drawn between the last two.
+constexpr bool rows_large(long long n, long long pop_bytes) { return n * (pop_bytes + 72) > (90LL << 20); }
+constexpr bool rows_pay(long long marked, long long n) { return marked * 8 <= n; }
+// Nodes ahead of its own that a block prefetches into L2 (half a wave of
+// resident threads), or 0 for a solve that stays in L2.  A step waits on two
+// loads in a row, table then populations; asked for half a wave early, both
+// come from L2.  256^3, porosity 0.35, rows: 184 -> 169 us per FP32 step,
+// 347 -> 319 in 64-bit deviation storage; at 128^3, in L2, 19.4 -> 20.3.
+// (A whole wave ahead 174, two waves 192 us: the lines are evicted again.)
+constexpr int prefetch_ahead(long long n, long long pop_bytes, long long table_bytes) {
+  return n * (pop_bytes + table_bytes) > (120LL << 20) ? 148 * 640 : 0;
+}
+
 constexpr int kSnapRows = kQ + 4;  // per-step record of a node: f_0..f_18, rho, ux, uy, uz
 
 // Boundary kernel: the face nodes [n_main, n) of one step (pull, rules, macro,
@@ -292,7 +328,8 @@ struct BcArgs {
 cudaError_t launch_boundary(Store kind, const BcArgs& a, cudaStream_t st);
 
 struct ReduceArgs {
-  const void* pop;        // [19][npad] post-collision of the last step
+  const void* pop;        // [19][npad] populations of the state
+  int phase;              // its Phase
   const int32_t* table;
   int n, npad;
   const void* rho_in;     // when the state is "given" (no step since set): use these
@@ -315,9 +352,10 @@ cudaError_t launch_reduce(Store kind, const ReduceArgs& a, cudaStream_t st);
 int reduce_blocks(int n);
 
 // f[(count+1)*19] reference AoS <-> device storage
-cudaError_t launch_export_pop(Store kind, const void* pop, const int32_t* table, const int32_t* ref_of,
+cudaError_t launch_export_pop(Store kind, const void* pop, int phase, const int32_t* table, const int32_t* ref_of,
                               int n, int npad, double fp16_scale, double* out, cudaStream_t st,
                               int n_main = 0, const double* bnd_f = nullptr);
+// (the imported state is a kPull state)
 cudaError_t launch_import_pop(Store kind, void* pop, const int32_t* table, const int32_t* ref_of, int n,
                               int npad, double fp16_scale, const double* in, cudaStream_t st);
 // rho/u reference-layout doubles -> device macro arrays of the storage's type
@@ -329,8 +367,8 @@ cudaError_t set_mi_constant(const double* mi361, cudaStream_t st);
 // True when M^-1 has the zero / power-of-two pattern the bit-exact FP64
 // kernel was compiled for (mi_pattern.h, generated from mrt.cpp).
 bool mi_pattern_matches(const double* mi361);
-// uniform post-streaming state f_q = feq[q] at every node, written through
-// the inverse pull so the next step pulls exactly feq
+// uniform post-streaming state f_q = feq[q] at every node, a kPull state
+// written through the inverse pull so the next step pulls exactly feq
 cudaError_t launch_init_uniform(Store kind, void* pop, const int32_t* table, int n, int npad, double fp16_scale,
                                 const double* feq19, cudaStream_t st);
 cudaError_t launch_fill_macro(Store kind, void* rho, void* u, int n, int npad, double rho0, const double* u3,

@@ -5,6 +5,7 @@
 // millisecond after its 16.8 MB mask is uploaded.
 #include <cub/device/device_scan.cuh>
 
+#include "row_table.cuh"
 #include "setup.h"
 
 namespace lbm {
@@ -44,6 +45,42 @@ __global__ void pull_table_kernel(const int32_t* __restrict__ coor_x, const int3
     const int m = cell_id[ip + nx * (jp + ny * kp)];
     const long long s = m >= 0 ? (long long)q * stride + begin + m : (long long)opp(q) * stride + begin + p;
     table[(size_t)(q - 1) * stride + begin + p] = (int32_t)s;
+  }
+}
+
+__global__ void __launch_bounds__(256) row_table_kernel(const int32_t* __restrict__ table, int stride, int begin, int n,
+                                                        int32_t* __restrict__ rows, int* __restrict__ marked) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  const int p = begin + i;
+  bool mark = false;
+  if (i < n) {
+    int32_t m[kQ];
+    uint32_t bits = 0;
+#pragma unroll
+    for (int q = 1; q < kQ; q++) {
+      m[q] = table[(size_t)(q - 1) * stride + p] - q * stride;
+      if ((uint32_t)m[q] < (uint32_t)stride) bits |= 1u << (q - 1);
+    }
+    auto fluid = [&](int q) { return (int)((bits >> (q - 1)) & 1u); };
+    if (fluid(1) && m[1] != p - 1) bits |= kRowLo;
+    if (fluid(2) && m[2] != p + 1) bits |= kRowHi;
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      const int ql = row_dir(r, 0), qm = row_dir(r, 1), qh = row_dir(r, 2);
+      const int fl = fluid(ql), fm = fluid(qm), fh = fluid(qh);
+      const int32_t base = fm ? m[qm] - fl : fl ? m[ql] : fh ? m[qh] : p;
+      if (fl && m[ql] != base) bits |= kRowLo;
+      if (fh && m[qh] != base + fl + fm) bits |= kRowHi;
+      rows[(size_t)r * stride + p] = base;
+    }
+#pragma unroll
+    for (int q = 11; q <= 14; q++) rows[(size_t)(q - 7) * stride + p] = fluid(q) ? m[q] : p;
+    rows[(size_t)8 * stride + p] = (int32_t)bits;
+    mark = (bits & (kRowLo | kRowHi)) != 0;
+  }
+  if (marked != nullptr) {
+    const int c = __popc(__ballot_sync(0xffffffffu, mark));
+    if ((threadIdx.x & 31) == 0 && c > 0) atomicAdd(marked, c);
   }
 }
 
@@ -154,6 +191,12 @@ lbm_status device_index_reference(const uint8_t* host_mask, int nx, int ny, int 
   }
   LBM_CUDA_TRY(cudaGetLastError());
   return LBM_OK;
+}
+
+cudaError_t launch_row_table(const int32_t* table, int stride, int begin, int n, int32_t* rows, int* marked,
+                             cudaStream_t st) {
+  if (n > 0) row_table_kernel<<<(n + 255) / 256, 256, 0, st>>>(table, stride, begin, n, rows, marked);
+  return cudaGetLastError();
 }
 
 lbm_status device_ref_coor(int nx, int ny, int nz, int count, const SetupScratch& s, int32_t* d_out,

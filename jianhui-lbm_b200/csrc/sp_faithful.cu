@@ -31,6 +31,7 @@
 #include <utility>
 
 #include "bc_kernels.cuh"
+#include "row_table.cuh"
 #include "mi_pattern.h"  // generated at build time from mrt.cpp's M^-1
 
 namespace lbm {
@@ -318,9 +319,10 @@ __device__ __forceinline__ double mi_row(const double (&m)[kQ], std::integer_seq
   return s;
 }
 
-template <bool GX, bool LAT, int... K>
+// put(Q, f*_Q) stores a post-collision population.
+template <bool GX, bool LAT, typename Put, int... K>
 __device__ __forceinline__ void collide_moments_(double (&m)[kQ], double rho, double ux, double uy, double uz,
-                                                 const StepArgs& a, int p, std::integer_sequence<int, K...>) {
+                                                 const StepArgs& a, Put&& put, std::integer_sequence<int, K...>) {
   {
     double feq[kQ];
     equilibrium_<LAT>(rho, ux, uy, uz, a.lat, feq, QSeq{});
@@ -331,27 +333,53 @@ __device__ __forceinline__ void collide_moments_(double (&m)[kQ], double rho, do
     guo_force_<GX, LAT>(ux, uy, uz, a.gx, a.gy, a.gz, a.lat, guo, QSeq{});
     (relax_force<LAT, K>(m[K], guo, a.s_v, a.s_o, a.lat.dt), ...);
   }
-  double* __restrict__ dst = static_cast<double*>(a.dst_pop) + p;
-  const size_t np = (size_t)a.npad;
-  ((dst[(size_t)K * np] = mi_row<K>(m, QSeq{})), ...);
+  (put(std::integral_constant<int, K>{}, mi_row<K>(m, QSeq{})), ...);
 }
 
 // Relaxation in moment space and back-transform for one node whose moments
 // m = M f (accumulated by the caller) and macro values are known; writes the
-// 19 post-collision populations of node p.
-template <bool GX, bool LAT = false>
+// 19 post-collision populations of node p: into its own slots after a step
+// from a kLocal state, else into the slots it read, slot(q) being the one of
+// f_q, which takes f*_opp(q).
+template <bool GX, bool LAT, bool LOCAL, typename Slot>
 __device__ __forceinline__ void collide_moments(double (&m)[kQ], double rho, double ux, double uy, double uz,
-                                                const StepArgs& a, int p) {
-  collide_moments_<GX, LAT>(m, rho, ux, uy, uz, a, p, QSeq{});
+                                                const StepArgs& a, int p, Slot&& slot) {
+  double* pop = static_cast<double*>(a.pop);
+  asm volatile("" ::: "memory");  // the slots are read again from where they were kept
+  collide_moments_<GX, LAT>(
+      m, rho, ux, uy, uz, a,
+      [&](auto q, double v) {
+        constexpr int Q = decltype(q)::value;
+        if constexpr (Q == 0)
+          pop[p] = v;
+        else if constexpr (LOCAL)
+          pop[(size_t)Q * a.npad + p] = v;
+        else
+          pop[slot(opp(Q))] = v;
+      },
+      QSeq{});
 }
 
 }  // namespace
 
-__device__ __forceinline__ void pull_f64(const StepArgs& a, int p, double (&f)[kQ]) {
-  const double* __restrict__ src = static_cast<const double*>(a.src_pop);
-  f[0] = __ldg(src + p);
+// Post-streaming populations of node p; got(q, slot) sees the slots they were
+// read from.
+template <bool LOCAL, bool ROWS, typename Got>
+__device__ __forceinline__ void pull_f64(const StepArgs& a, int p, double (&f)[kQ], Got&& got) {
+  const double* pop = static_cast<const double*>(a.pop);
+  f[0] = pop[p];
+  int32_t s[kQ];
+  if constexpr (ROWS) row_slots(a.rows, a.table, a.npad, p, s);
 #pragma unroll
-  for (int q = 1; q < kQ; q++) f[q] = __ldg(src + __ldg(a.table + (size_t)(q - 1) * a.npad + p));
+  for (int q = 1; q < kQ; q++) {
+    if constexpr (!ROWS) s[q] = LOCAL ? opp(q) * a.npad + p : __ldg(a.table + (size_t)(q - 1) * a.npad + p);
+    f[q] = pop[s[q]];
+    got(q, s[q]);
+  }
+}
+template <bool LOCAL>
+__device__ __forceinline__ void pull_f64(const StepArgs& a, int p, double (&f)[kQ]) {
+  pull_f64<LOCAL, false>(a, p, f, [](int, int32_t) {});
 }
 
 __device__ __forceinline__ void macro_in_out(const StepArgs& a, int p, bool given, bool write, const double (&f)[kQ],
@@ -388,15 +416,22 @@ constexpr int f64_min_blocks(int bs) { return bs == 64 ? 12 : 512 / bs; }
 // from the accumulated moments; with a self-defined lattice (LAT) j sums the
 // products e_a lat_c f_q, each rounded, in direction order, which the kernel
 // accumulates beside the moments.
-template <int BS, bool GIVEN, bool WRITE, bool GX, bool LAT>
+template <int BS, bool GIVEN, bool WRITE, bool GX, bool LAT, bool LOCAL, bool ROWS>
 __global__ void __launch_bounds__(BS, f64_min_blocks(BS)) step_f64_faithful(StepArgs a) {
   const int p = blockIdx.x * BS + threadIdx.x;
+  prefetch_block<BS, ROWS ? 9 : LOCAL ? 0 : 18>(static_cast<const double*>(a.pop), ROWS ? a.rows : a.table, a.npad,
+                                                a.ahead);
   if (p >= a.n_main) return;
+  // the slots of a kPull state's gathers, for the stores after the collision
+  // (each read by the thread that wrote it)
+  __shared__ int32_t keep[LOCAL ? 1 : kQ - 1][LOCAL ? 1 : BS];
   double m[kQ];
   double jx = 0.0, jy = 0.0, jz = 0.0;
   {
     double f[kQ];
-    pull_f64(a, p, f);
+    pull_f64<LOCAL, ROWS>(a, p, f, [&](int q, int32_t s) {
+      if constexpr (!LOCAL) keep[q - 1][threadIdx.x] = s;
+    });
     moments_by_column(m, f, QSeq{});
     if constexpr (LAT && !GIVEN) lattice_momentum(f, a.lat.c, jx, jy, jz);
   }
@@ -427,26 +462,26 @@ __global__ void __launch_bounds__(BS, f64_min_blocks(BS)) step_f64_faithful(Step
     u[2 * a.npad + p] = uz;
   }
   if (a.snap_dst != nullptr && p >= a.snap_begin) {
-    // nodes read by a face rule record their pulled state (pulled again:
-    // the source array is read-only during the launch)
+    // nodes read by a face rule record their pulled state (pulled again: only
+    // this thread writes these slots, further down)
     double f[kQ];
-    pull_f64(a, p, f);
+    pull_f64<LOCAL>(a, p, f);
     snap_write(a.snap_dst, a.nsnap, p - a.snap_begin, f, rho, ux, uy, uz);
   }
-  collide_moments<GX, LAT>(m, rho, ux, uy, uz, a, p);
+  collide_moments<GX, LAT, LOCAL>(m, rho, ux, uy, uz, a, p, [&](int q) { return keep[q - 1][threadIdx.x]; });
 }
 
 // Face nodes: pull, the boundary rules, macro step, record, collision.  With
 // a.bnd_f set: only the populations after the rules (current state).  LAT:
 // a self-defined lattice (the rules' equilibria, the macro step and the
 // collision on it).
-template <bool GIVEN, bool FINAL, bool LAT>
+template <bool GIVEN, bool FINAL, bool LAT, bool LOCAL>
 __global__ void __launch_bounds__(128) bc_f64_faithful(BcArgs a) {
   const int b = blockIdx.x * 128 + threadIdx.x;
   const int p = a.s.n_main + b;
   if (p >= a.s.n) return;
   double f[kQ];
-  pull_f64(a.s, p, f);
+  pull_f64<LOCAL>(a.s, p, f);
   if (!GIVEN) bc_apply(a, b, f, a.s.lat);
   if (FINAL) {
     const size_t nb = (size_t)(a.s.n - a.s.n_main);
@@ -459,27 +494,31 @@ __global__ void __launch_bounds__(128) bc_f64_faithful(BcArgs a) {
   snap_write(a.s.snap_dst, a.s.nsnap, p - a.s.snap_begin, f, rho, ux, uy, uz);
   double m[kQ];
   moments_by_column(m, f, QSeq{});
-  collide_moments<false, LAT>(m, rho, ux, uy, uz, a.s, p);
+  collide_moments<false, LAT, LOCAL>(m, rho, ux, uy, uz, a.s, p, [&](int q) {
+    return __ldg(a.s.table + (size_t)(q - 1) * a.s.npad + p);
+  });
 }
 
-template <bool LAT>
+template <bool LAT, bool LOCAL>
 static void launch_bc_f64(const BcArgs& a, int grid, cudaStream_t st) {
   if (a.bnd_f)
-    bc_f64_faithful<false, true, LAT><<<grid, 128, 0, st>>>(a);
+    bc_f64_faithful<false, true, LAT, LOCAL><<<grid, 128, 0, st>>>(a);
   else if (a.s.rho_in != nullptr)
-    bc_f64_faithful<true, false, LAT><<<grid, 128, 0, st>>>(a);
+    bc_f64_faithful<true, false, LAT, false><<<grid, 128, 0, st>>>(a);  // a given state is a kPull state
   else
-    bc_f64_faithful<false, false, LAT><<<grid, 128, 0, st>>>(a);
+    bc_f64_faithful<false, false, LAT, LOCAL><<<grid, 128, 0, st>>>(a);
 }
 
 cudaError_t launch_boundary_f64(const BcArgs& a, cudaStream_t st) {
   const int nb = a.s.n - a.s.n_main;
   if (nb <= 0) return cudaSuccess;
   const int grid = (nb + 127) / 128;
+  const bool local = a.s.phase == kLocal;
+  if (local && a.s.rho_in != nullptr) return cudaErrorInvalidValue;
   if (a.s.lat.on)
-    launch_bc_f64<true>(a, grid, st);
+    local ? launch_bc_f64<true, true>(a, grid, st) : launch_bc_f64<true, false>(a, grid, st);
   else
-    launch_bc_f64<false>(a, grid, st);
+    local ? launch_bc_f64<false, true>(a, grid, st) : launch_bc_f64<false, false>(a, grid, st);
   return cudaGetLastError();
 }
 
@@ -498,14 +537,23 @@ static cudaError_t launch_f64_bs(const StepArgs& a, cudaStream_t st) {
   const int grid = (a.n_main + BS - 1) / BS;
   if (grid == 0) return cudaSuccess;
   const bool given = a.rho_in != nullptr, write = a.rho_out != nullptr;
-  if (given && write)
-    step_f64_faithful<BS, true, true, GX, LAT><<<grid, BS, 0, st>>>(a);
-  else if (given)
-    step_f64_faithful<BS, true, false, GX, LAT><<<grid, BS, 0, st>>>(a);
-  else if (write)
-    step_f64_faithful<BS, false, true, GX, LAT><<<grid, BS, 0, st>>>(a);
-  else
-    step_f64_faithful<BS, false, false, GX, LAT><<<grid, BS, 0, st>>>(a);
+  if (a.phase == kLocal) {
+    if (given) return cudaErrorInvalidValue;  // a given state is a kPull state
+    if (write)
+      step_f64_faithful<BS, false, true, GX, LAT, true, false><<<grid, BS, 0, st>>>(a);
+    else
+      step_f64_faithful<BS, false, false, GX, LAT, true, false><<<grid, BS, 0, st>>>(a);
+  } else if (given && write) {
+    step_f64_faithful<BS, true, true, GX, LAT, false, false><<<grid, BS, 0, st>>>(a);
+  } else if (given) {
+    step_f64_faithful<BS, true, false, GX, LAT, false, false><<<grid, BS, 0, st>>>(a);
+  } else if (write) {
+    a.rows ? step_f64_faithful<BS, false, true, GX, LAT, false, true><<<grid, BS, 0, st>>>(a)
+           : step_f64_faithful<BS, false, true, GX, LAT, false, false><<<grid, BS, 0, st>>>(a);
+  } else {
+    a.rows ? step_f64_faithful<BS, false, false, GX, LAT, false, true><<<grid, BS, 0, st>>>(a)
+           : step_f64_faithful<BS, false, false, GX, LAT, false, false><<<grid, BS, 0, st>>>(a);
+  }
   return cudaGetLastError();
 }
 
@@ -529,9 +577,9 @@ cudaError_t launch_step_f64(const StepArgs& a, int block, cudaStream_t st) {
 }
 
 cudaError_t reduce_f64(const ReduceArgs& a, cudaStream_t st) { return reduce_dispatch<Store::F64>(a, st); }
-cudaError_t export_f64(const void* pop, const int32_t* table, const int32_t* ref_of, int n, int npad, double* out,
-                       cudaStream_t st, int n_main, const double* bnd_f) {
-  return export_dispatch<Store::F64>(pop, table, ref_of, n, npad, 1.0, out, st, n_main, bnd_f);
+cudaError_t export_f64(const void* pop, int phase, const int32_t* table, const int32_t* ref_of, int n, int npad,
+                       double* out, cudaStream_t st, int n_main, const double* bnd_f) {
+  return export_dispatch<Store::F64>(pop, phase, table, ref_of, n, npad, 1.0, out, st, n_main, bnd_f);
 }
 cudaError_t import_f64(void* pop, const int32_t* table, const int32_t* ref_of, int n, int npad, const double* in,
                        cudaStream_t st) {

@@ -1,18 +1,19 @@
 // Single-phase fused collide + pull-stream kernels in deviation storage
 // (FP32, FP16, FP64-fast) and the dispatch of every single-phase kernel.
 //
-// One thread owns one fluid node.  Per node and step it moves, from/to HBM:
-//   18 x int32 table entries (coalesced), 19 pulled populations (gathered
-//   through the table; neighbours are close in the node order), 19
-//   post-collision populations (coalesced stores)
-// = 2*19*s + 18*4 bytes, s = bytes per stored population.
+// One thread owns one fluid node and updates its 19 slots in place
+// (kernels_common.cuh).  Per node a step moves, from/to HBM, 19 populations
+// in and 19 out (2*19*s bytes, s = bytes per stored population); a step from
+// a kPull state gathers and scatters them through 18 int32 table entries
+// (72 bytes more), the step after it works on the node's own slots.
 #include "bc_kernels.cuh"
+#include "row_table.cuh"
 
 namespace lbm {
 
 cudaError_t launch_step_f64(const StepArgs& a, int block, cudaStream_t st);
 cudaError_t reduce_f64(const ReduceArgs& a, cudaStream_t st);
-cudaError_t export_f64(const void*, const int32_t*, const int32_t*, int, int, double*, cudaStream_t, int,
+cudaError_t export_f64(const void*, int, const int32_t*, const int32_t*, int, int, double*, cudaStream_t, int,
                        const double*);
 cudaError_t launch_boundary_f64(const BcArgs& a, cudaStream_t st);
 cudaError_t import_f64(void*, const int32_t*, const int32_t*, int, int, const double*, cudaStream_t);
@@ -63,24 +64,30 @@ cudaError_t launch_compact_table(const int32_t* table, int n, int npad, int32_t*
   return cudaGetLastError();
 }
 
-// Resident blocks per SM asked of the register allocator: the FP32 step at
-// 256 threads fits 5 blocks in 48 registers without spills (64 registers and
-// 4 blocks otherwise): 209-211 against 214-216 us per step on the 256^3
-// workload with the int32 table, 212 against 222-223 us with the compact one,
-// in alternating runs on one box with the same results bit for bit.
-constexpr int dev_min_blocks(Store k, int bs) { return (k == Store::F32 && bs == 256) ? 5 : 1; }
+// Where a step reads and writes: the node's own slots (a kLocal state), or
+// the slots of the int32 table, of its row form or of its compact form (a
+// kPull state).
+enum class Slots { Local, Table, Rows, Compact };
 
-template <Store K, int BS, bool GIVEN, bool WRITE, bool CT>
+// Resident blocks per SM asked of the register allocator.
+constexpr int dev_min_blocks(Store k, int bs) {
+  if (k == Store::F64D) return bs == 256 ? 2 : 1;
+  return 1280 / bs;
+}
+
+template <Store K, int BS, bool GIVEN, bool WRITE, Slots SL>
 __global__ void __launch_bounds__(BS, dev_min_blocks(K, BS)) step_dev_kernel(StepArgs a) {
   using T = typename Traits<K>::T;
   using A = typename Traits<K>::A;
   using Mac = typename Traits<K>::Mac;
+  constexpr bool CT = SL == Slots::Compact;
   const int p = blockIdx.x * BS + threadIdx.x;
   // the block's warp bases of the compact table, read once into shared
   // memory; the offset words are loaded before the barrier so that their
   // latency overlaps the bases'
   __shared__ int32_t sbase[CT ? 18 : 1][CT ? BS / 32 : 1];
   uint32_t ow[CT ? 9 : 1];
+  __shared__ SlotKeep<SL == Slots::Local ? 1 : BS> keep;
   if (CT) {
     if (p < a.n_main) {
       const uint32_t* __restrict__ off = reinterpret_cast<const uint32_t*>(a.ct_off);
@@ -94,29 +101,40 @@ __global__ void __launch_bounds__(BS, dev_min_blocks(K, BS)) step_dev_kernel(Ste
     }
     __syncthreads();
   }
+  prefetch_block<BS, SL == Slots::Rows ? 9 : SL == Slots::Table ? 18 : 0>(
+      static_cast<const T*>(a.pop), SL == Slots::Rows ? a.rows : a.table, a.npad, a.ahead);
   if (p >= a.n_main) return;
-  const T* __restrict__ src = static_cast<const T*>(a.src_pop);
-  T* __restrict__ dst = static_cast<T*>(a.dst_pop);
+  T* pop = static_cast<T*>(a.pop);
   const float scale = (float)a.fp16_scale;
   const float inv_scale = (float)(1.0 / a.fp16_scale);
 
   A f[kQ];
-  f[0] = load_pop<K>(src + p, inv_scale);
+  f[0] = load_pop_rw<K>(pop + p, inv_scale);
+  if constexpr (SL == Slots::Local) {
 #pragma unroll
-  if (CT) {
-    const int wl = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 1; q < kQ; q++) {
-      const int32_t b = sbase[q - 1][wl];
-      const int o = ((q - 1) & 1) ? (int)(ow[(q - 1) >> 1] >> 16) : (int)(ow[(q - 1) >> 1] & 0xFFFFu);
-      int32_t t = 0;
-      if (b < 0) t = __ldg(a.table + (size_t)(q - 1) * a.npad + p);
-      const int32_t c = o == 0xFFFF ? opp(q) * a.npad + p : q * a.npad + b + o;
-      f[q] = load_pop<K>(src + (b < 0 ? t : c), inv_scale);
-    }
+    for (int q = 1; q < kQ; q++) f[q] = load_pop_rw<K>(pop + (size_t)opp(q) * a.npad + p, inv_scale);
   } else {
+    int32_t slot[kQ];  // slot[q] holds f_q on entry and takes f*_opp(q)
+    if constexpr (CT) {
+      const int wl = threadIdx.x >> 5;
 #pragma unroll
-    for (int q = 1; q < kQ; q++) f[q] = load_pop<K>(src + __ldg(a.table + (size_t)(q - 1) * a.npad + p), inv_scale);
+      for (int q = 1; q < kQ; q++) {
+        const int32_t b = sbase[q - 1][wl];
+        const int o = ((q - 1) & 1) ? (int)(ow[(q - 1) >> 1] >> 16) : (int)(ow[(q - 1) >> 1] & 0xFFFFu);
+        int32_t t = 0;
+        if (b < 0) t = __ldg(a.table + (size_t)(q - 1) * a.npad + p);
+        const int32_t c = o == 0xFFFF ? opp(q) * a.npad + p : q * a.npad + b + o;
+        slot[q] = b < 0 ? t : c;
+      }
+    } else if constexpr (SL == Slots::Rows) {
+      row_slots(a.rows, a.table, a.npad, p, slot);
+    } else {
+#pragma unroll
+      for (int q = 1; q < kQ; q++) slot[q] = __ldg(a.table + (size_t)(q - 1) * a.npad + p);
+    }
+#pragma unroll
+    for (int q = 1; q < kQ; q++) f[q] = load_pop_rw<K>(pop + slot[q], inv_scale);
+    keep_slots(keep, threadIdx.x, [&](int q) { return slot[q]; });
   }
 
   PairSplit<A> ps;
@@ -151,8 +169,13 @@ __global__ void __launch_bounds__(BS, dev_min_blocks(K, BS)) step_dev_kernel(Ste
     snap_write(a.snap_dst, a.nsnap, p - a.snap_begin, full, rho, ux, uy, uz);
   }
   mrt_collide_dev<A>(f, ps, drho, rho, ux, uy, uz, A(a.gx), A(a.gy), A(a.gz), A(a.s_v), A(a.s_o));
+  store_pop<K>(pop + p, f[0], scale);
+  if constexpr (SL == Slots::Local) {
 #pragma unroll
-  for (int q = 0; q < kQ; q++) store_pop<K>(dst + (size_t)q * a.npad + p, f[q], scale);
+    for (int q = 1; q < kQ; q++) store_pop<K>(pop + (size_t)q * a.npad + p, f[q], scale);
+  } else {
+    for_kept_slots(keep, threadIdx.x, [&](int q, int32_t slot) { store_pop<K>(pop + slot, f[opp(q)], scale); });
+  }
 }
 
 // Face nodes in deviation storage: the rules act on full populations in
@@ -166,14 +189,14 @@ __global__ void __launch_bounds__(128) bc_dev_kernel(BcArgs a) {
   const int p = a.s.n_main + b;
   if (p >= a.s.n) return;
   const StepArgs& s = a.s;
-  const T* __restrict__ src = static_cast<const T*>(s.src_pop);
+  T* pop = static_cast<T*>(s.pop);
   const float scale = (float)s.fp16_scale;
   const float inv_scale = (float)(1.0 / s.fp16_scale);
   double F[kQ];
-  F[0] = to_full<K>(load_pop<K>(src + p, inv_scale), 0);
+  F[0] = to_full<K>(load_pop_rw<K>(pop + p, inv_scale), 0);
 #pragma unroll
   for (int q = 1; q < kQ; q++)
-    F[q] = to_full<K>(load_pop<K>(src + __ldg(s.table + (size_t)(q - 1) * s.npad + p), inv_scale), q);
+    F[q] = to_full<K>(load_pop_rw<K>(pop + state_slot(s.phase, s.table, s.npad, p, q), inv_scale), q);
   // the rules on the default lattice: velocities here are in units of lat_c
   if (!GIVEN) bc_apply(a, b, F, Lattice{});
   if (FINAL) {
@@ -210,9 +233,10 @@ __global__ void __launch_bounds__(128) bc_dev_kernel(BcArgs a) {
   }
   snap_write(s.snap_dst, s.nsnap, p - s.snap_begin, F, rho, ux, uy, uz);
   mrt_collide_dev<A>(f, ps, drho, rho, ux, uy, uz, A(s.gx), A(s.gy), A(s.gz), A(s.s_v), A(s.s_o));
-  T* __restrict__ dst = static_cast<T*>(s.dst_pop);
+  store_pop<K>(pop + p, f[0], scale);
 #pragma unroll
-  for (int q = 0; q < kQ; q++) store_pop<K>(dst + (size_t)q * s.npad + p, f[q], scale);
+  for (int q = 1; q < kQ; q++)
+    store_pop<K>(pop + state_slot(s.phase, s.table, s.npad, p, opp(q)), f[q], scale);
 }
 
 template <Store K>
@@ -239,31 +263,36 @@ cudaError_t launch_boundary(Store kind, const BcArgs& a, cudaStream_t st) {
   return cudaErrorInvalidValue;
 }
 
+template <Store K, int BS, Slots SL>
+static cudaError_t launch_dev_pull(const StepArgs& a, int grid, cudaStream_t st) {
+  const bool given = a.rho_in != nullptr, write = a.rho_out != nullptr;
+  if (given && write)
+    step_dev_kernel<K, BS, true, true, SL><<<grid, BS, 0, st>>>(a);
+  else if (given)
+    step_dev_kernel<K, BS, true, false, SL><<<grid, BS, 0, st>>>(a);
+  else if (write)
+    step_dev_kernel<K, BS, false, true, SL><<<grid, BS, 0, st>>>(a);
+  else
+    step_dev_kernel<K, BS, false, false, SL><<<grid, BS, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
 template <Store K, int BS>
 static cudaError_t launch_dev_bs(const StepArgs& a, cudaStream_t st) {
   const int grid = (a.n_main + BS - 1) / BS;
   if (grid == 0) return cudaSuccess;
-  const bool given = a.rho_in != nullptr, write = a.rho_out != nullptr;
-  if (a.ct_base != nullptr) {
-    if (given && write)
-      step_dev_kernel<K, BS, true, true, true><<<grid, BS, 0, st>>>(a);
-    else if (given)
-      step_dev_kernel<K, BS, true, false, true><<<grid, BS, 0, st>>>(a);
-    else if (write)
-      step_dev_kernel<K, BS, false, true, true><<<grid, BS, 0, st>>>(a);
+  if (a.phase == kLocal) {
+    // a given state is a kPull state
+    if (a.rho_in != nullptr) return cudaErrorInvalidValue;
+    if (a.rho_out != nullptr)
+      step_dev_kernel<K, BS, false, true, Slots::Local><<<grid, BS, 0, st>>>(a);
     else
-      step_dev_kernel<K, BS, false, false, true><<<grid, BS, 0, st>>>(a);
-  } else {
-    if (given && write)
-      step_dev_kernel<K, BS, true, true, false><<<grid, BS, 0, st>>>(a);
-    else if (given)
-      step_dev_kernel<K, BS, true, false, false><<<grid, BS, 0, st>>>(a);
-    else if (write)
-      step_dev_kernel<K, BS, false, true, false><<<grid, BS, 0, st>>>(a);
-    else
-      step_dev_kernel<K, BS, false, false, false><<<grid, BS, 0, st>>>(a);
+      step_dev_kernel<K, BS, false, false, Slots::Local><<<grid, BS, 0, st>>>(a);
+    return cudaGetLastError();
   }
-  return cudaGetLastError();
+  if (a.ct_base != nullptr) return launch_dev_pull<K, BS, Slots::Compact>(a, grid, st);
+  if (a.rows != nullptr) return launch_dev_pull<K, BS, Slots::Rows>(a, grid, st);
+  return launch_dev_pull<K, BS, Slots::Table>(a, grid, st);
 }
 
 template <Store K>
@@ -301,17 +330,17 @@ cudaError_t launch_reduce(Store kind, const ReduceArgs& a, cudaStream_t st) {
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_export_pop(Store kind, const void* pop, const int32_t* table, const int32_t* ref_of, int n,
+cudaError_t launch_export_pop(Store kind, const void* pop, int phase, const int32_t* table, const int32_t* ref_of, int n,
                               int npad, double fp16_scale, double* out, cudaStream_t st, int n_main,
                               const double* bnd_f) {
   switch (kind) {
-    case Store::F64: return export_f64(pop, table, ref_of, n, npad, out, st, n_main, bnd_f);
+    case Store::F64: return export_f64(pop, phase, table, ref_of, n, npad, out, st, n_main, bnd_f);
     case Store::F64D:
-      return export_dispatch<Store::F64D>(pop, table, ref_of, n, npad, fp16_scale, out, st, n_main, bnd_f);
+      return export_dispatch<Store::F64D>(pop, phase, table, ref_of, n, npad, fp16_scale, out, st, n_main, bnd_f);
     case Store::F32:
-      return export_dispatch<Store::F32>(pop, table, ref_of, n, npad, fp16_scale, out, st, n_main, bnd_f);
+      return export_dispatch<Store::F32>(pop, phase, table, ref_of, n, npad, fp16_scale, out, st, n_main, bnd_f);
     case Store::F16:
-      return export_dispatch<Store::F16>(pop, table, ref_of, n, npad, fp16_scale, out, st, n_main, bnd_f);
+      return export_dispatch<Store::F16>(pop, phase, table, ref_of, n, npad, fp16_scale, out, st, n_main, bnd_f);
   }
   return cudaErrorInvalidValue;
 }
