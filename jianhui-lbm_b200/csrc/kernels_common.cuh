@@ -86,19 +86,35 @@ __device__ __forceinline__ typename Traits<K>::A load_pop_rw(const typename Trai
 // them: held in registers across the collision they would cost the step a
 // resident block or spills.  Written and read by the same thread only, so no
 // barrier; 16 bytes per lane and access.
+template <int BS, int NODES>
+struct SlotKeep;
 template <int BS>
-struct SlotKeep {
+struct SlotKeep<BS, 1> {
   int4 a[4][BS];
   int2 b[BS];
 };
+template <int BS>
+struct SlotKeep<BS, 2> {  // (slot q of the two nodes, slot q + 1 of the two)
+  int4 a[9][BS];
+};
 template <int BS, typename F>
-__device__ __forceinline__ void keep_slots(SlotKeep<BS>& k, int t, F&& slot) {
+__device__ __forceinline__ void keep_slots(SlotKeep<BS, 1>& k, int t, F&& slot) {
 #pragma unroll
   for (int i = 0; i < 4; i++) k.a[i][t] = make_int4(slot(4 * i + 1), slot(4 * i + 2), slot(4 * i + 3), slot(4 * i + 4));
   k.b[t] = make_int2(slot(17), slot(18));
 }
 template <int BS, typename F>
-__device__ __forceinline__ void for_kept_slots(const SlotKeep<BS>& k, int t, F&& use) {
+__device__ __forceinline__ void for_kept_slots(const SlotKeep<BS, 2>& k, int t, F&& use) {
+  asm volatile("" ::: "memory");  // as below
+#pragma unroll
+  for (int i = 0; i < 9; i++) {
+    const int4 v = k.a[i][t];
+    use(2 * i + 1, v.x, v.y);
+    use(2 * i + 2, v.z, v.w);
+  }
+}
+template <int BS, typename F>
+__device__ __forceinline__ void for_kept_slots(const SlotKeep<BS, 1>& k, int t, F&& use) {
   asm volatile("" ::: "memory");  // else the compiler carries the stored values in registers
 #pragma unroll
   for (int i = 0; i < 4; i++) {
@@ -112,13 +128,14 @@ __device__ __forceinline__ void for_kept_slots(const SlotKeep<BS>& k, int t, F&&
   use(17, w.x);
   use(18, w.y);
 }
-// Prefetches into L2 the population rows, and the table rows if any, of the BS
-// nodes `ahead` nodes after the block's: one 128-byte line per thread.
-template <int BS, int TABLE_ROWS, typename T>
+// Prefetches into L2 the population rows, and the table rows if any, of the
+// NODES nodes `ahead` nodes after the block's: one 128-byte line per thread
+// and turn.
+template <int BS, int NODES, int TABLE_ROWS, typename T>
 __device__ __forceinline__ void prefetch_block(const T* pop, const int32_t* table, int npad, int ahead) {
-  const int p = blockIdx.x * BS + ahead;
-  if (ahead == 0 || p + BS > npad) return;
-  constexpr int kPopLines = BS * (int)sizeof(T) / 128, kTableLines = BS * 4 / 128;
+  const int p = blockIdx.x * NODES + ahead;
+  if (ahead == 0 || p + NODES > npad) return;
+  constexpr int kPopLines = NODES * (int)sizeof(T) / 128, kTableLines = NODES * 4 / 128;
   for (int i = threadIdx.x; i < kQ * kPopLines + TABLE_ROWS * kTableLines; i += BS) {
     const int j = i - kQ * kPopLines;
     const char* line = j < 0 ? reinterpret_cast<const char*>(pop + (size_t)(i / kPopLines) * npad + p) + (i % kPopLines) * 128

@@ -83,16 +83,20 @@ __device__ __forceinline__ void row_sources(const int32_t (&w)[9], const int32_t
     node(qh, hi[r], fluid(qh));
   }
 }
-// The pull slots of node p: slot[q] = q * stride + m, or opp(q) * stride + p
-// behind a wall.
+// The pull slots of node p with the words w: slot[q] = q * stride + m, or
+// opp(q) * stride + p behind a wall.
+__device__ __forceinline__ void row_slots(const int32_t (&w)[9], const int32_t* __restrict__ table, int stride, int p,
+                                          int32_t (&slot)[kQ]) {
+  row_sources(w, table, stride, p, [&](int q, int32_t m, uint32_t fluid) {
+    slot[q] = fluid ? q * stride + m : opp(q) * stride + p;
+  });
+}
 __device__ __forceinline__ void row_slots(const int32_t* __restrict__ rows, const int32_t* __restrict__ table,
                                           int stride, int p, int32_t (&slot)[kQ]) {
   int32_t w[9];
 #pragma unroll
   for (int i = 0; i < 9; i++) w[i] = __ldg(rows + (size_t)i * stride + p);
-  row_sources(w, table, stride, p, [&](int q, int32_t m, uint32_t fluid) {
-    slot[q] = fluid ? q * stride + m : opp(q) * stride + p;
-  });
+  row_slots(w, table, stride, p, slot);
 }
 #endif
 

@@ -419,7 +419,7 @@ constexpr int f64_min_blocks(int bs) { return bs == 64 ? 12 : 512 / bs; }
 template <int BS, bool GIVEN, bool WRITE, bool GX, bool LAT, bool LOCAL, bool ROWS>
 __global__ void __launch_bounds__(BS, f64_min_blocks(BS)) step_f64_faithful(StepArgs a) {
   const int p = blockIdx.x * BS + threadIdx.x;
-  prefetch_block<BS, ROWS ? 9 : LOCAL ? 0 : 18>(static_cast<const double*>(a.pop), ROWS ? a.rows : a.table, a.npad,
+  prefetch_block<BS, BS, ROWS ? 9 : LOCAL ? 0 : 18>(static_cast<const double*>(a.pop), ROWS ? a.rows : a.table, a.npad,
                                                 a.ahead);
   if (p >= a.n_main) return;
   // the slots of a kPull state's gathers, for the stores after the collision

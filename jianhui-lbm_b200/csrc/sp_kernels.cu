@@ -7,6 +7,7 @@
 // a kPull state gathers and scatters them through 18 int32 table entries
 // (72 bytes more), the step after it works on the node's own slots.
 #include "bc_kernels.cuh"
+#include "collide_vec.cuh"
 #include "row_table.cuh"
 
 namespace lbm {
@@ -64,103 +65,115 @@ cudaError_t launch_compact_table(const int32_t* table, int n, int npad, int32_t*
   return cudaGetLastError();
 }
 
+// Whether a thread of an FP32-arithmetic step takes two nodes: from one node
+// per thread of a full wave's threads on.  One | two nodes, us per FP32 step:
+// 4.28 | 4.35 at 92 K nodes, 5.93 | 5.52 at 179 K, 9.12 | 8.23 at 310 K,
+// 21.1 | 18.1 at 734 K, 169 | 164 at 5.9 M; FP16 19.1 | 16.9 and 159 | 137 at
+// the last two.
+static bool two_nodes(int n) { return n >= 148 * 1024; }
+
 // Where a step reads and writes: the node's own slots (a kLocal state), or
 // the slots of the int32 table, of its row form or of its compact form (a
 // kPull state).
 enum class Slots { Local, Table, Rows, Compact };
 
-// Resident blocks per SM asked of the register allocator.
-constexpr int dev_min_blocks(Store k, int bs) {
-  if (k == Store::F64D) return bs == 256 ? 2 : 1;
-  return 1280 / bs;
+// The block's warp bases of the compact table, in shared memory, and this
+// node's offset words: the words are loaded before the barrier so that their
+// latency overlaps the bases'.
+template <int BS>
+struct CompactBlock {
+  int32_t base[18][BS / 32];
+};
+template <int BS>
+__device__ __forceinline__ void compact_load(CompactBlock<BS>& cb, const StepArgs& a, int p, uint32_t (&ow)[9]) {
+  if (p < a.n_main) {
+    const uint32_t* __restrict__ off = reinterpret_cast<const uint32_t*>(a.ct_off);
+#pragma unroll
+    for (int i = 0; i < 9; i++) ow[i] = __ldg(off + (size_t)i * a.npad + p);
+  }
+  for (int k = threadIdx.x; k < 18 * (BS / 32); k += BS) {
+    const int qq = k / (BS / 32), w = k % (BS / 32);
+    const int gw = blockIdx.x * (BS / 32) + w;
+    cb.base[qq][w] = gw < a.nwarps ? __ldg(a.ct_base + (size_t)qq * a.nwarps + gw) : -1;
+  }
+  __syncthreads();
+}
+template <int BS>
+__device__ __forceinline__ void compact_slots(const CompactBlock<BS>& cb, const StepArgs& a, int p,
+                                              const uint32_t (&ow)[9], int32_t (&slot)[kQ]) {
+  const int wl = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 1; q < kQ; q++) {
+    const int32_t b = cb.base[q - 1][wl];
+    const int o = ((q - 1) & 1) ? (int)(ow[(q - 1) >> 1] >> 16) : (int)(ow[(q - 1) >> 1] & 0xFFFFu);
+    int32_t t = 0;
+    if (b < 0) t = __ldg(a.table + (size_t)(q - 1) * a.npad + p);
+    const int32_t c = o == 0xFFFF ? opp(q) * a.npad + p : q * a.npad + b + o;
+    slot[q] = b < 0 ? t : c;
+  }
+}
+// slot[q] of node p through the int32 table, its row form or its compact form
+template <Slots SL, int BS>
+__device__ __forceinline__ void read_slots(const CompactBlock<BS>& cb, const StepArgs& a, int p,
+                                           const uint32_t (&ow)[9], int32_t (&slot)[kQ]) {
+  if constexpr (SL == Slots::Compact) {
+    compact_slots(cb, a, p, ow, slot);
+  } else if constexpr (SL == Slots::Rows) {
+    row_slots(a.rows, a.table, a.npad, p, slot);
+  } else {
+#pragma unroll
+    for (int q = 1; q < kQ; q++) slot[q] = __ldg(a.table + (size_t)(q - 1) * a.npad + p);
+  }
 }
 
-template <Store K, int BS, bool GIVEN, bool WRITE, Slots SL>
-__global__ void __launch_bounds__(BS, dev_min_blocks(K, BS)) step_dev_kernel(StepArgs a) {
-  using T = typename Traits<K>::T;
-  using A = typename Traits<K>::A;
-  using Mac = typename Traits<K>::Mac;
-  constexpr bool CT = SL == Slots::Compact;
+// The step in FP64 deviation storage; 16-warp blocks per SM asked of the
+// register allocator at 256 threads (128 registers).
+template <int BS, bool GIVEN, bool WRITE, Slots SL>
+__global__ void __launch_bounds__(BS, BS == 256 ? 2 : 1) step_dev_kernel(StepArgs a) {
+  constexpr Store K = Store::F64D;
   const int p = blockIdx.x * BS + threadIdx.x;
-  // the block's warp bases of the compact table, read once into shared
-  // memory; the offset words are loaded before the barrier so that their
-  // latency overlaps the bases'
-  __shared__ int32_t sbase[CT ? 18 : 1][CT ? BS / 32 : 1];
-  uint32_t ow[CT ? 9 : 1];
-  __shared__ SlotKeep<SL == Slots::Local ? 1 : BS> keep;
-  if (CT) {
-    if (p < a.n_main) {
-      const uint32_t* __restrict__ off = reinterpret_cast<const uint32_t*>(a.ct_off);
-#pragma unroll
-      for (int i = 0; i < 9; i++) ow[i] = __ldg(off + (size_t)i * a.npad + p);
-    }
-    for (int k = threadIdx.x; k < 18 * (BS / 32); k += BS) {
-      const int qq = k / (BS / 32), w = k % (BS / 32);
-      const int gw = blockIdx.x * (BS / 32) + w;
-      sbase[qq][w] = gw < a.nwarps ? __ldg(a.ct_base + (size_t)qq * a.nwarps + gw) : -1;
-    }
-    __syncthreads();
-  }
-  prefetch_block<BS, SL == Slots::Rows ? 9 : SL == Slots::Table ? 18 : 0>(
-      static_cast<const T*>(a.pop), SL == Slots::Rows ? a.rows : a.table, a.npad, a.ahead);
+  __shared__ SlotKeep<SL == Slots::Local ? 1 : BS, 1> keep;
+  __shared__ CompactBlock<SL == Slots::Compact ? BS : 32> cb;
+  uint32_t ow[9] = {};
+  if constexpr (SL == Slots::Compact) compact_load(cb, a, p, ow);
+  prefetch_block<BS, BS, SL == Slots::Rows ? 9 : SL == Slots::Table ? 18 : 0>(
+      static_cast<const double*>(a.pop), SL == Slots::Rows ? a.rows : a.table, a.npad, a.ahead);
   if (p >= a.n_main) return;
-  T* pop = static_cast<T*>(a.pop);
-  const float scale = (float)a.fp16_scale;
-  const float inv_scale = (float)(1.0 / a.fp16_scale);
-
-  A f[kQ];
-  f[0] = load_pop_rw<K>(pop + p, inv_scale);
+  double* pop = static_cast<double*>(a.pop);
+  double f[kQ];
+  f[0] = pop[p];
   if constexpr (SL == Slots::Local) {
 #pragma unroll
-    for (int q = 1; q < kQ; q++) f[q] = load_pop_rw<K>(pop + (size_t)opp(q) * a.npad + p, inv_scale);
+    for (int q = 1; q < kQ; q++) f[q] = pop[(size_t)opp(q) * a.npad + p];
   } else {
-    int32_t slot[kQ];  // slot[q] holds f_q on entry and takes f*_opp(q)
-    if constexpr (CT) {
-      const int wl = threadIdx.x >> 5;
+    int32_t slot[kQ];
+    read_slots<SL>(cb, a, p, ow, slot);
 #pragma unroll
-      for (int q = 1; q < kQ; q++) {
-        const int32_t b = sbase[q - 1][wl];
-        const int o = ((q - 1) & 1) ? (int)(ow[(q - 1) >> 1] >> 16) : (int)(ow[(q - 1) >> 1] & 0xFFFFu);
-        int32_t t = 0;
-        if (b < 0) t = __ldg(a.table + (size_t)(q - 1) * a.npad + p);
-        const int32_t c = o == 0xFFFF ? opp(q) * a.npad + p : q * a.npad + b + o;
-        slot[q] = b < 0 ? t : c;
-      }
-    } else if constexpr (SL == Slots::Rows) {
-      row_slots(a.rows, a.table, a.npad, p, slot);
-    } else {
-#pragma unroll
-      for (int q = 1; q < kQ; q++) slot[q] = __ldg(a.table + (size_t)(q - 1) * a.npad + p);
-    }
-#pragma unroll
-    for (int q = 1; q < kQ; q++) f[q] = load_pop_rw<K>(pop + slot[q], inv_scale);
+    for (int q = 1; q < kQ; q++) f[q] = pop[slot[q]];
     keep_slots(keep, threadIdx.x, [&](int q) { return slot[q]; });
   }
-
-  PairSplit<A> ps;
+  PairSplit<double> ps;
   split_pairs(f, ps);
-  A drho, rho, ux, uy, uz;
+  double drho, rho, ux, uy, uz;
   // velocities in units of lat_c (1 on the default lattice, where the
   // scalings below are exact)
   if (GIVEN) {
-    const Mac* r = static_cast<const Mac*>(a.rho_in);
-    const Mac* u = static_cast<const Mac*>(a.u_in);
-    const A ic = A(a.lat.ic);
-    rho = (A)r[p];
-    drho = rho - A(1);
-    ux = (A)u[p] * ic;
-    uy = (A)u[a.npad + p] * ic;
-    uz = (A)u[2 * a.npad + p] * ic;
+    const double* r = static_cast<const double*>(a.rho_in);
+    const double* u = static_cast<const double*>(a.u_in);
+    rho = r[p];
+    drho = rho - 1.0;
+    ux = u[p] * a.lat.ic;
+    uy = u[a.npad + p] * a.lat.ic;
+    uz = u[2 * a.npad + p] * a.lat.ic;
   } else {
-    macro_dev<A>(f, ps, A(0.5 * a.gx), A(0.5 * a.gy), A(0.5 * a.gz), drho, rho, ux, uy, uz);
+    macro_dev<double>(f, ps, 0.5 * a.gx, 0.5 * a.gy, 0.5 * a.gz, drho, rho, ux, uy, uz);
   }
   if (WRITE) {
-    const A c = A(a.lat.c);
-    static_cast<Mac*>(a.rho_out)[p] = (Mac)rho;
-    Mac* u = static_cast<Mac*>(a.u_out);
-    u[p] = (Mac)(ux * c);
-    u[a.npad + p] = (Mac)(uy * c);
-    u[2 * a.npad + p] = (Mac)(uz * c);
+    static_cast<double*>(a.rho_out)[p] = rho;
+    double* u = static_cast<double*>(a.u_out);
+    u[p] = ux * a.lat.c;
+    u[a.npad + p] = uy * a.lat.c;
+    u[2 * a.npad + p] = uz * a.lat.c;
   }
   if (a.snap_dst != nullptr && p >= a.snap_begin) {
     double full[kQ];
@@ -168,13 +181,152 @@ __global__ void __launch_bounds__(BS, dev_min_blocks(K, BS)) step_dev_kernel(Ste
     for (int q = 0; q < kQ; q++) full[q] = to_full<K>(f[q], q);
     snap_write(a.snap_dst, a.nsnap, p - a.snap_begin, full, rho, ux, uy, uz);
   }
-  mrt_collide_dev<A>(f, ps, drho, rho, ux, uy, uz, A(a.gx), A(a.gy), A(a.gz), A(a.s_v), A(a.s_o));
-  store_pop<K>(pop + p, f[0], scale);
+  mrt_collide_dev<double>(f, ps, drho, rho, ux, uy, uz, a.gx, a.gy, a.gz, a.s_v, a.s_o);
+  pop[p] = f[0];
   if constexpr (SL == Slots::Local) {
 #pragma unroll
-    for (int q = 1; q < kQ; q++) store_pop<K>(pop + (size_t)q * a.npad + p, f[q], scale);
+    for (int q = 1; q < kQ; q++) pop[(size_t)q * a.npad + p] = f[q];
   } else {
+    for_kept_slots(keep, threadIdx.x, [&](int q, int32_t slot) { pop[slot] = f[opp(q)]; });
+  }
+}
+
+// Resident blocks per SM asked of the register allocator: one node per
+// thread fits 1280 threads (48 registers), two nodes 640 (96 registers; 512
+// threads and 128 registers: 19.6 against 18.4 us at 128^3; 768 threads spill
+// 150-230 bytes: 22.9 us).
+template <typename V>
+constexpr int vec_min_blocks(int bs) {
+  return (VecOf<V>::kNodes == 2 ? 640 : 1280) / bs;
+}
+
+// The step in FP32 arithmetic (FP32 and FP16 storage): one node per thread
+// (V = float) or two (V = F2, collide_vec.cuh).  On its own slots a thread
+// takes nodes p and p + 1, which one access loads and stores; through the
+// table it takes p and p + 32, so that the lanes of a gather or scatter stay
+// on consecutive nodes (with p and p + 1 every one of them would touch twice
+// the sectors, half filled).
+template <Store K, int BS, typename V, bool GIVEN, bool WRITE, Slots SL>
+__global__ void __launch_bounds__(BS, vec_min_blocks<V>(BS)) step_vec_kernel(StepArgs a) {
+  using T = typename Traits<K>::T;
+  constexpr int N = VecOf<V>::kNodes;
+  static_assert(N == 1 || (!GIVEN && SL != Slots::Compact), "given states and the compact table: one node per thread");
+  constexpr bool PAIR = N == 2 && SL == Slots::Local;  // p, p + 1
+  const int p = N == 1 ? blockIdx.x * BS + threadIdx.x
+                : PAIR ? (blockIdx.x * BS + threadIdx.x) * 2
+                       : blockIdx.x * BS * 2 + (threadIdx.x >> 5) * 64 + (threadIdx.x & 31);
+  const int second = p + (PAIR ? 1 : 32);
+  __shared__ SlotKeep<SL == Slots::Local ? 1 : BS, N> keep;
+  __shared__ CompactBlock<SL == Slots::Compact ? BS : 32> cb;
+  uint32_t ow[9] = {};
+  if constexpr (SL == Slots::Compact) compact_load(cb, a, p, ow);
+  prefetch_block<BS, BS * N, SL == Slots::Rows ? 9 : SL == Slots::Table ? 18 : 0>(
+      static_cast<const T*>(a.pop), SL == Slots::Rows ? a.rows : a.table, a.npad, a.ahead);
+  if (p >= a.n_main) return;
+  const bool both = N == 2 && second < a.n_main;
+  const int p1 = both ? second : p;  // a missing second node is worked on as the first and not stored
+  T* pop = static_cast<T*>(a.pop);
+  const float scale = (float)a.fp16_scale;
+  const float inv_scale = (float)(1.0 / a.fp16_scale);
+  V f[kQ];
+  if constexpr (N == 1 || PAIR)
+    load_row<K>(pop + p, inv_scale, f[0]);
+  else
+    f[0] = make_f2(load_pop_rw<K>(pop + p, inv_scale), load_pop_rw<K>(pop + p1, inv_scale));
+  if constexpr (SL == Slots::Local) {
+#pragma unroll
+    for (int q = 1; q < kQ; q++) load_row<K>(pop + (size_t)opp(q) * a.npad + p, inv_scale, f[q]);
+  } else if constexpr (N == 1) {
+    int32_t slot[kQ];  // slot[q] holds f_q on entry and takes f*_opp(q)
+    read_slots<SL>(cb, a, p, ow, slot);
+#pragma unroll
+    for (int q = 1; q < kQ; q++) f[q] = load_pop_rw<K>(pop + slot[q], inv_scale);
+    keep_slots(keep, threadIdx.x, [&](int q) { return slot[q]; });
+  } else {
+    int32_t s0[kQ], s1[kQ];
+    if constexpr (SL == Slots::Rows) {
+      int32_t w0[9], w1[9];
+#pragma unroll
+      for (int i = 0; i < 9; i++) {
+        w0[i] = __ldg(a.rows + (size_t)i * a.npad + p);
+        w1[i] = __ldg(a.rows + (size_t)i * a.npad + p1);
+      }
+      row_slots(w0, a.table, a.npad, p, s0);
+      row_slots(w1, a.table, a.npad, p1, s1);
+    } else {
+#pragma unroll
+      for (int q = 1; q < kQ; q++) {
+        s0[q] = __ldg(a.table + (size_t)(q - 1) * a.npad + p);
+        s1[q] = __ldg(a.table + (size_t)(q - 1) * a.npad + p1);
+      }
+    }
+#pragma unroll
+    for (int q = 1; q < kQ; q++)
+      f[q] = make_f2(load_pop_rw<K>(pop + s0[q], inv_scale), load_pop_rw<K>(pop + s1[q], inv_scale));
+#pragma unroll
+    for (int i = 0; i < 9; i++)
+      keep.a[i][threadIdx.x] = make_int4(s0[2 * i + 1], s1[2 * i + 1], s0[2 * i + 2], s1[2 * i + 2]);
+  }
+
+  // velocities in units of lat_c (1 on the default lattice, where the
+  // scalings below are exact)
+  V drho, rho, ux, uy, uz;
+  if constexpr (GIVEN) {
+    const float* r = static_cast<const float*>(a.rho_in);
+    const float* u = static_cast<const float*>(a.u_in);
+    const float ic = (float)a.lat.ic;
+    rho = r[p];
+    drho = rho - 1.f;
+    ux = u[p] * ic;
+    uy = u[a.npad + p] * ic;
+    uz = u[2 * a.npad + p] * ic;
+  } else {
+    macro_vec<V>(f, (float)(0.5 * a.gx), (float)(0.5 * a.gy), (float)(0.5 * a.gz), drho, rho, ux, uy, uz);
+  }
+  if (WRITE) {
+    const V c = VecOf<V>::splat((float)a.lat.c);
+    float* u = static_cast<float*>(a.u_out);
+    const V cux = vmul(ux, c), cuy = vmul(uy, c), cuz = vmul(uz, c);
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+      const int pj = j == 0 ? p : p1;  // the first node's values again where there is no second
+      const int l = both ? j : 0;
+      static_cast<float*>(a.rho_out)[pj] = lane(rho, l);
+      u[pj] = lane(cux, l);
+      u[a.npad + pj] = lane(cuy, l);
+      u[2 * a.npad + pj] = lane(cuz, l);
+    }
+  }
+  if (a.snap_dst != nullptr) {
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+      const int pj = j == 0 ? p : second;
+      if (pj < a.snap_begin || (j == 1 && !both)) continue;
+      double full[kQ];
+#pragma unroll
+      for (int q = 0; q < kQ; q++) full[q] = to_full<K>(lane(f[q], j), q);
+      snap_write(a.snap_dst, a.nsnap, pj - a.snap_begin, full, lane(rho, j), lane(ux, j), lane(uy, j), lane(uz, j));
+    }
+  }
+  collide_vec<V>(f, drho, rho, ux, uy, uz,
+                 collide_scalars((float)a.gx, (float)a.gy, (float)a.gz, (float)a.s_v, (float)a.s_o));
+  if constexpr (N == 1 || PAIR) {
+    store_row<K>(pop + p, f[0], scale, both);
+  } else {
+    store_pop<K>(pop + p, lane(f[0], 0), scale);
+    if (both) store_pop<K>(pop + p1, lane(f[0], 1), scale);
+  }
+  if constexpr (SL == Slots::Local) {
+#pragma unroll
+    for (int q = 1; q < kQ; q++) store_row<K>(pop + (size_t)q * a.npad + p, f[q], scale, both);
+  } else if constexpr (N == 1) {
     for_kept_slots(keep, threadIdx.x, [&](int q, int32_t slot) { store_pop<K>(pop + slot, f[opp(q)], scale); });
+  } else {
+    for_kept_slots(keep, threadIdx.x, [&](int q, int32_t slot0, int32_t slot1) {
+      const float2 v = split_f2(f[opp(q)]);
+      store_pop<K>(pop + slot0, v.x, scale);
+      if (both) store_pop<K>(pop + slot1, v.y, scale);
+    });
   }
 }
 
@@ -221,7 +373,10 @@ __global__ void __launch_bounds__(128) bc_dev_kernel(BcArgs a) {
     uy = (A)u[s.npad + p] * ic;
     uz = (A)u[2 * s.npad + p] * ic;
   } else {
-    macro_dev<A>(f, ps, A(0.5 * s.gx), A(0.5 * s.gy), A(0.5 * s.gz), drho, rho, ux, uy, uz);
+    if constexpr (sizeof(A) == 4)
+      macro_vec<float>(f, (float)(0.5 * s.gx), (float)(0.5 * s.gy), (float)(0.5 * s.gz), drho, rho, ux, uy, uz);
+    else
+      macro_dev<A>(f, ps, A(0.5 * s.gx), A(0.5 * s.gy), A(0.5 * s.gz), drho, rho, ux, uy, uz);
   }
   if (s.rho_out != nullptr) {
     const A c = A(s.lat.c);
@@ -232,7 +387,11 @@ __global__ void __launch_bounds__(128) bc_dev_kernel(BcArgs a) {
     u[2 * s.npad + p] = (Mac)(uz * c);
   }
   snap_write(s.snap_dst, s.nsnap, p - s.snap_begin, F, rho, ux, uy, uz);
-  mrt_collide_dev<A>(f, ps, drho, rho, ux, uy, uz, A(s.gx), A(s.gy), A(s.gz), A(s.s_v), A(s.s_o));
+  if constexpr (sizeof(A) == 4)
+    collide_vec<float>(f, drho, rho, ux, uy, uz,
+                       collide_scalars((float)s.gx, (float)s.gy, (float)s.gz, (float)s.s_v, (float)s.s_o));
+  else
+    mrt_collide_dev<A>(f, ps, drho, rho, ux, uy, uz, A(s.gx), A(s.gy), A(s.gz), A(s.s_v), A(s.s_o));
   store_pop<K>(pop + p, f[0], scale);
 #pragma unroll
   for (int q = 1; q < kQ; q++)
@@ -263,36 +422,58 @@ cudaError_t launch_boundary(Store kind, const BcArgs& a, cudaStream_t st) {
   return cudaErrorInvalidValue;
 }
 
-template <Store K, int BS, Slots SL>
-static cudaError_t launch_dev_pull(const StepArgs& a, int grid, cudaStream_t st) {
+template <int BS, Slots SL>
+static void launch_f64d(const StepArgs& a, int grid, cudaStream_t st) {
   const bool given = a.rho_in != nullptr, write = a.rho_out != nullptr;
-  if (given && write)
-    step_dev_kernel<K, BS, true, true, SL><<<grid, BS, 0, st>>>(a);
-  else if (given)
-    step_dev_kernel<K, BS, true, false, SL><<<grid, BS, 0, st>>>(a);
-  else if (write)
-    step_dev_kernel<K, BS, false, true, SL><<<grid, BS, 0, st>>>(a);
-  else
-    step_dev_kernel<K, BS, false, false, SL><<<grid, BS, 0, st>>>(a);
-  return cudaGetLastError();
+  if constexpr (SL != Slots::Local) {
+    if (given)
+      return write ? step_dev_kernel<BS, true, true, SL><<<grid, BS, 0, st>>>(a)
+                   : step_dev_kernel<BS, true, false, SL><<<grid, BS, 0, st>>>(a);
+  }
+  write ? step_dev_kernel<BS, false, true, SL><<<grid, BS, 0, st>>>(a)
+        : step_dev_kernel<BS, false, false, SL><<<grid, BS, 0, st>>>(a);
+}
+template <Store K, int BS, typename V, Slots SL>
+static void launch_vec(const StepArgs& a, int grid, cudaStream_t st) {
+  const bool given = a.rho_in != nullptr, write = a.rho_out != nullptr;
+  if constexpr (SL != Slots::Local && VecOf<V>::kNodes == 1) {
+    if (given)
+      return write ? step_vec_kernel<K, BS, V, true, true, SL><<<grid, BS, 0, st>>>(a)
+                   : step_vec_kernel<K, BS, V, true, false, SL><<<grid, BS, 0, st>>>(a);
+  }
+  write ? step_vec_kernel<K, BS, V, false, true, SL><<<grid, BS, 0, st>>>(a)
+        : step_vec_kernel<K, BS, V, false, false, SL><<<grid, BS, 0, st>>>(a);
 }
 
 template <Store K, int BS>
 static cudaError_t launch_dev_bs(const StepArgs& a, cudaStream_t st) {
-  const int grid = (a.n_main + BS - 1) / BS;
-  if (grid == 0) return cudaSuccess;
-  if (a.phase == kLocal) {
-    // a given state is a kPull state
-    if (a.rho_in != nullptr) return cudaErrorInvalidValue;
-    if (a.rho_out != nullptr)
-      step_dev_kernel<K, BS, false, true, Slots::Local><<<grid, BS, 0, st>>>(a);
-    else
-      step_dev_kernel<K, BS, false, false, Slots::Local><<<grid, BS, 0, st>>>(a);
-    return cudaGetLastError();
+  if (a.n_main <= 0) return cudaSuccess;
+  const bool local = a.phase == kLocal;
+  if (local && a.rho_in != nullptr) return cudaErrorInvalidValue;  // a given state is a kPull state
+  const Slots sl = local ? Slots::Local : a.ct_base ? Slots::Compact : a.rows ? Slots::Rows : Slots::Table;
+  const int grid = (a.n_main + BS - 1) / BS;  // BS nodes per block, by BS or BS / 2 threads
+  if constexpr (K == Store::F64D) {
+    switch (sl) {
+      case Slots::Local: launch_f64d<BS, Slots::Local>(a, grid, st); break;
+      case Slots::Table: launch_f64d<BS, Slots::Table>(a, grid, st); break;
+      case Slots::Rows: launch_f64d<BS, Slots::Rows>(a, grid, st); break;
+      case Slots::Compact: launch_f64d<BS, Slots::Compact>(a, grid, st); break;
+    }
+  } else if (a.rho_in == nullptr && sl != Slots::Compact && two_nodes(a.n_main)) {
+    switch (sl) {
+      case Slots::Local: launch_vec<K, BS / 2, F2, Slots::Local>(a, grid, st); break;
+      case Slots::Rows: launch_vec<K, BS / 2, F2, Slots::Rows>(a, grid, st); break;
+      default: launch_vec<K, BS / 2, F2, Slots::Table>(a, grid, st); break;
+    }
+  } else {
+    switch (sl) {
+      case Slots::Local: launch_vec<K, BS, float, Slots::Local>(a, grid, st); break;
+      case Slots::Table: launch_vec<K, BS, float, Slots::Table>(a, grid, st); break;
+      case Slots::Rows: launch_vec<K, BS, float, Slots::Rows>(a, grid, st); break;
+      case Slots::Compact: launch_vec<K, BS, float, Slots::Compact>(a, grid, st); break;
+    }
   }
-  if (a.ct_base != nullptr) return launch_dev_pull<K, BS, Slots::Compact>(a, grid, st);
-  if (a.rows != nullptr) return launch_dev_pull<K, BS, Slots::Rows>(a, grid, st);
-  return launch_dev_pull<K, BS, Slots::Table>(a, grid, st);
+  return cudaGetLastError();
 }
 
 template <Store K>
