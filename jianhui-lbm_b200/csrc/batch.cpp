@@ -110,15 +110,15 @@ struct Pool {
   int block = 256, grid = 0;
   int ordering = LBM_ORDER_REFERENCE;
   double fp16_scale = 1.0;
-  Buf pop[2], table, tile_inst, inst, state, partials, active_tiles, n_active, work, slot_off;
+  Buf pop, table, rows, tile_inst, inst, state, partials, active_tiles, n_active, work, slot_off;
   SetupScratch setup;
   std::vector<InstParams> h_inst;
   InstState* h_state = nullptr;  // pinned
   std::vector<int> h_tile_inst;
   std::map<int, int> free_tiles;  // first tile -> length
   std::vector<std::unique_ptr<Job>> slot_job;
-  std::vector<int> slot_parity;  // buffer holding a finished slot's state
-  int cur = 0;
+  std::vector<int> slot_phase;  // phase of a finished slot's state
+  int cur = kPull;              // phase of the stepping slots' state
   // chain graphs per step grid (the grid follows the stepping tile count,
   // rounded up to a power of two, so a few graphs cover every pool state)
   std::map<int, std::array<cudaGraphExec_t, 2>> graphs;
@@ -172,8 +172,11 @@ struct Pool {
     LBM_CUDA_TRY(cudaEventCreate(&chain_ev0));
     LBM_CUDA_TRY(cudaEventCreate(&chain_ev1));
     const size_t s = store_bytes(kind);
-    for (auto& b : pop) LBM_CUDA_TRY(b.alloc((size_t)kQ * cap * s));
+    LBM_CUDA_TRY(pop.alloc((size_t)kQ * cap * s));
     LBM_CUDA_TRY(table.alloc((size_t)18 * cap * sizeof(int32_t)));
+    // the row form of the table, for pools whose chains may exceed L2
+    if (ordering == LBM_ORDER_REFERENCE && rows_large(cap, kQ * (long long)s))
+      LBM_CUDA_TRY(rows.alloc((size_t)9 * cap * sizeof(int32_t)));
     LBM_CUDA_TRY(tile_inst.alloc((size_t)ntiles * sizeof(int)));
     LBM_CUDA_TRY(inst.alloc((size_t)nslots * sizeof(InstParams)));
     LBM_CUDA_TRY(state.alloc((size_t)nslots * sizeof(InstState)));
@@ -188,7 +191,7 @@ struct Pool {
     h_inst.assign(nslots, InstParams{});
     h_tile_inst.assign(ntiles, -1);
     slot_job.resize(nslots);
-    slot_parity.assign(nslots, 0);
+    slot_phase.assign(nslots, kPull);
     free_tiles.clear();
     free_tiles[0] = ntiles;
     LBM_CUDA_TRY(cudaMemcpyAsync(tile_inst.p, h_tile_inst.data(), (size_t)ntiles * sizeof(int),
@@ -269,12 +272,15 @@ struct Pool {
                                      cudaMemcpyHostToDevice, stream));
       LBM_CUDA_TRY(cudaStreamSynchronize(stream));  // rows is a host temporary
     }
+    if (rows.p)
+      LBM_CUDA_TRY(launch_row_table(table.as<int32_t>(), cap, ip.begin, j.geo.count, rows.as<int32_t>(), nullptr,
+                                    stream));
     for (int t = ip.tile_begin; t < ip.tile_end; t++) h_tile_inst[t] = slot;
     LBM_CUDA_TRY(cudaMemcpyAsync(tile_inst.as<int>() + ip.tile_begin, h_tile_inst.data() + ip.tile_begin,
                                  sizeof(int) * (ip.tile_end - ip.tile_begin), cudaMemcpyHostToDevice, stream));
     LBM_CUDA_TRY(cudaMemcpyAsync(inst.as<InstParams>() + slot, &h_inst[slot], sizeof(InstParams),
                                  cudaMemcpyHostToDevice, stream));
-    LBM_CUDA_TRY(launch_batch_init(kind, pop[cur].p, table.as<int32_t>(), cap, ip.begin, j.geo.count, ip, stream));
+    LBM_CUDA_TRY(launch_batch_init(kind, pop.p, cur, table.as<int32_t>(), cap, ip.begin, j.geo.count, ip, stream));
     InstState st{};
     st.active = 1;
     st.fresh = 1;
@@ -300,11 +306,16 @@ struct Pool {
     return LBM_OK;
   }
 
-  BatchStepArgs step_args(int c) const {
+  // A step from phase c over step_grid tiles; the row form of the table where
+  // they exceed L2 (its marked nodes are the x wraps in reference order).
+  BatchStepArgs step_args(int c, int step_grid) const {
     BatchStepArgs a{};
-    a.src_pop = pop[c].p;
-    a.dst_pop = pop[1 - c].p;
+    a.pop = pop.p;
+    a.phase = c;
     a.table = table.as<int32_t>();
+    if (rows.p && ordering == LBM_ORDER_REFERENCE &&
+        rows_large((long long)step_grid * kTile, kQ * (long long)store_bytes(kind)))
+      a.rows = rows.as<int32_t>();
     a.cap = cap;
     a.ntiles = ntiles;
     a.tile_inst = tile_inst.as<int>();
@@ -317,7 +328,8 @@ struct Pool {
   }
   BatchReduceArgs reduce_args(int c) const {
     BatchReduceArgs r{};
-    r.pop = pop[c].p;
+    r.pop = pop.p;
+    r.phase = c;
     r.table = table.as<int32_t>();
     r.cap = cap;
     r.ntiles = ntiles;
@@ -341,7 +353,7 @@ struct Pool {
     cudaError_t err = launch_batch_list(reduce_args(c0), step_grid, block, stream);
     int c = c0;
     for (int s = 0; s < chain && err == cudaSuccess; s++) {
-      err = launch_batch_step(kind, step_args(c), block, step_grid, s, stream);
+      err = launch_batch_step(kind, step_args(c, step_grid), block, step_grid, s, stream);
       c = 1 - c;
     }
     if (err == cudaSuccess) err = launch_batch_check(kind, reduce_args(c), chain, tol, max_steps, stream);
@@ -430,7 +442,7 @@ struct Pool {
     LBM_CUDA_TRY(cudaMemcpyAsync(ref.p, ref_src, sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream));
     LBM_CUDA_TRY(cudaMemsetAsync(r.p, 0, r.bytes, stream));
     LBM_CUDA_TRY(cudaMemsetAsync(v.p, 0, v.bytes, stream));
-    LBM_CUDA_TRY(launch_batch_export_macro(kind, pop[slot_parity[slot]].p, table.as<int32_t>(), cap, ip.begin, n,
+    LBM_CUDA_TRY(launch_batch_export_macro(kind, pop.p, slot_phase[slot], table.as<int32_t>(), cap, ip.begin, n,
                                            ref.as<int32_t>(), ip, r.as<double>(), v.as<double>(), stream));
     if (rho) LBM_CUDA_TRY(cudaMemcpyAsync(rho, r.p, r.bytes, cudaMemcpyDeviceToHost, stream));
     if (u) LBM_CUDA_TRY(cudaMemcpyAsync(u, v.p, v.bytes, cudaMemcpyDeviceToHost, stream));
@@ -509,7 +521,7 @@ lbm_status batch_layout(lbm_batch* b) {
   for (int i = 0; i < b->n; i++) {
     lbm_status st = P.place(i, b->first_tile[i]);
     if (st != LBM_OK) return st;
-    P.slot_parity[i] = 0;
+    P.slot_phase[i] = kPull;
   }
   P.drop_graphs();
   return LBM_OK;
@@ -517,11 +529,11 @@ lbm_status batch_layout(lbm_batch* b) {
 
 lbm_status batch_reset(lbm_batch* b) {
   Pool& P = b->pool;
-  P.cur = 0;
+  P.cur = kPull;
   for (int i = 0; i < b->n; i++) {
     lbm_status st = P.place(i, b->first_tile[i]);
     if (st != LBM_OK) return st;
-    P.slot_parity[i] = 0;
+    P.slot_phase[i] = kPull;
   }
   return LBM_OK;
 }
@@ -600,10 +612,10 @@ lbm_status lbm_batch_run(lbm_batch* b, double tol, int check_every, long long ma
     lbm_status st = P.launch_chain(check_every, tol, max_steps);
     if (st != LBM_OK) return st;
     if ((st = P.wait_chain()) != LBM_OK) return st;
-    // a solve that stopped in this chain keeps its last state in the buffer
+    // a solve that stopped in this chain keeps its last state in the phase
     // the chain ended on; later chains skip its tiles
     for (int i = 0; i < b->n; i++)
-      if (was_active[i] && !P.h_state[i].active) P.slot_parity[i] = P.cur;
+      if (was_active[i] && !P.h_state[i].active) P.slot_phase[i] = P.cur;
   }
   LBM_CUDA_TRY(cudaEventRecord(P.ev1, P.stream));
   LBM_CUDA_TRY(cudaEventSynchronize(P.ev1));
@@ -651,12 +663,12 @@ lbm_status lbm_batch_autotune(lbm_batch* b, int trial_steps, int* ordering_out, 
       if ((st = batch_reset(b)) != LBM_OK) return st;
       LBM_CUDA_TRY(launch_batch_list(P.reduce_args(P.cur), P.grid, P.block, P.stream));
       for (int s = 0; s < 2; s++) {  // warm-up
-        LBM_CUDA_TRY(launch_batch_step(P.kind, P.step_args(P.cur), P.block, P.grid, s, P.stream));
+        LBM_CUDA_TRY(launch_batch_step(P.kind, P.step_args(P.cur, P.grid), P.block, P.grid, s, P.stream));
         P.cur = 1 - P.cur;
       }
       LBM_CUDA_TRY(cudaEventRecord(P.ev0, P.stream));
       for (int s = 0; s < trial_steps; s++) {
-        LBM_CUDA_TRY(launch_batch_step(P.kind, P.step_args(P.cur), P.block, P.grid, 1, P.stream));
+        LBM_CUDA_TRY(launch_batch_step(P.kind, P.step_args(P.cur, P.grid), P.block, P.grid, 1, P.stream));
         P.cur = 1 - P.cur;
       }
       LBM_CUDA_TRY(cudaEventRecord(P.ev1, P.stream));

@@ -43,9 +43,10 @@ struct TileWork {
 };
 
 struct BatchStepArgs {
-  const void* src_pop;
-  void* dst_pop;
+  void* pop;   // [19][cap], updated in place (kernels_common.cuh)
+  int phase;   // Phase of the pool's state
   const int32_t* table;
+  const int32_t* rows;  // [9][cap] row form of the table, or null (read `table`)
   int cap;     // pool nodes (row stride)
   int ntiles;  // cap / kTile
   const int* tile_inst;
@@ -58,6 +59,7 @@ struct BatchStepArgs {
 
 struct BatchReduceArgs {
   const void* pop;
+  int phase;
   const int32_t* table;
   int cap;
   int ntiles;
@@ -80,10 +82,10 @@ cudaError_t launch_batch_step(Store kind, const BatchStepArgs& a, int block, int
                               cudaStream_t st);
 cudaError_t launch_batch_check(Store kind, const BatchReduceArgs& a, int chain_len, double tol, long long max_steps,
                                cudaStream_t st);
-cudaError_t launch_batch_export_macro(Store kind, const void* pop, const int32_t* table, int cap, int begin, int n,
+cudaError_t launch_batch_export_macro(Store kind, const void* pop, int phase, const int32_t* table, int cap, int begin, int n,
                                       const int32_t* ref_of, const InstParams& ip, double* rho, double* u,
                                       cudaStream_t st);
-cudaError_t launch_batch_init(Store kind, void* pop, const int32_t* table, int cap, int begin, int n,
+cudaError_t launch_batch_init(Store kind, void* pop, int phase, const int32_t* table, int cap, int begin, int n,
                               const InstParams& ip, cudaStream_t st);
 // Largest step grid of a pool: one block per tile of the pool (a block steps
 // its tile in kTile / block passes).

@@ -1,7 +1,9 @@
 // Many independent single-phase solves in one node pool.
 //
 // Layout: every instance owns a contiguous, tile-aligned node range
-// [begin, end) of one population pool pop[19][cap] and one pull table
+// [begin, end) of one population pool pop[19][cap], stepped in place
+// (kernels_common.cuh: all stepping instances are in the same phase, a
+// stopped one keeps the phase of its last chain's end), and one pull table
 // [18][cap] whose entries are flat indices q*cap + m into the same pool (an
 // instance only ever pulls from its own range).  The pool is cut into tiles
 // of kTile nodes; tile_inst[t] names the instance slot owning tile t (-1 =
@@ -17,56 +19,90 @@
 // applies the reference's stop test |(u_ave_prev - u_ave)/u_ave_prev| < tol
 // (SP:812-816, u_ave from Comput_Perm SP3:3634-3638) per instance.
 #include "batch.h"
-#include "kernels_common.cuh"
+#include "collide_vec.cuh"
+#include "row_table.cuh"
 
 namespace lbm {
 
 // Block b steps tile b of the work list (the stepping tiles in list order):
-// kTile / BS passes of BS nodes, all on the one broadcast load of the tile's
+// kTile / (2 BS) passes of 2 BS nodes, all on the one broadcast load of the tile's
 // entry (the single-domain step waits on none).  The host launches at least
 // as many blocks as there are stepping tiles (a power of two at or above
 // their count, chain_grid), and the list kernels fill the entries past the
 // stepping tiles with an empty node range, so a block needs no count of the
 // stepping tiles: the blocks past the list read an empty entry and exit.
-// FP32 at 256 threads: 5 resident blocks per SM in 48 registers without
-// spills, as the single-domain step (16 sphere packs to the stop test:
-// 0.427-0.429 against 0.430-0.432 s at 4 blocks, alternating runs).
-template <Store K, int BS>
-__global__ void __launch_bounds__(BS, (K == Store::F32 && BS == 256) ? 5 : 1)
-    batch_step_kernel(BatchStepArgs a, int chain_step) {
+// A thread takes two nodes (collide_vec.cuh), neighbours on the node's own
+// slots and 32 apart through the table, as the single-domain step; BS threads
+// step 2 BS nodes a pass, 5 blocks of 128 threads per SM in 96 registers.
+template <Store K, int BS, bool LOCAL, bool ROWS>
+__global__ void __launch_bounds__(BS, 640 / BS) batch_step_kernel(BatchStepArgs a, int chain_step) {
   using T = typename Traits<K>::T;
-  using A = typename Traits<K>::A;
-  constexpr int kSub = kTile / BS;
-  const T* __restrict__ src = static_cast<const T*>(a.src_pop);
-  T* __restrict__ dst = static_cast<T*>(a.dst_pop);
-  const size_t cap = (size_t)a.cap;
+  constexpr int kSub = kTile / (2 * BS);
+  T* pop = static_cast<T*>(a.pop);
+  const int cap = a.cap;
   const int i = blockIdx.x;
   if (i >= a.ntiles) return;
+  __shared__ SlotKeep<LOCAL ? 1 : BS, 2> keep;
   const TileWork w = a.work[i];
   const float scale = w.fp16_scale, inv_scale = 1.0f / w.fp16_scale;
+  const CollideScalars cs = collide_scalars(w.g[0], w.g[1], w.g[2], w.s_v, w.s_o);
 #pragma unroll 1
   for (int sub = 0; sub < kSub; sub++) {
-    const int p = w.p0 + sub * BS + threadIdx.x;
-    if (p >= w.end) return;
-    A f[kQ];
-    f[0] = load_pop<K>(src + p, inv_scale);
+    const int base = w.p0 + sub * 2 * BS;
+    const int p = LOCAL ? base + 2 * threadIdx.x : base + (threadIdx.x >> 5) * 64 + (threadIdx.x & 31);
+    if (p >= w.end) continue;  // a warp's first nodes ascend with the pass
+    const int second = p + (LOCAL ? 1 : 32);
+    const bool both = second < w.end;
+    const int p1 = both ? second : p;  // a missing second node is worked on as the first and not stored
+    F2 f[kQ];
+    if constexpr (LOCAL) {
+      load_row<K>(pop + p, inv_scale, f[0]);
 #pragma unroll
-    for (int q = 1; q < kQ; q++) f[q] = load_pop<K>(src + __ldg(a.table + (size_t)(q - 1) * cap + p), inv_scale);
-    PairSplit<A> ps;
-    split_pairs(f, ps);
-    A drho, rho, ux, uy, uz;
-    if (chain_step == 0 && w.fresh) {
-      rho = A(1);
-      drho = A(0);
-      ux = A(w.u0[0]);
-      uy = A(w.u0[1]);
-      uz = A(w.u0[2]);
+      for (int q = 1; q < kQ; q++) load_row<K>(pop + (size_t)opp(q) * cap + p, inv_scale, f[q]);
     } else {
-      macro_dev<A>(f, ps, A(0.5f * w.g[0]), A(0.5f * w.g[1]), A(0.5f * w.g[2]), drho, rho, ux, uy, uz);
-    }
-    mrt_collide_dev<A>(f, ps, drho, rho, ux, uy, uz, A(w.g[0]), A(w.g[1]), A(w.g[2]), A(w.s_v), A(w.s_o));
+      f[0] = make_f2(load_pop_rw<K>(pop + p, inv_scale), load_pop_rw<K>(pop + p1, inv_scale));
+      int32_t s0[kQ], s1[kQ];
+      if constexpr (ROWS) {
+        row_slots(a.rows, a.table, cap, p, s0);
+        row_slots(a.rows, a.table, cap, p1, s1);
+      } else {
 #pragma unroll
-    for (int q = 0; q < kQ; q++) store_pop<K>(dst + (size_t)q * cap + p, f[q], scale);
+        for (int q = 1; q < kQ; q++) {
+          s0[q] = __ldg(a.table + (size_t)(q - 1) * cap + p);
+          s1[q] = __ldg(a.table + (size_t)(q - 1) * cap + p1);
+        }
+      }
+#pragma unroll
+      for (int q = 1; q < kQ; q++)
+        f[q] = make_f2(load_pop_rw<K>(pop + s0[q], inv_scale), load_pop_rw<K>(pop + s1[q], inv_scale));
+#pragma unroll
+      for (int j = 0; j < 9; j++)
+        keep.a[j][threadIdx.x] = make_int4(s0[2 * j + 1], s1[2 * j + 1], s0[2 * j + 2], s1[2 * j + 2]);
+    }
+    F2 drho, rho, ux, uy, uz;
+    if (chain_step == 0 && w.fresh) {
+      rho = VecOf<F2>::splat(1.f);
+      drho = VecOf<F2>::splat(0.f);
+      ux = VecOf<F2>::splat(w.u0[0]);
+      uy = VecOf<F2>::splat(w.u0[1]);
+      uz = VecOf<F2>::splat(w.u0[2]);
+    } else {
+      macro_vec<F2>(f, 0.5f * w.g[0], 0.5f * w.g[1], 0.5f * w.g[2], drho, rho, ux, uy, uz);
+    }
+    collide_vec<F2>(f, drho, rho, ux, uy, uz, cs);
+    if constexpr (LOCAL) {
+      store_row<K>(pop + p, f[0], scale, both);
+#pragma unroll
+      for (int q = 1; q < kQ; q++) store_row<K>(pop + (size_t)q * cap + p, f[q], scale, both);
+    } else {
+      store_pop<K>(pop + p, lane(f[0], 0), scale);
+      if (both) store_pop<K>(pop + p1, lane(f[0], 1), scale);
+      for_kept_slots(keep, threadIdx.x, [&](int q, int32_t slot0, int32_t slot1) {
+        const float2 v = split_f2(f[opp(q)]);
+        store_pop<K>(pop + slot0, v.x, scale);
+        if (both) store_pop<K>(pop + slot1, v.y, scale);
+      });
+    }
   }
 }
 
@@ -164,7 +200,7 @@ __device__ __forceinline__ void batch_tile_sum(const BatchReduceArgs& a, int t, 
     A f[kQ];
     f[0] = load_pop<K>(pop + p, inv_scale);
 #pragma unroll
-    for (int q = 1; q < kQ; q++) f[q] = load_pop<K>(pop + __ldg(a.table + (size_t)(q - 1) * cap + p), inv_scale);
+    for (int q = 1; q < kQ; q++) f[q] = load_pop<K>(pop + state_slot(a.phase, a.table, a.cap, p, q), inv_scale);
     PairSplit<A> ps;
     split_pairs(f, ps);
     A drho, rho, ux, uy, uz;
@@ -238,7 +274,8 @@ __global__ void __launch_bounds__(256) batch_update_kernel(BatchReduceArgs a, in
 
 // Post-streaming macro fields of one instance (reference layout, double).
 template <Store K>
-__global__ void batch_export_macro_kernel(const typename Traits<K>::T* __restrict__ pop, const int32_t* __restrict__ table,
+__global__ void batch_export_macro_kernel(const typename Traits<K>::T* __restrict__ pop, int phase,
+                                          const int32_t* __restrict__ table,
                                           int cap, int begin, int n, const int32_t* __restrict__ ref_of,
                                           InstParams ip, double* __restrict__ rho_ref, double* __restrict__ u_ref) {
   using A = typename Traits<K>::A;
@@ -249,7 +286,7 @@ __global__ void batch_export_macro_kernel(const typename Traits<K>::T* __restric
   A f[kQ];
   f[0] = load_pop<K>(pop + p, inv_scale);
 #pragma unroll
-  for (int q = 1; q < kQ; q++) f[q] = load_pop<K>(pop + table[(size_t)(q - 1) * cap + p], inv_scale);
+  for (int q = 1; q < kQ; q++) f[q] = load_pop<K>(pop + state_slot(phase, table, cap, p, q), inv_scale);
   PairSplit<A> ps;
   split_pairs(f, ps);
   A drho, rho, ux, uy, uz;
@@ -263,10 +300,12 @@ __global__ void batch_export_macro_kernel(const typename Traits<K>::T* __restric
   }
 }
 
-// Uniform initial state feq(1, u0) of one instance's nodes, through the
-// inverse pull (the table is a permutation of the instance's slots).
+// Uniform initial state feq(1, u0) of one instance's nodes in the pool's
+// phase: in the slots the next step reads (the table is a permutation of the
+// instance's slots).
 template <Store K>
-__global__ void batch_init_kernel(typename Traits<K>::T* __restrict__ pop, const int32_t* __restrict__ table, int cap,
+__global__ void batch_init_kernel(typename Traits<K>::T* __restrict__ pop, int phase,
+                                  const int32_t* __restrict__ table, int cap,
                                   int begin, int n, InstParams ip) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -277,17 +316,27 @@ __global__ void batch_init_kernel(typename Traits<K>::T* __restrict__ pop, const
     const double eu = cx(q) * u[0] + cy(q) * u[1] + cz(q) * u[2];
     const double uv = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
     const double feq = weight(q) * (1.0 + 3.0 * eu + 4.5 * eu * eu - 1.5 * uv);
-    const size_t dst = q == 0 ? (size_t)p : (size_t)table[(size_t)(q - 1) * cap + p];
+    const size_t dst = q == 0 ? (size_t)p : (size_t)state_slot(phase, table, cap, p, q);
     store_pop<K>(pop + dst, from_full<K>(feq, q), ip.fp16_scale);
   }
 }
 
+template <Store K, int BS>
+static void step_bs(const BatchStepArgs& a, int grid, int chain_step, cudaStream_t st) {
+  if (a.phase == kLocal)
+    batch_step_kernel<K, BS, true, false><<<grid, BS, 0, st>>>(a, chain_step);
+  else if (a.rows != nullptr)
+    batch_step_kernel<K, BS, false, true><<<grid, BS, 0, st>>>(a, chain_step);
+  else
+    batch_step_kernel<K, BS, false, false><<<grid, BS, 0, st>>>(a, chain_step);
+}
+// `block` nodes a pass, two per thread.
 template <Store K>
 static cudaError_t step_k(const BatchStepArgs& a, int block, int grid, int chain_step, cudaStream_t st) {
   switch (block) {
-    case 128: batch_step_kernel<K, 128><<<grid, 128, 0, st>>>(a, chain_step); break;
-    case 512: batch_step_kernel<K, 512><<<grid, 512, 0, st>>>(a, chain_step); break;
-    default: batch_step_kernel<K, 256><<<grid, 256, 0, st>>>(a, chain_step); break;
+    case 128: step_bs<K, 64>(a, grid, chain_step, st); break;
+    case 512: step_bs<K, 256>(a, grid, chain_step, st); break;
+    default: step_bs<K, 128>(a, grid, chain_step, st); break;
   }
   return cudaGetLastError();
 }
@@ -322,26 +371,26 @@ cudaError_t launch_batch_check(Store kind, const BatchReduceArgs& a, int chain_l
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_export_macro(Store kind, const void* pop, const int32_t* table, int cap, int begin, int n,
+cudaError_t launch_batch_export_macro(Store kind, const void* pop, int phase, const int32_t* table, int cap, int begin, int n,
                                       const int32_t* ref_of, const InstParams& ip, double* rho, double* u,
                                       cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   const int g = (n + 255) / 256;
   if (kind == Store::F16)
-    batch_export_macro_kernel<Store::F16><<<g, 256, 0, st>>>((const __half*)pop, table, cap, begin, n, ref_of, ip, rho, u);
+    batch_export_macro_kernel<Store::F16><<<g, 256, 0, st>>>((const __half*)pop, phase, table, cap, begin, n, ref_of, ip, rho, u);
   else
-    batch_export_macro_kernel<Store::F32><<<g, 256, 0, st>>>((const float*)pop, table, cap, begin, n, ref_of, ip, rho, u);
+    batch_export_macro_kernel<Store::F32><<<g, 256, 0, st>>>((const float*)pop, phase, table, cap, begin, n, ref_of, ip, rho, u);
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_init(Store kind, void* pop, const int32_t* table, int cap, int begin, int n,
+cudaError_t launch_batch_init(Store kind, void* pop, int phase, const int32_t* table, int cap, int begin, int n,
                               const InstParams& ip, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   const int g = (n + 255) / 256;
   if (kind == Store::F16)
-    batch_init_kernel<Store::F16><<<g, 256, 0, st>>>((__half*)pop, table, cap, begin, n, ip);
+    batch_init_kernel<Store::F16><<<g, 256, 0, st>>>((__half*)pop, phase, table, cap, begin, n, ip);
   else
-    batch_init_kernel<Store::F32><<<g, 256, 0, st>>>((float*)pop, table, cap, begin, n, ip);
+    batch_init_kernel<Store::F32><<<g, 256, 0, st>>>((float*)pop, phase, table, cap, begin, n, ip);
   return cudaGetLastError();
 }
 
