@@ -52,15 +52,25 @@ struct lbm_st7_handle {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   Geometry geo;
-  Mem g[2], table, u, c0, ref_of;
-  int cur = 0;
+  Mem g, table, rows, u, c0, ref_of;
+  int cur = kPull;  // phase of g
+  bool rows_on = false;
+  // captured step chains, one per starting phase
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};
   bool given = true;
   long long step = 0;
   double tau_s = 1.0;
   double c2 = 1.0, c4 = 1.0;  // lat_c^2, lat_c^4 (lattice_v)
   double last_ms = 0;
   int nq = 7;  // 7: D3Q7 solute program, 19: D3Q19 solute program
+  void drop_graphs() {
+    for (auto& e : graph) {
+      if (e) cudaGraphExecDestroy(e);
+      e = nullptr;
+    }
+  }
   ~lbm_st7_handle() {
+    drop_graphs();
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (stream) cudaStreamDestroy(stream);
@@ -71,9 +81,12 @@ namespace {
 
 St7Args st7_args(lbm_st7_handle* h, bool given) {
   St7Args a{};
-  a.src = h->g[h->cur].p;
-  a.dst = h->g[1 - h->cur].p;
+  a.g = h->g.p;
+  a.phase = h->cur;
   a.table = static_cast<const int32_t*>(h->table.p);
+  const long long bytes = (long long)(h->nq == kQ ? kQ : 6) * (h->f64 ? 8 : 4), ub = 3LL * (h->f64 ? 8 : 4);
+  a.rows = h->rows_on ? static_cast<const int32_t*>(h->rows.p) : nullptr;
+  a.ahead = prefetch_ahead(h->geo.count, bytes + ub, h->nq == kQ ? (h->rows_on ? 36 : 72) : 24);
   a.u = h->u.p;
   a.c_given = given ? h->c0.p : nullptr;
   a.n = h->geo.count;
@@ -88,6 +101,31 @@ St7Args st7_args(lbm_st7_handle* h, bool given) {
 template <typename T>
 std::vector<T> to_type(const std::vector<double>& v) {
   return std::vector<T>(v.begin(), v.end());
+}
+
+constexpr int kSoluteGraphSteps = 16;  // even: a replay leaves the phase unchanged
+
+// A chain of steps from phase c0, captured once (launched one by one, steps
+// of small solves wait on the host: 4.1 us per step at 48^3).
+lbm_status solute_graph(lbm_st7_handle* h, int c0) {
+  if (h->graph[c0]) return LBM_OK;
+  cudaGraph_t g = nullptr;
+  LBM_CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+  cudaError_t err = cudaSuccess;
+  St7Args a = st7_args(h, false);
+  for (int s = 0; s < kSoluteGraphSteps && err == cudaSuccess; s++) {
+    a.phase = (c0 + s) & 1;
+    err = st7_launch_step(h->f64, a, h->stream);
+  }
+  const cudaError_t end = cudaStreamEndCapture(h->stream, &g);
+  if (err != cudaSuccess || end != cudaSuccess) {
+    if (g) cudaGraphDestroy(g);
+    return fail(LBM_ERR_CUDA, std::string("solute graph capture: ") + cudaGetErrorString(err ? err : end));
+  }
+  const cudaError_t ie = cudaGraphInstantiate(&h->graph[c0], g, 0);
+  cudaGraphDestroy(g);
+  LBM_CUDA_TRY(ie);
+  return LBM_OK;
 }
 
 lbm_status upload_as(lbm_st7_handle* h, Mem& m, const std::vector<double>& v) {
@@ -135,7 +173,7 @@ lbm_status create_solute(const lbm_st7_params* p, const uint8_t* mask, int nx, i
   const int n = g.count, npad = g.npad;
   const size_t s = h->f64 ? 8 : 4;
   const int rows = nq == kQ ? kQ : 6;  // D3Q7 keeps only directions 1..6
-  for (auto& b : h->g) LBM_CUDA_TRY(b.alloc((size_t)rows * npad * s));
+  LBM_CUDA_TRY(h->g.alloc((size_t)rows * npad * s));
   LBM_CUDA_TRY(h->table.alloc((size_t)18 * npad * sizeof(int32_t)));
   LBM_CUDA_TRY(h->u.alloc((size_t)3 * npad * s));
   LBM_CUDA_TRY(h->c0.alloc((size_t)npad * s));
@@ -143,6 +181,18 @@ lbm_status create_solute(const lbm_st7_params* p, const uint8_t* mask, int nx, i
   LBM_CUDA_TRY(cudaMemcpyAsync(h->table.p, g.src.data(), sizeof(int32_t) * 18 * (size_t)npad, cudaMemcpyHostToDevice,
                                h->stream));
   LBM_CUDA_TRY(cudaMemcpyAsync(h->ref_of.p, g.ref_of.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, h->stream));
+  if (nq == kQ && rows_large(n, (kQ + 3LL) * (long long)s)) {
+    Mem marked;
+    int count = 0;
+    LBM_CUDA_TRY(h->rows.alloc((size_t)9 * npad * sizeof(int32_t)));
+    LBM_CUDA_TRY(marked.alloc(sizeof(int)));
+    LBM_CUDA_TRY(cudaMemsetAsync(marked.p, 0, sizeof(int), h->stream));
+    LBM_CUDA_TRY(launch_row_table(static_cast<const int32_t*>(h->table.p), npad, 0, n, static_cast<int32_t*>(h->rows.p),
+                                  static_cast<int*>(marked.p), h->stream));
+    LBM_CUDA_TRY(cudaMemcpyAsync(&count, marked.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+    h->rows_on = rows_pay(count, n);
+  }
   std::vector<double> uu((size_t)3 * npad, 0.0), cc((size_t)npad, 0.0);
   for (int x = 0; x < n; x++) {
     const int r = g.ref_of[x];
@@ -154,9 +204,8 @@ lbm_status create_solute(const lbm_st7_params* p, const uint8_t* mask, int nx, i
   lbm_status st;
   if ((st = upload_as(h.get(), h->u, uu)) != LBM_OK) return st;
   if ((st = upload_as(h.get(), h->c0, cc)) != LBM_OK) return st;
-  LBM_CUDA_TRY(cudaMemsetAsync(h->g[0].p, 0, h->g[0].bytes, h->stream));
-  St7Args a = st7_args(h.get(), true);
-  a.dst = h->g[0].p;  // the initial state is the pre-image of the first pull
+  LBM_CUDA_TRY(cudaMemsetAsync(h->g.p, 0, h->g.bytes, h->stream));
+  const St7Args a = st7_args(h.get(), true);  // the initial state is the pre-image of the first pull
   LBM_CUDA_TRY(st7_launch_init(h->f64, a, h->stream));
   LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
   *out = h.release();
@@ -215,17 +264,28 @@ lbm_status lbm_st7_set_lattice(lbm_st7_handle* h, double dx, double dt) {
   h->tau_s = h->prm.diffusivity / (c_s2 * dt) + 0.5;
   h->c2 = lat_c * lat_c;
   h->c4 = h->c2 * h->c2;
+  h->drop_graphs();
   return LBM_OK;
 }
 
 lbm_status lbm_st7_step(lbm_st7_handle* h, int nsteps) {
   if (!h || nsteps < 0) return fail(LBM_ERR_ARG, "lbm_st7_step: bad argument");
   LBM_CUDA_TRY(cudaSetDevice(h->device));
+  lbm_status st;
+  if (nsteps - (h->given ? 1 : 0) >= kSoluteGraphSteps)
+    for (int c = 0; c < 2; c++)
+      if ((st = solute_graph(h, c)) != LBM_OK) return st;
   LBM_CUDA_TRY(cudaEventRecord(h->ev0, h->stream));
-  for (int s = 0; s < nsteps; s++) {
+  for (int left = nsteps; left > 0;) {
+    if (!h->given && left >= kSoluteGraphSteps) {
+      LBM_CUDA_TRY(cudaGraphLaunch(h->graph[h->cur], h->stream));
+      left -= kSoluteGraphSteps;
+      continue;
+    }
     LBM_CUDA_TRY(st7_launch_step(h->f64, st7_args(h, h->given), h->stream));
     h->cur = 1 - h->cur;
     h->given = false;
+    left--;
   }
   LBM_CUDA_TRY(cudaEventRecord(h->ev1, h->stream));
   LBM_CUDA_TRY(cudaEventSynchronize(h->ev1));
@@ -274,8 +334,8 @@ lbm_status lbm_st7_set_state(lbm_st7_handle* h, const double* g, const double* c
   const size_t bytes = sizeof(double) * (size_t)(n + 1) * h->nq;
   LBM_CUDA_TRY(in.alloc(bytes));
   LBM_CUDA_TRY(cudaMemcpyAsync(in.p, g, bytes, cudaMemcpyHostToDevice, h->stream));
-  St7Args a = st7_args(h, true);
-  a.dst = h->g[h->cur].p;  // the buffer the next step pulls from
+  h->cur = kPull;
+  const St7Args a = st7_args(h, true);
   LBM_CUDA_TRY(st7_launch_import(h->f64, a, static_cast<const int32_t*>(h->ref_of.p), static_cast<const double*>(in.p),
                                  h->stream));
   // the first step takes C as given, like the restored rho_r of the reference

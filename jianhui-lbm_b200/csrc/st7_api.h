@@ -6,9 +6,11 @@
 namespace lbm {
 
 struct St7Args {
-  const void* src;        // [6][npad] post-collision g of the previous step
-  void* dst;              // [6][npad]
-  const int32_t* table;   // D3Q19 pull table [18][npad]; rows 0..5 used
+  void* g;                // [6][npad] or [19][npad], stepped in place (kernels_common.cuh)
+  int phase;              // Phase of the state
+  const int32_t* table;   // D3Q19 pull table [18][npad]; D3Q7: rows 0..5 used
+  const int32_t* rows;    // D3Q19: row form of the table (row_table.cuh), or null
+  int ahead;              // nodes ahead that a block prefetches into L2, 0 = none
   const void* u;          // [3][npad] advecting velocity
   const void* c_given;    // [npad] C for the first step after init, else null
   void* c_out;            // optional [npad]: C of this step's macro
@@ -23,7 +25,7 @@ cudaError_t st7_launch_step_f64(const St7Args& a, cudaStream_t st);  // st7_fait
 cudaError_t st19_launch_step_f64(const St7Args& a, cudaStream_t st);  // st7_faithful.cu, -fmad=false
 cudaError_t st7_launch_conc(bool f64, const St7Args& a, double* out, cudaStream_t st);
 cudaError_t st7_launch_init(bool f64, const St7Args& a, cudaStream_t st);
-// a.src: the state to export; a.dst: the buffer the next step pulls from
+// the imported (or initial) state is a kPull state
 cudaError_t st7_launch_export(bool f64, const St7Args& a, const int32_t* ref_of, double* out, cudaStream_t st);
 cudaError_t st7_launch_import(bool f64, const St7Args& a, const int32_t* ref_of, const double* in, cudaStream_t st);
 

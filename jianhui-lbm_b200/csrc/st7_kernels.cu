@@ -5,11 +5,11 @@
 // C/6 (1 + 3 e.u) with tau_s (ST7:1464-1471), push streaming with halfway
 // bounce-back (ST7:1475-1528) and C = sum of the six g (ST7:1619-1633).
 //
-// Here: g is stored post-collision as six rows [6][npad] (directions 1..6,
-// which are also directions 1..6 of the D3Q19 pull table), pulled through
-// those six table rows: a table entry q'*npad + m of a D3Q7 direction has
-// q' in 1..6, so the row-6 storage index is entry - npad.  One thread per
-// node; 2*6*s + 6*4 + 3*s bytes per update.  The step kernel lives in
+// Here: g is stored as six rows [6][npad] (directions 1..6, which are also
+// directions 1..6 of the D3Q19 pull table), stepped in place through those
+// six table rows: a table entry q'*npad + m of a D3Q7 direction has q' in
+// 1..6, so the row-6 storage index is entry - npad.  One thread per node;
+// 2*6*s + 3*s bytes per update and 6*4 more on every second one.  The step kernel lives in
 // st7_kernels.cuh; its FP64 instantiation is built in st7_faithful.cu with
 // -fmad=false (the reference's unfused arithmetic), this file keeps FMA
 // contraction for the FP32 path.
@@ -19,18 +19,23 @@ namespace lbm {
 
 namespace {
 
+// Slot of node x's g_q in the state's phase.
+__device__ __forceinline__ size_t st7_slot(const St7Args& a, int x, int q) {
+  return (size_t)(state_slot(a.phase, a.table, a.npad, x, q) - a.npad);
+}
+
 // C of every node from the pulled g (the macro step), internal order.
 template <typename T>
 __global__ void st7_conc_kernel(St7Args a, double* __restrict__ out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= a.n) return;
-  const T* __restrict__ src = static_cast<const T*>(a.src);
+  const T* __restrict__ src = static_cast<const T*>(a.g);
   T C = T(0);
   if (a.c_given) {
     C = static_cast<const T*>(a.c_given)[x];
   } else {
 #pragma unroll
-    for (int q = 1; q < 7; q++) C = C + src[a.table[(size_t)(q - 1) * a.npad + x] - (size_t)a.npad];
+    for (int q = 1; q < 7; q++) C = C + src[st7_slot(a, x, q)];
   }
   out[x] = (double)C;
 }
@@ -45,13 +50,11 @@ __global__ void st7_init_kernel(St7Args a) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= a.n) return;
   const T C = static_cast<const T*>(a.c_given)[x];
-  const size_t npad = (size_t)a.npad;
-  T* __restrict__ g = static_cast<T*>(a.dst);
+  T* __restrict__ g = static_cast<T*>(a.g);
   const T eu = T(0);
 #pragma unroll
   for (int q = 1; q < 7; q++) {
-    const size_t s = a.table[(size_t)(q - 1) * npad + x] - npad;
-    g[s] = T(1.0 / 6.0) * C * (T(1) + T(3) * eu);
+    g[st7_slot(a, x, q)] = T(1.0 / 6.0) * C * (T(1) + T(3) * eu);
   }
 }
 
@@ -61,29 +64,27 @@ template <typename T>
 __global__ void st7_export_kernel(St7Args a, const int32_t* __restrict__ ref_of, double* __restrict__ out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= a.n) return;
-  const T* __restrict__ src = static_cast<const T*>(a.src);
-  const size_t npad = (size_t)a.npad;
+  const T* __restrict__ src = static_cast<const T*>(a.g);
   double* row = out + (size_t)ref_of[x] * 7;
   row[0] = 0.0;
 #pragma unroll
-  for (int q = 1; q < 7; q++) row[q] = (double)src[a.table[(size_t)(q - 1) * npad + x] - npad];
+  for (int q = 1; q < 7; q++) row[q] = (double)src[st7_slot(a, x, q)];
 }
 
 template <typename T>
 __global__ void st7_import_kernel(St7Args a, const int32_t* __restrict__ ref_of, const double* __restrict__ in) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= a.n) return;
-  T* __restrict__ dst = static_cast<T*>(a.dst);
-  const size_t npad = (size_t)a.npad;
+  T* __restrict__ dst = static_cast<T*>(a.g);
   const double* row = in + (size_t)ref_of[x] * 7;
 #pragma unroll
-  for (int q = 1; q < 7; q++) dst[a.table[(size_t)(q - 1) * npad + x] - npad] = (T)row[q];
+  for (int q = 1; q < 7; q++) dst[st7_slot(a, x, q)] = (T)row[q];
 }
 
 // D3Q19 (the solute program with 19 directions): g is [19][npad]; a node's
-// pulled value of storage row q is g[x] for q = 0, else g[table[q-1][x]].
+// rest population is at x, the others at their slots of the state's phase.
 __device__ __forceinline__ size_t st19_slot(const St7Args& a, int x, int q) {
-  return q == 0 ? (size_t)x : (size_t)a.table[(size_t)(q - 1) * a.npad + x];
+  return q == 0 ? (size_t)x : (size_t)state_slot(a.phase, a.table, a.npad, x, q);
 }
 
 // C = sum of the pulled g in the program's direction order (ST19:1636-1650).
@@ -91,7 +92,7 @@ template <typename T>
 __global__ void st19_conc_kernel(St7Args a, double* __restrict__ out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= a.n) return;
-  const T* __restrict__ src = static_cast<const T*>(a.src);
+  const T* __restrict__ src = static_cast<const T*>(a.g);
   T C = T(0);
   if (a.c_given) {
     C = static_cast<const T*>(a.c_given)[x];
@@ -109,7 +110,7 @@ __global__ void st19_init_kernel(St7Args a) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= a.n) return;
   const T C = static_cast<const T*>(a.c_given)[x];
-  T* __restrict__ g = static_cast<T*>(a.dst);
+  T* __restrict__ g = static_cast<T*>(a.g);
 #pragma unroll
   for (int q = 0; q < kQ; q++) g[st19_slot(a, x, q)] = T(weight(q)) * C * (T(1) + T(3) * T(0));
 }
@@ -120,7 +121,7 @@ template <typename T>
 __global__ void st19_export_kernel(St7Args a, const int32_t* __restrict__ ref_of, double* __restrict__ out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= a.n) return;
-  const T* __restrict__ src = static_cast<const T*>(a.src);
+  const T* __restrict__ src = static_cast<const T*>(a.g);
   double* row = out + (size_t)ref_of[x] * kQ;
 #pragma unroll
   for (int k = 0; k < kQ; k++) row[k] = (double)src[st19_slot(a, x, cg::row(k))];
@@ -130,7 +131,7 @@ template <typename T>
 __global__ void st19_import_kernel(St7Args a, const int32_t* __restrict__ ref_of, const double* __restrict__ in) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= a.n) return;
-  T* __restrict__ dst = static_cast<T*>(a.dst);
+  T* __restrict__ dst = static_cast<T*>(a.g);
   const double* row = in + (size_t)ref_of[x] * kQ;
 #pragma unroll
   for (int k = 0; k < kQ; k++) dst[st19_slot(a, x, cg::row(k))] = (T)row[k];

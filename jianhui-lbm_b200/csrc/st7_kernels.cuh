@@ -7,26 +7,56 @@
 // six g (ST7:1619-1633).  Here g is pulled through rows 1..6 of the flow's
 // pull table (a D3Q7 direction q is D3Q19 direction q, so a table entry
 // q'*npad + m has q' in 1..6 and its row-6 storage index is entry - npad).
+//
+// Both solutes step in place (kernels_common.cuh): every second step works on
+// the node's own slots and reads no table, and a solve needs one array.  They
+// are bound by their bytes; a block prefetches the rows of nodes half a wave
+// ahead into L2 when the solve exceeds it, as the flow step does.
 #pragma once
 
 #include "cg_basis.h"
+#include "kernels_common.cuh"
+#include "row_table.cuh"
 #include "st7_api.h"
 
 namespace lbm {
 namespace st7_detail {
 
-template <typename T, bool GIVEN>
+// Prefetches the g (ROWS_G rows), u and table rows (TABLE_ROWS) of the 256
+// nodes `ahead` after the block's into L2, one 128-byte line per turn.
+template <int ROWS_G, int TABLE_ROWS, typename T>
+__device__ __forceinline__ void prefetch_solute(const St7Args& a, const int32_t* table) {
+  const int p = blockIdx.x * 256 + a.ahead;
+  if (a.ahead == 0 || p + 256 > a.npad) return;
+  constexpr int kLines = 256 * (int)sizeof(T) / 128;
+  const T* g = static_cast<const T*>(a.g);
+  const T* u = static_cast<const T*>(a.u);
+  for (int i = threadIdx.x; i < (ROWS_G + 3) * kLines + TABLE_ROWS * 8; i += 256) {
+    const int j = i - (ROWS_G + 3) * kLines, row = i / kLines;
+    const char* line =
+        j >= 0 ? reinterpret_cast<const char*>(table + (size_t)(j / 8) * a.npad + p) + (j % 8) * 128
+               : reinterpret_cast<const char*>((row < ROWS_G ? g + (size_t)row * a.npad : u + (size_t)(row - ROWS_G) * a.npad) + p) +
+                     (i % kLines) * 128;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(line));
+  }
+}
+
+template <typename T, bool GIVEN, bool LOCAL>
 __global__ void __launch_bounds__(256) st7_step_kernel(St7Args a) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  prefetch_solute<6, LOCAL ? 0 : 6, T>(a, a.table);
   if (x >= a.n) return;
-  const T* __restrict__ src = static_cast<const T*>(a.src);
-  T* __restrict__ dst = static_cast<T*>(a.dst);
+  T* pop = static_cast<T*>(a.g);
   const T* __restrict__ u = static_cast<const T*>(a.u);
-  const size_t npad = (size_t)a.npad;
+  const int npad = a.npad;
   T g[7];
+  int32_t slot[7];  // slot[q] holds g_q and takes g*_opp(q)
   g[0] = T(0);
 #pragma unroll
-  for (int q = 1; q < 7; q++) g[q] = __ldg(src + (__ldg(a.table + (size_t)(q - 1) * npad + x) - npad));
+  for (int q = 1; q < 7; q++) {
+    slot[q] = LOCAL ? (opp(q) - 1) * npad + x : __ldg(a.table + (size_t)(q - 1) * npad + x) - npad;
+    g[q] = pop[slot[q]];
+  }
   T C;
   if (GIVEN) {
     C = static_cast<const T*>(a.c_given)[x];
@@ -36,13 +66,13 @@ __global__ void __launch_bounds__(256) st7_step_kernel(St7Args a) {
     for (int q = 1; q < 7; q++) C = C + g[q];
   }
   if (a.c_out) static_cast<T*>(a.c_out)[x] = C;
-  const T ux = u[x], uy = u[npad + x], uz = u[2 * npad + x];
+  const T ux = u[x], uy = u[npad + x], uz = u[2 * (size_t)npad + x];
   const T tau = T(a.tau_s);
 #pragma unroll
   for (int q = 1; q < 7; q++) {
     const T eu = T(cx(q)) * ux + T(cy(q)) * uy + T(cz(q)) * uz;
     const T nv = g[q] - (g[q] - T(1.0 / 6.0) * C * (T(1) + T(3) * eu)) / tau;
-    dst[(size_t)(q - 1) * npad + x] = nv;
+    pop[slot[opp(q)]] = nv;
   }
 }
 
@@ -74,18 +104,37 @@ __device__ __forceinline__ double st19_edot(double ux, double uy, double uz) {
 // UNIT: the default lattice (lat_c = 1), where the program's divisions by
 // c2 = c4 = 1 are exact and left out; otherwise (lattice_v, ST19:1259-1268)
 // 3 e.u / c2, 4.5 (e.u)^2 / c4 and 1.5 u.u / c2 as the program writes them.
-template <typename T, bool GIVEN, bool UNIT>
+// SLOTS: 0 the node's own slots (a kLocal state), 1 the int32 table, 2 its
+// row form.
+template <typename T, bool GIVEN, bool UNIT, int SLOTS>
 __global__ void __launch_bounds__(256) st19_step_kernel(St7Args a) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  prefetch_solute<kQ, SLOTS == 1 ? 18 : SLOTS == 2 ? 9 : 0, T>(a, SLOTS == 2 ? a.rows : a.table);
   if (x >= a.n) return;
-  const T* __restrict__ src = static_cast<const T*>(a.src);
-  T* __restrict__ dst = static_cast<T*>(a.dst);
+  T* pop = static_cast<T*>(a.g);
+  __shared__ int32_t keep[SLOTS ? kQ - 1 : 1][SLOTS ? 256 : 1];  // each thread's own slots, for its stores
   const T* __restrict__ u = static_cast<const T*>(a.u);
   const size_t npad = (size_t)a.npad;
   T g[kQ];
-  g[0] = __ldg(src + x);
+  g[0] = pop[x];
+  if constexpr (SLOTS == 0) {
 #pragma unroll
-  for (int q = 1; q < kQ; q++) g[q] = __ldg(src + __ldg(a.table + (size_t)(q - 1) * npad + x));
+    for (int q = 1; q < kQ; q++) g[q] = pop[opp(q) * npad + x];
+  } else {
+    int32_t slot[kQ];
+    if constexpr (SLOTS == 2) {
+      row_slots(a.rows, a.table, a.npad, x, slot);
+    } else {
+#pragma unroll
+      for (int q = 1; q < kQ; q++) slot[q] = __ldg(a.table + (size_t)(q - 1) * npad + x);
+    }
+#pragma unroll
+    for (int q = 1; q < kQ; q++) {
+      g[q] = pop[slot[q]];
+      keep[q - 1][threadIdx.x] = slot[q];
+    }
+    asm volatile("" ::: "memory");  // the slots are read again from where they were kept
+  }
   T C;
   if (GIVEN) {
     C = static_cast<const T*>(a.c_given)[x];
@@ -102,7 +151,7 @@ __global__ void __launch_bounds__(256) st19_step_kernel(St7Args a) {
     const T eq = UNIT ? T(weight(0)) * C * (T(1) - T(1.5) * uu)
                       : T(weight(0)) * C * (T(1) + T(3) * T(0) / T(a.c2) + T(4.5) * T(0) * T(0) / T(a.c4) -
                                             T(1.5) * uu / T(a.c2));
-    dst[x] = g[0] - (g[0] - eq) / tau;
+    pop[x] = g[0] - (g[0] - eq) / tau;
   }
 #pragma unroll
   for (int q = 1; q < kQ; q++) {
@@ -128,31 +177,42 @@ __global__ void __launch_bounds__(256) st19_step_kernel(St7Args a) {
     const T eq = UNIT ? T(weight(q)) * C * (T(1) + T(3) * eu + T(4.5) * eu * eu - T(1.5) * uu)
                       : T(weight(q)) * C * (T(1) + T(3) * eu / T(a.c2) + T(4.5) * eu * eu / T(a.c4) -
                                             T(1.5) * uu / T(a.c2));
-    dst[(size_t)q * npad + x] = g[q] - (g[q] - eq) / tau;
+    pop[SLOTS == 0 ? q * npad + x : (size_t)keep[opp(q) - 1][threadIdx.x]] = g[q] - (g[q] - eq) / tau;
   }
+}
+
+template <typename T, bool UNIT>
+void launch_step19_unit(const St7Args& a, int grid, cudaStream_t st) {
+  if (a.c_given != nullptr)
+    st19_step_kernel<T, true, UNIT, 1><<<grid, 256, 0, st>>>(a);
+  else if (a.phase == kLocal)
+    st19_step_kernel<T, false, UNIT, 0><<<grid, 256, 0, st>>>(a);
+  else if (a.rows != nullptr)
+    st19_step_kernel<T, false, UNIT, 2><<<grid, 256, 0, st>>>(a);
+  else
+    st19_step_kernel<T, false, UNIT, 1><<<grid, 256, 0, st>>>(a);
 }
 
 template <typename T>
 cudaError_t launch_step19(const St7Args& a, cudaStream_t st) {
   if (a.n == 0) return cudaSuccess;
+  if (a.c_given != nullptr && a.phase == kLocal) return cudaErrorInvalidValue;  // a given state is a kPull state
   const int g = (a.n + 255) / 256;
-  const bool unit = a.c2 == 1.0 && a.c4 == 1.0;
-  if (a.c_given != nullptr)
-    unit ? st19_step_kernel<T, true, true><<<g, 256, 0, st>>>(a) : st19_step_kernel<T, true, false><<<g, 256, 0, st>>>(a);
-  else
-    unit ? st19_step_kernel<T, false, true><<<g, 256, 0, st>>>(a)
-         : st19_step_kernel<T, false, false><<<g, 256, 0, st>>>(a);
+  a.c2 == 1.0 && a.c4 == 1.0 ? launch_step19_unit<T, true>(a, g, st) : launch_step19_unit<T, false>(a, g, st);
   return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_step(const St7Args& a, cudaStream_t st) {
   if (a.n == 0) return cudaSuccess;
+  if (a.c_given != nullptr && a.phase == kLocal) return cudaErrorInvalidValue;
   const int g = (a.n + 255) / 256;
   if (a.c_given != nullptr)
-    st7_step_kernel<T, true><<<g, 256, 0, st>>>(a);
+    st7_step_kernel<T, true, false><<<g, 256, 0, st>>>(a);
+  else if (a.phase == kLocal)
+    st7_step_kernel<T, false, true><<<g, 256, 0, st>>>(a);
   else
-    st7_step_kernel<T, false><<<g, 256, 0, st>>>(a);
+    st7_step_kernel<T, false, false><<<g, 256, 0, st>>>(a);
   return cudaGetLastError();
 }
 
