@@ -110,6 +110,7 @@ struct Pool {
   int block = 256, grid = 0;
   int ordering = LBM_ORDER_REFERENCE;
   double fp16_scale = 1.0;
+  Buf x_fields;  // field export
   Buf pop, table, rows, tile_inst, inst, state, partials, active_tiles, n_active, work, slot_off;
   SetupScratch setup;
   std::vector<InstParams> h_inst;
@@ -199,6 +200,7 @@ struct Pool {
     LBM_CUDA_TRY(cudaMemcpyAsync(state.p, h_state, (size_t)nslots * sizeof(InstState), cudaMemcpyHostToDevice,
                                  stream));
     grid = batch_step_grid(ntiles, block);
+    LBM_CUDA_TRY(stage_pool_prime());  // the process's staging memory for field reads
     return LBM_OK;
   }
 
@@ -289,6 +291,20 @@ struct Pool {
                                  cudaMemcpyHostToDevice, stream));
     // the pinned h_state row is the copy source: wait before it can change
     LBM_CUDA_TRY(cudaStreamSynchronize(stream));
+    return LBM_OK;
+  }
+
+  // The initial state of a placed solve again (its table and constants stand);
+  // the caller waits for the stream before h_state can change.
+  lbm_status restart(int slot) {
+    const InstParams& ip = h_inst[slot];
+    LBM_CUDA_TRY(launch_batch_init(kind, pop.p, cur, table.as<int32_t>(), cap, ip.begin, ip.end - ip.begin, ip, stream));
+    InstState st{};
+    st.active = 1;
+    st.fresh = 1;
+    h_state[slot] = st;
+    LBM_CUDA_TRY(cudaMemcpyAsync(state.as<InstState>() + slot, &h_state[slot], sizeof(InstState),
+                                 cudaMemcpyHostToDevice, stream));
     return LBM_OK;
   }
 
@@ -428,24 +444,22 @@ struct Pool {
     const Job& j = *slot_job[slot];
     const InstParams& ip = h_inst[slot];
     const int n = j.geo.count;
-    Buf ref, r, v;
-    LBM_CUDA_TRY(ref.alloc(sizeof(int32_t) * n));
-    LBM_CUDA_TRY(r.alloc(sizeof(double) * (n + 1)));
-    LBM_CUDA_TRY(v.alloc(sizeof(double) * 3 * (n + 1)));
-    std::vector<int32_t> iota;
-    const int32_t* ref_src = j.geo.ref_of.data();
-    if (j.geo.ref_of.empty()) {  // reference order: internal index p is reference id p + 1
-      iota.resize(n);
-      for (int p = 0; p < n; p++) iota[p] = p + 1;
-      ref_src = iota.data();
+    // rho [n + 1] and u [n + 1][3]; kept between calls, grown to the largest
+    // instance read
+    const size_t rows = (size_t)n + 1, need = 4 * rows * sizeof(double);
+    if (x_fields.bytes < need) LBM_CUDA_TRY(x_fields.alloc(need));
+    double* r = x_fields.as<double>();
+    double* v = r + rows;
+    Buf ref;  // reference order: internal index p is reference id p + 1
+    if (!j.geo.ref_of.empty()) {
+      LBM_CUDA_TRY(ref.alloc(sizeof(int32_t) * n));
+      LBM_CUDA_TRY(cudaMemcpyAsync(ref.p, j.geo.ref_of.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream));
     }
-    LBM_CUDA_TRY(cudaMemcpyAsync(ref.p, ref_src, sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream));
-    LBM_CUDA_TRY(cudaMemsetAsync(r.p, 0, r.bytes, stream));
-    LBM_CUDA_TRY(cudaMemsetAsync(v.p, 0, v.bytes, stream));
+    LBM_CUDA_TRY(cudaMemsetAsync(r, 0, need, stream));
     LBM_CUDA_TRY(launch_batch_export_macro(kind, pop.p, slot_phase[slot], table.as<int32_t>(), cap, ip.begin, n,
-                                           ref.as<int32_t>(), ip, r.as<double>(), v.as<double>(), stream));
-    if (rho) LBM_CUDA_TRY(cudaMemcpyAsync(rho, r.p, r.bytes, cudaMemcpyDeviceToHost, stream));
-    if (u) LBM_CUDA_TRY(cudaMemcpyAsync(u, v.p, v.bytes, cudaMemcpyDeviceToHost, stream));
+                                           ref.as<int32_t>(), ip, r, v, stream));
+    if (rho) LBM_CUDA_TRY(d2h_staged(rho, r, rows * sizeof(double), stream));
+    if (u) LBM_CUDA_TRY(d2h_staged(u, v, 3 * rows * sizeof(double), stream));
     LBM_CUDA_TRY(cudaStreamSynchronize(stream));
     return LBM_OK;
   }
@@ -531,10 +545,11 @@ lbm_status batch_reset(lbm_batch* b) {
   Pool& P = b->pool;
   P.cur = kPull;
   for (int i = 0; i < b->n; i++) {
-    lbm_status st = P.place(i, b->first_tile[i]);
+    lbm_status st = P.restart(i);
     if (st != LBM_OK) return st;
     P.slot_phase[i] = kPull;
   }
+  LBM_CUDA_TRY(cudaStreamSynchronize(P.stream));
   return LBM_OK;
 }
 

@@ -291,7 +291,7 @@ __global__ void batch_export_macro_kernel(const typename Traits<K>::T* __restric
   split_pairs(f, ps);
   A drho, rho, ux, uy, uz;
   macro_dev<A>(f, ps, A(0.5f * ip.g[0]), A(0.5f * ip.g[1]), A(0.5f * ip.g[2]), drho, rho, ux, uy, uz);
-  const int r = ref_of[i];
+  const int r = ref_of ? ref_of[i] : i + 1;
   if (rho_ref) rho_ref[r] = rho;
   if (u_ref) {
     u_ref[(size_t)r * 3 + 0] = ux;

@@ -82,6 +82,7 @@ struct lbm_cg_handle {
   bool colour_done = false;
   double rand_sat = -1.0;                 // ini_Sat: threshold of the random phase faces
   unsigned long long rand_seed = 0;       // seed of the random phase faces
+  Dev x_fields;                           // field export, kept between calls
   Dev zero_sigma;                         // zero-surface-tension layer flags, or none
   int nface = 0;
   std::vector<double> psi0;               // initial phase per node (internal order), as read
@@ -537,6 +538,7 @@ lbm_status lbm_cg_create_bc(const lbm_cg_params* p, const lbm_boundary* bc, cons
     LBM_CUDA_TRY(cudaMemcpyAsync(h->rho_b.p, c.data(), sizeof(float) * npad, cudaMemcpyHostToDevice, h->stream));
     LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
   }
+  LBM_CUDA_TRY(stage_pool_prime());  // the process's staging memory for field reads
   if (h->gr.p) LBM_CUDA_TRY(cudaMemsetAsync(h->gr.p, 0, h->gr.bytes, h->stream));
   if (h->gb.p) LBM_CUDA_TRY(cudaMemsetAsync(h->gb.p, 0, h->gb.bytes, h->stream));
   if (h->rec.p) LBM_CUDA_TRY(cudaMemsetAsync(h->rec.p, 0, h->rec.bytes, h->stream));
@@ -643,36 +645,27 @@ lbm_status lbm_cg_get_fields(lbm_cg_handle* h, double* rho, double* u, double* p
   lbm_status st = cg_check(h);
   if (st != LBM_OK) return st;
   const int n = h->geo.count, npad = h->geo.npad;
-  Dev rint, uint_, rref, uref;
-  LBM_CUDA_TRY(rint.alloc((size_t)npad * sizeof(double)));
-  LBM_CUDA_TRY(uint_.alloc((size_t)3 * npad * sizeof(double)));
-  LBM_CUDA_TRY(rref.alloc((size_t)(n + 1) * sizeof(double)));
-  LBM_CUDA_TRY(uref.alloc((size_t)(n + 1) * 3 * sizeof(double)));
+  // internal-order rho and u, then the fields in the reference's order; kept
+  // between calls, and filled and ordered on the device: the host only copies
+  const size_t rows = (size_t)n + 1;
+  const size_t need = ((size_t)4 * npad + 4 * rows) * sizeof(double);
+  if (h->x_fields.bytes != need) LBM_CUDA_TRY(h->x_fields.alloc(need));
+  double* rint = h->x_fields.as<double>();
+  double* uint_ = rint + npad;
+  double* rref = uint_ + (size_t)3 * npad;
+  double* uref = rref + rows;
   double r[8];
-  if ((st = cg_reduce_raw(h, r, rint.as<double>(), uint_.as<double>())) != LBM_OK) return st;
-  LBM_CUDA_TRY(cudaMemsetAsync(rref.p, 0, rref.bytes, h->stream));
-  LBM_CUDA_TRY(cudaMemsetAsync(uref.p, 0, uref.bytes, h->stream));
-  LBM_CUDA_TRY(launch_export_macro(rint.as<double>(), uint_.as<double>(), h->ref_of.as<int32_t>(), n, npad,
-                                   rref.as<double>(), uref.as<double>(), h->stream));
-  if (rho) LBM_CUDA_TRY(cudaMemcpyAsync(rho, rref.p, rref.bytes, cudaMemcpyDeviceToHost, h->stream));
-  if (u) LBM_CUDA_TRY(cudaMemcpyAsync(u, uref.p, uref.bytes, cudaMemcpyDeviceToHost, h->stream));
-  // scalar fields: internal order equals reference order - 1 for this solver
-  std::vector<double> tmp(npad);
-  std::vector<float> tmpf(npad);
+  if ((st = cg_reduce_raw(h, r, rint, uint_)) != LBM_OK) return st;
+  LBM_CUDA_TRY(cudaMemsetAsync(rref, 0, 4 * rows * sizeof(double), h->stream));
+  LBM_CUDA_TRY(launch_export_macro(rint, uint_, h->ref_of.as<int32_t>(), n, npad, rref, uref, h->stream));
+  if (rho) LBM_CUDA_TRY(d2h_staged(rho, rref, rows * sizeof(double), h->stream));
+  if (u) LBM_CUDA_TRY(d2h_staged(u, uref, 3 * rows * sizeof(double), h->stream));
   double* outs[3] = {psi, rho_r, rho_b};
-  Dev* srcs[3] = {&h->psi, &h->rho_r, &h->rho_b};
+  const Dev* srcs[3] = {&h->psi, &h->rho_r, &h->rho_b};
   for (int i = 0; i < 3; i++) {
     if (!outs[i]) continue;
-    if (h->f64) {
-      LBM_CUDA_TRY(cudaMemcpyAsync(tmp.data(), srcs[i]->p, sizeof(double) * npad, cudaMemcpyDeviceToHost, h->stream));
-      LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    } else {
-      LBM_CUDA_TRY(cudaMemcpyAsync(tmpf.data(), srcs[i]->p, sizeof(float) * npad, cudaMemcpyDeviceToHost, h->stream));
-      LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
-      for (int x = 0; x < npad; x++) tmp[x] = tmpf[x];
-    }
-    outs[i][0] = 0.0;
-    for (int x = 0; x < n; x++) outs[i][h->geo.ref_of[x]] = tmp[x];
+    LBM_CUDA_TRY(launch_export_scalar(h->f64, srcs[i]->p, h->ref_of.as<int32_t>(), n, rref, h->stream));
+    LBM_CUDA_TRY(d2h_staged(outs[i], rref, rows * sizeof(double), h->stream));
   }
   LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
   return LBM_OK;
@@ -689,8 +682,7 @@ lbm_status lbm_cg_get_populations(lbm_cg_handle* h, double* f) {
   LBM_CUDA_TRY(cudaMemsetAsync(o.p, 0, o.bytes, h->stream));
   LBM_CUDA_TRY(cg_export_f(h->f64, h->f[h->cur].p, h->table.as<int32_t>(), h->ref_of.as<int32_t>(), n, h->geo.npad,
                            o.as<double>(), h->stream));
-  LBM_CUDA_TRY(cudaMemcpyAsync(f, o.p, o.bytes, cudaMemcpyDeviceToHost, h->stream));
-  LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+  LBM_CUDA_TRY(d2h_staged(f, o.p, o.bytes, h->stream));
   return LBM_OK;
 }
 

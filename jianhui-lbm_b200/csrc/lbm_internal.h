@@ -363,6 +363,8 @@ cudaError_t launch_import_macro(Store kind, void* rho, void* u, const int32_t* r
                                 const double* rho_in, const double* u_in, cudaStream_t st);
 cudaError_t launch_export_macro(const double* rho_int, const double* u_int, const int32_t* ref_of, int n,
                                 int npad, double* rho_ref, double* u_ref, cudaStream_t st);
+// out[0] = 0, out[ref_of[p]] = src[p] as double (FP64 or FP32 source)
+cudaError_t launch_export_scalar(bool f64, const void* src, const int32_t* ref_of, int n, double* out, cudaStream_t st);
 cudaError_t set_mi_constant(const double* mi361, cudaStream_t st);
 // True when M^-1 has the zero / power-of-two pattern the bit-exact FP64
 // kernel was compiled for (mi_pattern.h, generated from mrt.cpp).

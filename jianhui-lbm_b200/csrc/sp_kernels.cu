@@ -569,6 +569,25 @@ cudaError_t launch_export_macro(const double* rho_int, const double* u_int, cons
   return cudaGetLastError();
 }
 
+// One scalar field in the reference's order, row 0 zero.
+template <typename T>
+__global__ void export_scalar_kernel(const T* __restrict__ src, const int32_t* __restrict__ ref_of, int n,
+                                     double* __restrict__ out) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p == 0) out[0] = 0.0;
+  if (p < n) out[ref_of[p]] = (double)src[p];
+}
+
+cudaError_t launch_export_scalar(bool f64, const void* src, const int32_t* ref_of, int n, double* out,
+                                 cudaStream_t st) {
+  const int g = n > 0 ? (n + 255) / 256 : 1;
+  if (f64)
+    export_scalar_kernel<<<g, 256, 0, st>>>(static_cast<const double*>(src), ref_of, n, out);
+  else
+    export_scalar_kernel<<<g, 256, 0, st>>>(static_cast<const float*>(src), ref_of, n, out);
+  return cudaGetLastError();
+}
+
 struct Feq19 {
   double v[kQ];
 };

@@ -52,7 +52,7 @@ struct lbm_st7_handle {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   Geometry geo;
-  Mem g, table, rows, u, c0, ref_of;
+  Mem g, table, rows, u, c0, ref_of, x_conc;
   int cur = kPull;  // phase of g
   bool rows_on = false;
   // captured step chains, one per starting phase
@@ -207,6 +207,7 @@ lbm_status create_solute(const lbm_st7_params* p, const uint8_t* mask, int nx, i
   LBM_CUDA_TRY(cudaMemsetAsync(h->g.p, 0, h->g.bytes, h->stream));
   const St7Args a = st7_args(h.get(), true);  // the initial state is the pre-image of the first pull
   LBM_CUDA_TRY(st7_launch_init(h->f64, a, h->stream));
+  LBM_CUDA_TRY(stage_pool_prime());  // the process's staging memory for field reads
   LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
   *out = h.release();
   return LBM_OK;
@@ -300,14 +301,13 @@ lbm_status lbm_st7_get_concentration(lbm_st7_handle* h, double* c) {
   if (!h || !c) return fail(LBM_ERR_ARG, "lbm_st7_get_concentration: bad argument");
   LBM_CUDA_TRY(cudaSetDevice(h->device));
   const int n = h->geo.count;
-  Mem out;
-  LBM_CUDA_TRY(out.alloc(sizeof(double) * (size_t)h->geo.npad));
-  LBM_CUDA_TRY(st7_launch_conc(h->f64, st7_args(h, h->given), static_cast<double*>(out.p), h->stream));
-  std::vector<double> tmp(n);
-  LBM_CUDA_TRY(cudaMemcpyAsync(tmp.data(), out.p, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream));
-  LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
-  c[0] = 0.0;
-  for (int x = 0; x < n; x++) c[h->geo.ref_of[x]] = tmp[x];
+  const size_t need = sizeof(double) * ((size_t)h->geo.npad + n + 1);
+  if (h->x_conc.bytes != need) LBM_CUDA_TRY(h->x_conc.alloc(need));  // kept between calls
+  double* inner = static_cast<double*>(h->x_conc.p);
+  double* ref = inner + h->geo.npad;
+  LBM_CUDA_TRY(st7_launch_conc(h->f64, st7_args(h, h->given), inner, h->stream));
+  LBM_CUDA_TRY(launch_export_scalar(true, inner, static_cast<const int32_t*>(h->ref_of.p), n, ref, h->stream));
+  LBM_CUDA_TRY(d2h_staged(c, ref, sizeof(double) * ((size_t)n + 1), h->stream));
   return LBM_OK;
 }
 
@@ -321,8 +321,7 @@ lbm_status lbm_st7_get_populations(lbm_st7_handle* h, double* g) {
   LBM_CUDA_TRY(cudaMemsetAsync(out.p, 0, bytes, h->stream));
   LBM_CUDA_TRY(st7_launch_export(h->f64, st7_args(h, false), static_cast<const int32_t*>(h->ref_of.p),
                                  static_cast<double*>(out.p), h->stream));
-  LBM_CUDA_TRY(cudaMemcpyAsync(g, out.p, bytes, cudaMemcpyDeviceToHost, h->stream));
-  LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+  LBM_CUDA_TRY(d2h_staged(g, out.p, bytes, h->stream));
   return LBM_OK;
 }
 
