@@ -160,17 +160,14 @@ struct lbm_handle {
   int last_p = -1;
   double fp16_scale = 1.0;
   double last_ms = 0.0;
-  // captured step chains, one per starting phase
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};
-  int graph_steps = 0;
+  cudaGraphExec_t graph = nullptr;  // captured step chain, from a kPull state
   // false when the layout was built on the device and the host copies of the
   // compaction / node order (needed only for exports and re-layouts) are not
   // built yet
   bool host_geo = true;
 
   ~lbm_handle() {
-    for (auto& g : graph)
-      if (g) cudaGraphExecDestroy(g);
+    if (graph) cudaGraphExecDestroy(graph);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (ev_fork) cudaEventDestroy(ev_fork);
@@ -180,11 +177,8 @@ struct lbm_handle {
   }
   size_t mac_bytes() const { return (kind == Store::F64 || kind == Store::F64D) ? 8 : 4; }
   void drop_graphs() {
-    for (auto& g : graph)
-      if (g) {
-        cudaGraphExecDestroy(g);
-        g = nullptr;
-      }
+    if (graph) cudaGraphExecDestroy(graph);
+    graph = nullptr;
   }
 };
 
@@ -387,6 +381,7 @@ StepArgs step_args(lbm_handle* h, bool write) {
   a.s_v = h->mrt.s_v;
   a.s_o = h->mrt.s_o;
   a.fp16_scale = h->fp16_scale;
+  a.fp16_inv = (float)(1.0 / h->fp16_scale);
   const int n = h->geo.count;
   a.n_main = h->bc.active ? h->bc.n_main : n;
   if (h->ct_ok && h->ct_on) {
@@ -468,16 +463,21 @@ lbm_status one_step(lbm_handle* h, bool write) {
 
 constexpr int kGraphSteps = 16;  // even: a replay leaves the phase unchanged
 
+// The chain of kGraphSteps steps from a kPull state (a caller in the other
+// phase steps once first: capturing and instantiating a second chain costs
+// more than that step).
 lbm_status ensure_graph(lbm_handle* h) {
-  if (h->graph[h->cur]) return LBM_OK;
+  if (h->graph) return LBM_OK;
   cudaGraph_t g = nullptr;
-  const int cur0 = h->cur;
   LBM_CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  int c = cur0;
+  int c = kPull;
   cudaError_t err = cudaSuccess;
+  // (with faces the steps are joined by events)
+  const bool chain = !h->bc.active && chain_pays(h->geo.count, h->mac_bytes() == 8 ? 148 * 256 : 148 * 1024);
   for (int s = 0; s < kGraphSteps && err == cudaSuccess; s++) {
     StepArgs a = step_args(h, false);
     a.phase = c;
+    a.chained = s > 0 && chain;
     a.rho_in = a.u_in = nullptr;
     if (h->bc.active) a.snap_dst = h->snap[1 - c].as<double>();
     err = launch_full_step(h, a, c);
@@ -489,42 +489,34 @@ lbm_status ensure_graph(lbm_handle* h) {
     return fail(LBM_ERR_CUDA, std::string("graph capture failed: ") +
                                   cudaGetErrorString(err != cudaSuccess ? err : end));
   }
-  const cudaError_t inst = cudaGraphInstantiate(&h->graph[cur0], g, 0);
+  const cudaError_t inst = cudaGraphInstantiate(&h->graph, g, 0);
   cudaGraphDestroy(g);
   LBM_CUDA_TRY(inst);
-  h->graph_steps = kGraphSteps;
   return LBM_OK;
 }
 
 lbm_status run_steps(lbm_handle* h, int nsteps) {
   if (nsteps <= 0) return LBM_OK;
   lbm_status st;
-  // capture the step chains before the start event: capture and instantiation
-  // are host work and must not count as step time
-  if (nsteps - (h->given_macro ? 1 : 0) - 1 >= kGraphSteps) {
-    const int cur0 = h->cur;
-    for (int parity = 0; parity < 2; parity++) {
-      h->cur = parity;
-      if ((st = ensure_graph(h)) != LBM_OK) {
-        h->cur = cur0;
-        return st;
-      }
-    }
-    h->cur = cur0;
-  }
-  LBM_CUDA_TRY(cudaEventRecord(h->ev0, h->stream));
+  // steps outside the chains: the first of a given state or out of a kLocal
+  // one, and the last of the call, which writes the pre-collision macro
+  // fields (the velocity one step before the new state)
   int left = nsteps;
-  if (h->given_macro) {
-    if ((st = one_step(h, left == 1)) != LBM_OK) return st;
-    left--;
-  }
-  // all but the last step through captured chains, the last one writes the
-  // pre-collision macro fields (the velocity one step before the new state)
-  while (left - 1 >= kGraphSteps) {
-    if ((st = ensure_graph(h)) != LBM_OK) return st;
-    LBM_CUDA_TRY(cudaGraphLaunch(h->graph[h->cur], h->stream));
-    h->step += kGraphSteps;
-    left -= kGraphSteps;
+  const bool lead_given = h->given_macro;
+  const int after_given = lead_given ? kLocal : h->cur;
+  const int lead = (lead_given ? 1 : 0) + (after_given == kLocal ? 1 : 0);
+  const bool chains = nsteps - lead - 1 >= kGraphSteps;
+  // capture before the start event: capture and instantiation are host work
+  // and must not count as step time
+  if (chains && (st = ensure_graph(h)) != LBM_OK) return st;
+  LBM_CUDA_TRY(cudaEventRecord(h->ev0, h->stream));
+  if (chains) {
+    for (int i = 0; i < lead; i++, left--)
+      if ((st = one_step(h, false)) != LBM_OK) return st;
+    for (; left - 1 >= kGraphSteps; left -= kGraphSteps) {
+      LBM_CUDA_TRY(cudaGraphLaunch(h->graph, h->stream));
+      h->step += kGraphSteps;
+    }
   }
   while (left > 0) {
     if ((st = one_step(h, left == 1)) != LBM_OK) return st;

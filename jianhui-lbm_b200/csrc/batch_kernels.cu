@@ -43,7 +43,8 @@ __global__ void __launch_bounds__(BS, 640 / BS) batch_step_kernel(BatchStepArgs 
   const int i = blockIdx.x;
   if (i >= a.ntiles) return;
   __shared__ SlotKeep<LOCAL ? 1 : BS, 2> keep;
-  const TileWork w = a.work[i];
+  step_begin();
+  const TileWork w = a.work[i];  // written before the chain's first step, which is launched in order
   const float scale = w.fp16_scale, inv_scale = 1.0f / w.fp16_scale;
   const CollideScalars cs = collide_scalars(w.g[0], w.g[1], w.g[2], w.s_v, w.s_o);
 #pragma unroll 1
@@ -56,11 +57,11 @@ __global__ void __launch_bounds__(BS, 640 / BS) batch_step_kernel(BatchStepArgs 
     const int p1 = both ? second : p;  // a missing second node is worked on as the first and not stored
     F2 f[kQ];
     if constexpr (LOCAL) {
+      step_wait();
       load_row<K>(pop + p, inv_scale, f[0]);
 #pragma unroll
       for (int q = 1; q < kQ; q++) load_row<K>(pop + (size_t)opp(q) * cap + p, inv_scale, f[q]);
     } else {
-      f[0] = make_f2(load_pop_rw<K>(pop + p, inv_scale), load_pop_rw<K>(pop + p1, inv_scale));
       int32_t s0[kQ], s1[kQ];
       if constexpr (ROWS) {
         row_slots(a.rows, a.table, cap, p, s0);
@@ -72,6 +73,8 @@ __global__ void __launch_bounds__(BS, 640 / BS) batch_step_kernel(BatchStepArgs 
           s1[q] = __ldg(a.table + (size_t)(q - 1) * cap + p1);
         }
       }
+      step_wait();
+      f[0] = make_f2(load_pop_rw<K>(pop + p, inv_scale), load_pop_rw<K>(pop + p1, inv_scale));
 #pragma unroll
       for (int q = 1; q < kQ; q++)
         f[q] = make_f2(load_pop_rw<K>(pop + s0[q], inv_scale), load_pop_rw<K>(pop + s1[q], inv_scale));
@@ -322,23 +325,27 @@ __global__ void batch_init_kernel(typename Traits<K>::T* __restrict__ pop, int p
 }
 
 template <Store K, int BS>
-static void step_bs(const BatchStepArgs& a, int grid, int chain_step, cudaStream_t st) {
+static cudaError_t step_bs(const BatchStepArgs& a, int grid, int chain_step, cudaStream_t st) {
+  // the chain's first step follows the list kernels; see chain_pays
+  const bool chained = chain_step > 0 && (grid <= 32 || grid >= 1024);
   if (a.phase == kLocal)
-    batch_step_kernel<K, BS, true, false><<<grid, BS, 0, st>>>(a, chain_step);
-  else if (a.rows != nullptr)
-    batch_step_kernel<K, BS, false, true><<<grid, BS, 0, st>>>(a, chain_step);
-  else
-    batch_step_kernel<K, BS, false, false><<<grid, BS, 0, st>>>(a, chain_step);
+    return launch_chained(batch_step_kernel<K, BS, true, false>, grid, BS, st, chained, a, chain_step);
+  if (a.rows != nullptr)
+    return launch_chained(batch_step_kernel<K, BS, false, true>, grid, BS, st, chained, a, chain_step);
+  return launch_chained(batch_step_kernel<K, BS, false, false>, grid, BS, st, chained, a, chain_step);
 }
-// `block` nodes a pass, two per thread.
+// `block` nodes a pass, two per thread; a tile in one pass where there are
+// too few tiles to fill the chip in two (one | two passes: 3.50 | 3.98 us per
+// step at 5.5 K nodes, 4.25 | 4.73 at 44 K, 5.58 | 5.75 at 88 K, 7.93 | 7.17 at
+// 177 K, a grid of 512).
 template <Store K>
 static cudaError_t step_k(const BatchStepArgs& a, int block, int grid, int chain_step, cudaStream_t st) {
+  if (grid <= 256) block = 512;
   switch (block) {
-    case 128: step_bs<K, 64>(a, grid, chain_step, st); break;
-    case 512: step_bs<K, 256>(a, grid, chain_step, st); break;
-    default: step_bs<K, 128>(a, grid, chain_step, st); break;
+    case 128: return step_bs<K, 64>(a, grid, chain_step, st);
+    case 512: return step_bs<K, 256>(a, grid, chain_step, st);
+    default: return step_bs<K, 128>(a, grid, chain_step, st);
   }
-  return cudaGetLastError();
 }
 
 int batch_step_grid(int ntiles, int block) {

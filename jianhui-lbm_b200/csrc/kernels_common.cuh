@@ -59,6 +59,33 @@ struct Traits<Store::F16> {
   static constexpr bool kDev = true;
 };
 
+// Programmatic dependent launch between the steps of a chain.  A step lets
+// the next one launch as soon as its own blocks run (step_begin); the next
+// reads what no step writes, the table, and waits for the previous step's end
+// before it touches populations (step_wait).  A kernel that was launched
+// without the attribute waits for nothing here.
+__device__ __forceinline__ void step_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename Args, typename... More>
+cudaError_t launch_chained(void (*kernel)(Args, More...), int grid, int block, cudaStream_t st, bool chained,
+                           const Args& a, More... more) {
+  if (!chained) {
+    kernel<<<grid, block, 0, st>>>(a, more...);
+    return cudaGetLastError();
+  }
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)block);
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, a, more...);
+}
+
 // Read-only (non-coherent) loads, for the table and for populations that the
 // launch does not write.
 __device__ __forceinline__ double ldg_(const double* p) { return __ldg(p); }

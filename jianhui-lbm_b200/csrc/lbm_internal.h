@@ -240,6 +240,7 @@ struct StepArgs {
   const int32_t* table;  // [18][npad]
   const int32_t* rows;   // [9][npad] row form of the table (row_table.cuh), or null
   int ahead;             // nodes ahead that a block prefetches into L2, 0 = none
+  int chained;           // launched as a programmatic dependent of the step before it
   int n;                 // fluid nodes
   int npad;
   // macro input for a step that must use given rho/u (first step after init
@@ -252,6 +253,7 @@ struct StepArgs {
   double gx, gy, gz;
   double s_v, s_o;
   double fp16_scale;
+  float fp16_inv;        // (float)(1 / fp16_scale): a division in double per thread else
   // pressure/velocity faces: nodes [n_main, n) are left to the boundary
   // kernel; nodes [snap_begin, n_main) record their post-streaming state in
   // snap_dst ([23][nsnap] doubles: f_0..f_18, rho, ux, uy, uz; slot = p -
@@ -309,6 +311,18 @@ constexpr bool rows_pay(long long marked, long long n) { return marked * 8 <= n;
 constexpr int prefetch_ahead(long long n, long long pop_bytes, long long table_bytes) {
   return n * (pop_bytes + table_bytes) > (120LL << 20) ? 148 * 640 : 0;
 }
+
+// Whether the steps of a chain are launched as programmatic dependents
+// (kernels_common.cuh), for n nodes and `full` nodes from which the chip is
+// full.  The next step's blocks then start in the slots the running one
+// leaves, which saves a launch gap per step, but where the two together
+// neither leave SMs free nor fill them they land unevenly.  us per step,
+// chained | not, cubes at porosity 0.35:
+//   FP32  5 K nodes 2.27 | 2.72, 22 K 2.85 | 2.82, 49 K 4.00 | 3.47, 101 K
+//         5.07 | 4.23, 131 K 5.25 | 5.25, 179 K 5.14 | 5.52, 310 K 7.83 | 8.21,
+//         734 K 17.0 | 18.1, 5.9 M 161 | 164
+//   FP64  11 K 5.82 | 6.17, 22 K 7.49 | 6.29, 39 K 8.57 | 8.72, 92 K 12.2 | 12.6
+constexpr bool chain_pays(long long n, long long full) { return n <= 74 * 256 || n >= full; }
 
 constexpr int kSnapRows = kQ + 4;  // per-step record of a node: f_0..f_18, rho, ux, uy, uz
 

@@ -19,8 +19,8 @@ struct SetupScratch {
   ~SetupScratch() { release(); }
   lbm_status reserve(long long cells, int nodes);
   // Places the arrays in [base, base + bytes) of a device buffer that is not
-  // in use until the indexing has finished (a solver's second population
-  // array), saving their allocation and release; false when they do not fit
+  // in use until the indexing has finished (a solver's population
+  // array before its initial state), saving their allocation and release; false when they do not fit
   // (then reserve allocates them).
   bool borrow(void* base, size_t bytes, long long cells, int nodes);
   void release();

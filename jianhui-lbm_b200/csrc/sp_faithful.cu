@@ -367,12 +367,15 @@ __device__ __forceinline__ void collide_moments(double (&m)[kQ], double rho, dou
 template <bool LOCAL, bool ROWS, typename Got>
 __device__ __forceinline__ void pull_f64(const StepArgs& a, int p, double (&f)[kQ], Got&& got) {
   const double* pop = static_cast<const double*>(a.pop);
-  f[0] = pop[p];
   int32_t s[kQ];
   if constexpr (ROWS) row_slots(a.rows, a.table, a.npad, p, s);
 #pragma unroll
-  for (int q = 1; q < kQ; q++) {
+  for (int q = 1; q < kQ; q++)
     if constexpr (!ROWS) s[q] = LOCAL ? opp(q) * a.npad + p : __ldg(a.table + (size_t)(q - 1) * a.npad + p);
+  step_wait();
+  f[0] = pop[p];
+#pragma unroll
+  for (int q = 1; q < kQ; q++) {
     f[q] = pop[s[q]];
     got(q, s[q]);
   }
@@ -421,6 +424,7 @@ __global__ void __launch_bounds__(BS, f64_min_blocks(BS)) step_f64_faithful(Step
   const int p = blockIdx.x * BS + threadIdx.x;
   prefetch_block<BS, BS, ROWS ? 9 : LOCAL ? 0 : 18>(static_cast<const double*>(a.pop), ROWS ? a.rows : a.table, a.npad,
                                                 a.ahead);
+  step_begin();
   if (p >= a.n_main) return;
   // the slots of a kPull state's gathers, for the stores after the collision
   // (each read by the thread that wrote it)
@@ -540,21 +544,19 @@ static cudaError_t launch_f64_bs(const StepArgs& a, cudaStream_t st) {
   if (a.phase == kLocal) {
     if (given) return cudaErrorInvalidValue;  // a given state is a kPull state
     if (write)
-      step_f64_faithful<BS, false, true, GX, LAT, true, false><<<grid, BS, 0, st>>>(a);
-    else
-      step_f64_faithful<BS, false, false, GX, LAT, true, false><<<grid, BS, 0, st>>>(a);
+      return launch_chained(step_f64_faithful<BS, false, true, GX, LAT, true, false>, grid, BS, st, a.chained != 0, a);
+    return launch_chained(step_f64_faithful<BS, false, false, GX, LAT, true, false>, grid, BS, st, a.chained != 0, a);
   } else if (given && write) {
-    step_f64_faithful<BS, true, true, GX, LAT, false, false><<<grid, BS, 0, st>>>(a);
+    return launch_chained(step_f64_faithful<BS, true, true, GX, LAT, false, false>, grid, BS, st, a.chained != 0, a);
   } else if (given) {
-    step_f64_faithful<BS, true, false, GX, LAT, false, false><<<grid, BS, 0, st>>>(a);
+    return launch_chained(step_f64_faithful<BS, true, false, GX, LAT, false, false>, grid, BS, st, a.chained != 0, a);
   } else if (write) {
-    a.rows ? step_f64_faithful<BS, false, true, GX, LAT, false, true><<<grid, BS, 0, st>>>(a)
-           : step_f64_faithful<BS, false, true, GX, LAT, false, false><<<grid, BS, 0, st>>>(a);
+    return a.rows ? launch_chained(step_f64_faithful<BS, false, true, GX, LAT, false, true>, grid, BS, st, a.chained != 0, a)
+           : launch_chained(step_f64_faithful<BS, false, true, GX, LAT, false, false>, grid, BS, st, a.chained != 0, a);
   } else {
-    a.rows ? step_f64_faithful<BS, false, false, GX, LAT, false, true><<<grid, BS, 0, st>>>(a)
-           : step_f64_faithful<BS, false, false, GX, LAT, false, false><<<grid, BS, 0, st>>>(a);
+    return a.rows ? launch_chained(step_f64_faithful<BS, false, false, GX, LAT, false, true>, grid, BS, st, a.chained != 0, a)
+           : launch_chained(step_f64_faithful<BS, false, false, GX, LAT, false, false>, grid, BS, st, a.chained != 0, a);
   }
-  return cudaGetLastError();
 }
 
 template <int BS>

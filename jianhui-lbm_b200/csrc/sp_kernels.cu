@@ -138,20 +138,23 @@ __global__ void __launch_bounds__(BS, BS == 256 ? 2 : 1) step_dev_kernel(StepArg
   if constexpr (SL == Slots::Compact) compact_load(cb, a, p, ow);
   prefetch_block<BS, BS, SL == Slots::Rows ? 9 : SL == Slots::Table ? 18 : 0>(
       static_cast<const double*>(a.pop), SL == Slots::Rows ? a.rows : a.table, a.npad, a.ahead);
+  step_begin();
   if (p >= a.n_main) return;
   double* pop = static_cast<double*>(a.pop);
   double f[kQ];
-  f[0] = pop[p];
   if constexpr (SL == Slots::Local) {
+    step_wait();
 #pragma unroll
     for (int q = 1; q < kQ; q++) f[q] = pop[(size_t)opp(q) * a.npad + p];
   } else {
     int32_t slot[kQ];
     read_slots<SL>(cb, a, p, ow, slot);
+    step_wait();
 #pragma unroll
     for (int q = 1; q < kQ; q++) f[q] = pop[slot[q]];
     keep_slots(keep, threadIdx.x, [&](int q) { return slot[q]; });
   }
+  f[0] = pop[p];
   PairSplit<double> ps;
   split_pairs(f, ps);
   double drho, rho, ux, uy, uz;
@@ -222,23 +225,22 @@ __global__ void __launch_bounds__(BS, vec_min_blocks<V>(BS)) step_vec_kernel(Ste
   if constexpr (SL == Slots::Compact) compact_load(cb, a, p, ow);
   prefetch_block<BS, BS * N, SL == Slots::Rows ? 9 : SL == Slots::Table ? 18 : 0>(
       static_cast<const T*>(a.pop), SL == Slots::Rows ? a.rows : a.table, a.npad, a.ahead);
+  step_begin();
   if (p >= a.n_main) return;
   const bool both = N == 2 && second < a.n_main;
   const int p1 = both ? second : p;  // a missing second node is worked on as the first and not stored
   T* pop = static_cast<T*>(a.pop);
   const float scale = (float)a.fp16_scale;
-  const float inv_scale = (float)(1.0 / a.fp16_scale);
+  const float inv_scale = a.fp16_inv;
   V f[kQ];
-  if constexpr (N == 1 || PAIR)
-    load_row<K>(pop + p, inv_scale, f[0]);
-  else
-    f[0] = make_f2(load_pop_rw<K>(pop + p, inv_scale), load_pop_rw<K>(pop + p1, inv_scale));
   if constexpr (SL == Slots::Local) {
+    step_wait();
 #pragma unroll
     for (int q = 1; q < kQ; q++) load_row<K>(pop + (size_t)opp(q) * a.npad + p, inv_scale, f[q]);
   } else if constexpr (N == 1) {
     int32_t slot[kQ];  // slot[q] holds f_q on entry and takes f*_opp(q)
     read_slots<SL>(cb, a, p, ow, slot);
+    step_wait();
 #pragma unroll
     for (int q = 1; q < kQ; q++) f[q] = load_pop_rw<K>(pop + slot[q], inv_scale);
     keep_slots(keep, threadIdx.x, [&](int q) { return slot[q]; });
@@ -260,6 +262,7 @@ __global__ void __launch_bounds__(BS, vec_min_blocks<V>(BS)) step_vec_kernel(Ste
         s1[q] = __ldg(a.table + (size_t)(q - 1) * a.npad + p1);
       }
     }
+    step_wait();
 #pragma unroll
     for (int q = 1; q < kQ; q++)
       f[q] = make_f2(load_pop_rw<K>(pop + s0[q], inv_scale), load_pop_rw<K>(pop + s1[q], inv_scale));
@@ -267,6 +270,11 @@ __global__ void __launch_bounds__(BS, vec_min_blocks<V>(BS)) step_vec_kernel(Ste
     for (int i = 0; i < 9; i++)
       keep.a[i][threadIdx.x] = make_int4(s0[2 * i + 1], s1[2 * i + 1], s0[2 * i + 2], s1[2 * i + 2]);
   }
+
+  if constexpr (N == 1 || PAIR)
+    load_row<K>(pop + p, inv_scale, f[0]);
+  else
+    f[0] = make_f2(load_pop_rw<K>(pop + p, inv_scale), load_pop_rw<K>(pop + p1, inv_scale));
 
   // velocities in units of lat_c (1 on the default lattice, where the
   // scalings below are exact)
@@ -423,26 +431,26 @@ cudaError_t launch_boundary(Store kind, const BcArgs& a, cudaStream_t st) {
 }
 
 template <int BS, Slots SL>
-static void launch_f64d(const StepArgs& a, int grid, cudaStream_t st) {
+static cudaError_t launch_f64d(const StepArgs& a, int grid, cudaStream_t st) {
   const bool given = a.rho_in != nullptr, write = a.rho_out != nullptr;
   if constexpr (SL != Slots::Local) {
     if (given)
-      return write ? step_dev_kernel<BS, true, true, SL><<<grid, BS, 0, st>>>(a)
-                   : step_dev_kernel<BS, true, false, SL><<<grid, BS, 0, st>>>(a);
+      return write ? launch_chained(step_dev_kernel<BS, true, true, SL>, grid, BS, st, a.chained != 0, a)
+                   : launch_chained(step_dev_kernel<BS, true, false, SL>, grid, BS, st, a.chained != 0, a);
   }
-  write ? step_dev_kernel<BS, false, true, SL><<<grid, BS, 0, st>>>(a)
-        : step_dev_kernel<BS, false, false, SL><<<grid, BS, 0, st>>>(a);
+  return write ? launch_chained(step_dev_kernel<BS, false, true, SL>, grid, BS, st, a.chained != 0, a)
+        : launch_chained(step_dev_kernel<BS, false, false, SL>, grid, BS, st, a.chained != 0, a);
 }
 template <Store K, int BS, typename V, Slots SL>
-static void launch_vec(const StepArgs& a, int grid, cudaStream_t st) {
+static cudaError_t launch_vec(const StepArgs& a, int grid, cudaStream_t st) {
   const bool given = a.rho_in != nullptr, write = a.rho_out != nullptr;
   if constexpr (SL != Slots::Local && VecOf<V>::kNodes == 1) {
     if (given)
-      return write ? step_vec_kernel<K, BS, V, true, true, SL><<<grid, BS, 0, st>>>(a)
-                   : step_vec_kernel<K, BS, V, true, false, SL><<<grid, BS, 0, st>>>(a);
+      return write ? launch_chained(step_vec_kernel<K, BS, V, true, true, SL>, grid, BS, st, a.chained != 0, a)
+                   : launch_chained(step_vec_kernel<K, BS, V, true, false, SL>, grid, BS, st, a.chained != 0, a);
   }
-  write ? step_vec_kernel<K, BS, V, false, true, SL><<<grid, BS, 0, st>>>(a)
-        : step_vec_kernel<K, BS, V, false, false, SL><<<grid, BS, 0, st>>>(a);
+  return write ? launch_chained(step_vec_kernel<K, BS, V, false, true, SL>, grid, BS, st, a.chained != 0, a)
+        : launch_chained(step_vec_kernel<K, BS, V, false, false, SL>, grid, BS, st, a.chained != 0, a);
 }
 
 template <Store K, int BS>
@@ -454,26 +462,26 @@ static cudaError_t launch_dev_bs(const StepArgs& a, cudaStream_t st) {
   const int grid = (a.n_main + BS - 1) / BS;  // BS nodes per block, by BS or BS / 2 threads
   if constexpr (K == Store::F64D) {
     switch (sl) {
-      case Slots::Local: launch_f64d<BS, Slots::Local>(a, grid, st); break;
-      case Slots::Table: launch_f64d<BS, Slots::Table>(a, grid, st); break;
-      case Slots::Rows: launch_f64d<BS, Slots::Rows>(a, grid, st); break;
-      case Slots::Compact: launch_f64d<BS, Slots::Compact>(a, grid, st); break;
+      case Slots::Local: return launch_f64d<BS, Slots::Local>(a, grid, st);
+      case Slots::Table: return launch_f64d<BS, Slots::Table>(a, grid, st);
+      case Slots::Rows: return launch_f64d<BS, Slots::Rows>(a, grid, st);
+      case Slots::Compact: return launch_f64d<BS, Slots::Compact>(a, grid, st);
     }
   } else if (a.rho_in == nullptr && sl != Slots::Compact && two_nodes(a.n_main)) {
     switch (sl) {
-      case Slots::Local: launch_vec<K, BS / 2, F2, Slots::Local>(a, grid, st); break;
-      case Slots::Rows: launch_vec<K, BS / 2, F2, Slots::Rows>(a, grid, st); break;
-      default: launch_vec<K, BS / 2, F2, Slots::Table>(a, grid, st); break;
+      case Slots::Local: return launch_vec<K, BS / 2, F2, Slots::Local>(a, grid, st);
+      case Slots::Rows: return launch_vec<K, BS / 2, F2, Slots::Rows>(a, grid, st);
+      default: return launch_vec<K, BS / 2, F2, Slots::Table>(a, grid, st);
     }
   } else {
     switch (sl) {
-      case Slots::Local: launch_vec<K, BS, float, Slots::Local>(a, grid, st); break;
-      case Slots::Table: launch_vec<K, BS, float, Slots::Table>(a, grid, st); break;
-      case Slots::Rows: launch_vec<K, BS, float, Slots::Rows>(a, grid, st); break;
-      case Slots::Compact: launch_vec<K, BS, float, Slots::Compact>(a, grid, st); break;
+      case Slots::Local: return launch_vec<K, BS, float, Slots::Local>(a, grid, st);
+      case Slots::Table: return launch_vec<K, BS, float, Slots::Table>(a, grid, st);
+      case Slots::Rows: return launch_vec<K, BS, float, Slots::Rows>(a, grid, st);
+      case Slots::Compact: return launch_vec<K, BS, float, Slots::Compact>(a, grid, st);
     }
   }
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 template <Store K>

@@ -115,6 +115,7 @@ lbm_status solute_graph(lbm_st7_handle* h, int c0) {
   St7Args a = st7_args(h, false);
   for (int s = 0; s < kSoluteGraphSteps && err == cudaSuccess; s++) {
     a.phase = (c0 + s) & 1;
+    a.chained = s > 0 && chain_pays(h->geo.count, 148 * 1024);
     err = st7_launch_step(h->f64, a, h->stream);
   }
   const cudaError_t end = cudaStreamEndCapture(h->stream, &g);

@@ -11,6 +11,7 @@ struct St7Args {
   const int32_t* table;   // D3Q19 pull table [18][npad]; D3Q7: rows 0..5 used
   const int32_t* rows;    // D3Q19: row form of the table (row_table.cuh), or null
   int ahead;              // nodes ahead that a block prefetches into L2, 0 = none
+  int chained;            // launched as a programmatic dependent of the step before it
   const void* u;          // [3][npad] advecting velocity
   const void* c_given;    // [npad] C for the first step after init, else null
   void* c_out;            // optional [npad]: C of this step's macro

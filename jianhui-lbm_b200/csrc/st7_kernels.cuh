@@ -45,6 +45,7 @@ template <typename T, bool GIVEN, bool LOCAL>
 __global__ void __launch_bounds__(256) st7_step_kernel(St7Args a) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   prefetch_solute<6, LOCAL ? 0 : 6, T>(a, a.table);
+  step_begin();
   if (x >= a.n) return;
   T* pop = static_cast<T*>(a.g);
   const T* __restrict__ u = static_cast<const T*>(a.u);
@@ -55,8 +56,10 @@ __global__ void __launch_bounds__(256) st7_step_kernel(St7Args a) {
 #pragma unroll
   for (int q = 1; q < 7; q++) {
     slot[q] = LOCAL ? (opp(q) - 1) * npad + x : __ldg(a.table + (size_t)(q - 1) * npad + x) - npad;
-    g[q] = pop[slot[q]];
   }
+  step_wait();
+#pragma unroll
+  for (int q = 1; q < 7; q++) g[q] = pop[slot[q]];
   T C;
   if (GIVEN) {
     C = static_cast<const T*>(a.c_given)[x];
@@ -109,6 +112,7 @@ __device__ __forceinline__ double st19_edot(double ux, double uy, double uz) {
 template <typename T, bool GIVEN, bool UNIT, int SLOTS>
 __global__ void __launch_bounds__(256) st19_step_kernel(St7Args a) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  step_begin();
   prefetch_solute<kQ, SLOTS == 1 ? 18 : SLOTS == 2 ? 9 : 0, T>(a, SLOTS == 2 ? a.rows : a.table);
   if (x >= a.n) return;
   T* pop = static_cast<T*>(a.g);
@@ -116,8 +120,8 @@ __global__ void __launch_bounds__(256) st19_step_kernel(St7Args a) {
   const T* __restrict__ u = static_cast<const T*>(a.u);
   const size_t npad = (size_t)a.npad;
   T g[kQ];
-  g[0] = pop[x];
   if constexpr (SLOTS == 0) {
+    step_wait();
 #pragma unroll
     for (int q = 1; q < kQ; q++) g[q] = pop[opp(q) * npad + x];
   } else {
@@ -128,6 +132,7 @@ __global__ void __launch_bounds__(256) st19_step_kernel(St7Args a) {
 #pragma unroll
       for (int q = 1; q < kQ; q++) slot[q] = __ldg(a.table + (size_t)(q - 1) * npad + x);
     }
+    step_wait();
 #pragma unroll
     for (int q = 1; q < kQ; q++) {
       g[q] = pop[slot[q]];
@@ -135,6 +140,7 @@ __global__ void __launch_bounds__(256) st19_step_kernel(St7Args a) {
     }
     asm volatile("" ::: "memory");  // the slots are read again from where they were kept
   }
+  g[0] = pop[x];
   T C;
   if (GIVEN) {
     C = static_cast<const T*>(a.c_given)[x];
@@ -182,15 +188,14 @@ __global__ void __launch_bounds__(256) st19_step_kernel(St7Args a) {
 }
 
 template <typename T, bool UNIT>
-void launch_step19_unit(const St7Args& a, int grid, cudaStream_t st) {
+cudaError_t launch_step19_unit(const St7Args& a, int grid, cudaStream_t st) {
   if (a.c_given != nullptr)
-    st19_step_kernel<T, true, UNIT, 1><<<grid, 256, 0, st>>>(a);
-  else if (a.phase == kLocal)
-    st19_step_kernel<T, false, UNIT, 0><<<grid, 256, 0, st>>>(a);
-  else if (a.rows != nullptr)
-    st19_step_kernel<T, false, UNIT, 2><<<grid, 256, 0, st>>>(a);
-  else
-    st19_step_kernel<T, false, UNIT, 1><<<grid, 256, 0, st>>>(a);
+    return launch_chained(st19_step_kernel<T, true, UNIT, 1>, grid, 256, st, a.chained != 0, a);
+  if (a.phase == kLocal)
+    return launch_chained(st19_step_kernel<T, false, UNIT, 0>, grid, 256, st, a.chained != 0, a);
+  if (a.rows != nullptr)
+    return launch_chained(st19_step_kernel<T, false, UNIT, 2>, grid, 256, st, a.chained != 0, a);
+  return launch_chained(st19_step_kernel<T, false, UNIT, 1>, grid, 256, st, a.chained != 0, a);
 }
 
 template <typename T>
@@ -198,8 +203,7 @@ cudaError_t launch_step19(const St7Args& a, cudaStream_t st) {
   if (a.n == 0) return cudaSuccess;
   if (a.c_given != nullptr && a.phase == kLocal) return cudaErrorInvalidValue;  // a given state is a kPull state
   const int g = (a.n + 255) / 256;
-  a.c2 == 1.0 && a.c4 == 1.0 ? launch_step19_unit<T, true>(a, g, st) : launch_step19_unit<T, false>(a, g, st);
-  return cudaGetLastError();
+  return a.c2 == 1.0 && a.c4 == 1.0 ? launch_step19_unit<T, true>(a, g, st) : launch_step19_unit<T, false>(a, g, st);
 }
 
 template <typename T>
@@ -208,12 +212,10 @@ cudaError_t launch_step(const St7Args& a, cudaStream_t st) {
   if (a.c_given != nullptr && a.phase == kLocal) return cudaErrorInvalidValue;
   const int g = (a.n + 255) / 256;
   if (a.c_given != nullptr)
-    st7_step_kernel<T, true, false><<<g, 256, 0, st>>>(a);
-  else if (a.phase == kLocal)
-    st7_step_kernel<T, false, true><<<g, 256, 0, st>>>(a);
-  else
-    st7_step_kernel<T, false, false><<<g, 256, 0, st>>>(a);
-  return cudaGetLastError();
+    return launch_chained(st7_step_kernel<T, true, false>, g, 256, st, a.chained != 0, a);
+  if (a.phase == kLocal)
+    return launch_chained(st7_step_kernel<T, false, true>, g, 256, st, a.chained != 0, a);
+  return launch_chained(st7_step_kernel<T, false, false>, g, 256, st, a.chained != 0, a);
 }
 
 }  // namespace st7_detail
