@@ -707,8 +707,9 @@ def run_cg(a):
 def run_solute(a):
     """D3Q7 solute transport on the config-2 geometry (256^3 spheres, 5.87 M
     fluid nodes) advected by the FP32 flow after 300 steps: solute MLUPS in
-    FP32 and FP64, against the 2*6*s + 6*4 + 3*s bytes per update; the D3Q19
-    solute step beside it (2*19*s + 18*4 + 3*s bytes per update)."""
+    FP32 and FP64, against the 2*6*s + 3*s bytes per update, and the table's
+    6*4 on every second one; the D3Q19 solute step beside it (2*19*s + 3*s,
+    and the row table's 9*4 on every second one)."""
     world, rank, local, pg = dist_setup()
     import lbm_b200
 
@@ -732,7 +733,7 @@ def run_solute(a):
         return 0
     peak, peak_src = measured_peak()
     (ms32, n, m32), (ms64, _, m64) = out["f32"], out["f64"]
-    b32, b64 = 2 * 6 * 4 + 6 * 4 + 3 * 4, 2 * 6 * 8 + 6 * 4 + 3 * 8
+    b32, b64 = 2 * 6 * 4 + 3 * 4 + 3 * 4, 2 * 6 * 8 + 3 * 4 + 3 * 8
     line = {"metric": "D3Q7 solute MLUPS (FP32)", "value": n / (ms32 * 1e-3) / 1e6, "unit": "MLUPS",
             "n_gpus": world, "higher_is_better": True, "dtype": "f32", "data": "synthetic", "steps": steps,
             "warmup": a.warmup,
@@ -744,7 +745,7 @@ def run_solute(a):
             "fp64": {"mlups": n / (ms64 * 1e-3) / 1e6, "gbs": n * b64 / (ms64 * 1e-3) / 1e9, "bytes_per_lu": b64},
             "mass_rel_diff_f32_vs_f64": abs(m32 - m64) / abs(m64), "clocks": clk.summary()}
     (q32, _, n32), (q64, _, n64) = out["f32_q19"], out["f64_q19"]
-    c32, c64 = 2 * 19 * 4 + 18 * 4 + 3 * 4, 2 * 19 * 8 + 18 * 4 + 3 * 8
+    c32, c64 = 2 * 19 * 4 + 9 * 2 + 3 * 4, 2 * 19 * 8 + 9 * 2 + 3 * 8
     line["d3q19"] = {"what": "the D3Q19 solute program's step (lbm_st19_create_from_flow), same flow and C0",
                      "f32": {"mlups": n / (q32 * 1e-3) / 1e6, "gbs": n * c32 / (q32 * 1e-3) / 1e9,
                              "frac": n * c32 / (q32 * 1e-3) / 1e9 / peak, "bytes_per_lu": c32},

@@ -286,8 +286,9 @@ LBM_API lbm_status lbm_autotune(lbm_handle* h, int trial_steps, int* ordering_ou
 LBM_API lbm_status lbm_last_step_ms(lbm_handle* h, double* ms);
 
 /* Memory facts: bytes of device memory the handle holds and the algorithmic
- * bytes one fluid-node update moves (2*19*s populations + the pull-table
- * bytes of lbm_table_info). */
+ * bytes one fluid-node update moves on average (2*19*s populations + half
+ * the table bytes per node that the step reads: every second step reads no
+ * table). */
 LBM_API lbm_status lbm_memory(lbm_handle* h, size_t* device_bytes, double* bytes_per_lu);
 
 /* Device memory of every solver (single-phase, colour-gradient, solute, node
@@ -299,7 +300,9 @@ LBM_API lbm_status lbm_memory(lbm_handle* h, size_t* device_bytes, double* bytes
 LBM_API lbm_status lbm_release_cached_memory(void);
 
 /* Form of the pull table the step kernel reads (the reference's nei_loc,
- * SP3:1099-1151, as a pull table).  compact = 0 (default): the int32 table.
+ * SP3:1099-1151, as a pull table).  compact = 0 (default): the int32 table,
+ * which large solves in the reference's node order read in a 36-byte row
+ * form of their own choice.
  * compact = 1: per aligned group of 32 nodes and direction one int32 base
  * and per node a 16-bit offset from it, 18*2 + 18*4/32 bytes per node
  * instead of 18*4; groups whose sources spread wider than the offsets reach
@@ -309,7 +312,7 @@ LBM_API lbm_status lbm_release_cached_memory(void);
  * the int32 table.  The compact form (18*2.125 bytes per node of device
  * memory) is built when it is first chosen or asked about, not at creation. */
 LBM_API lbm_status lbm_set_table_mode(lbm_handle* h, int compact);
-/* current mode, table bytes per node the step reads, and the share of
+/* current mode, bytes per node of that mode's table, and the share of
  * (group, direction) pairs that fall back to the int32 table (asking for
  * the share builds the compact form if it was not built yet) */
 LBM_API lbm_status lbm_table_info(lbm_handle* h, int* compact, double* table_bytes_per_node,

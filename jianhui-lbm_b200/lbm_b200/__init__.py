@@ -1029,7 +1029,7 @@ class SinglePhase:
         _check(lib().lbm_set_lattice(self._h, float(dx), float(dt)))
 
     def set_table_mode(self, compact):
-        """1: compact pull table (default), 0: the int32 table; identical results."""
+        """1: compact pull table, 0 (default): the int32 table; identical results."""
         _check(lib().lbm_set_table_mode(self._h, int(compact)))
 
     def table_info(self):
