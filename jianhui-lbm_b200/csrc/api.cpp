@@ -425,12 +425,13 @@ BcArgs bc_args(lbm_handle* h, const StepArgs& s, int c) {
 // runs on the side stream beside the step kernel and the step ends when both
 // have.
 cudaError_t launch_full_step(lbm_handle* h, const StepArgs& a, int c) {
-  if (!h->bc.active) return launch_step(h->kind, a, h->block, h->stream);
+  const int block = h->block == 256 ? default_block(h->kind, a.n_main) : h->block;
+  if (!h->bc.active) return launch_step(h->kind, a, block, h->stream);
   cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
   if (e == cudaSuccess) e = launch_boundary(h->kind, bc_args(h, a, c), h->side);
   if (e == cudaSuccess) e = cudaEventRecord(h->ev_bc, h->side);
-  if (e == cudaSuccess) e = launch_step(h->kind, a, h->block, h->stream);
+  if (e == cudaSuccess) e = launch_step(h->kind, a, block, h->stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(h->stream, h->ev_bc, 0);
   return e;
 }

@@ -277,6 +277,18 @@ struct StepArgs {
   // written times lat_c)
   Lattice lat;
 };
+// Threads per block of the step where the caller left the default of 256: 64
+// for small solves, whose few large blocks leave SMs idle or give some twice
+// the work of others, and for the bit-exact FP64 step, whose blocks keep the
+// FP64 pipe busier when they end one by one.  us per step, 64 | 256 threads:
+// FP64 5 K nodes 4.28 | 5.66, 92 K 11.5 | 12.3, 310 K 28.2 | 30.9, 5.9 M 504 | 529;
+// FP64 deviation 5 K 2.15 | 3.00, 310 K 13.3 | 14.3, 734 K 45.5 | 43.8; FP32 5 K
+// 1.85 | 2.32, 49 K 3.12 | 3.51, 131 K 4.79 | 5.30 (above that two nodes per
+// thread, 310 K 7.99 | 7.82).
+constexpr int default_block(Store kind, long long n) {
+  return kind == Store::F64 || n < (kind == Store::F64D ? 400000 : 148 * 1024) ? 64 : 256;
+}
+
 cudaError_t launch_step(Store kind, const StepArgs& a, int block, cudaStream_t st);
 // Builds the compact pull table from `table` ([18][npad], n fluid nodes);
 // counts the (warp, direction) pairs left on the full table in *wide (device).

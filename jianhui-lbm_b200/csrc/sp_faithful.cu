@@ -409,9 +409,8 @@ __device__ __forceinline__ void macro_in_out(const StepArgs& a, int p, bool give
 }
 
 // Resident blocks per SM asked of the register allocator: 16 warps (128
-// registers, no spills) for 128-512 threads; 24 warps for 64-thread blocks
-// (80 registers with a few spills) -- the autotuner times both.
-constexpr int f64_min_blocks(int bs) { return bs == 64 ? 12 : 512 / bs; }
+// registers, no spills).
+constexpr int f64_min_blocks(int bs) { return 512 / bs; }
 
 // One node per thread.  The macro step of the reference (comput_macro_variables,
 // SP3:2414-2439) is rho = sum f and u = (j + dt g/2) / rho.  On the default
