@@ -43,24 +43,6 @@ static double feq_ref(int q, double rho, const double* u, const Lattice& L) {
   return weight(q) * rho * (1.0 + 3.0 * eu / c2 + 4.5 * eu * eu / c4 - 1.5 * uv / c2);
 }
 
-struct DevBuf {
-  void* p = nullptr;
-  size_t bytes = 0;
-  ~DevBuf() {
-    if (p) lbm::dev_free(p);
-  }
-  cudaError_t alloc(size_t b) {
-    if (p) lbm::dev_free(p);
-    p = nullptr;
-    bytes = b;
-    return b ? lbm::dev_alloc(&p, b) : cudaSuccess;
-  }
-  template <typename T>
-  T* as() const {
-    return static_cast<T*>(p);
-  }
-};
-
 // Allocator whose value-less construct leaves the element uninitialised, so
 // that resizing a byte vector that is overwritten at once does not first
 // zero it on one thread.

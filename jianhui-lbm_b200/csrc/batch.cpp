@@ -23,26 +23,6 @@ void order_nodes(const uint8_t* mask, int ordering, Geometry* g);
 
 namespace {
 
-struct Buf {
-  void* p = nullptr;
-  size_t bytes = 0;
-  ~Buf() { release(); }
-  void release() {
-    if (p) lbm::dev_free(p);
-    p = nullptr;
-    bytes = 0;
-  }
-  cudaError_t alloc(size_t b) {
-    release();
-    bytes = b;
-    return b ? lbm::dev_alloc(&p, b) : cudaSuccess;
-  }
-  template <typename T>
-  T* as() const {
-    return static_cast<T*>(p);
-  }
-};
-
 // A solve's host-side description and layout.
 struct Job {
   long long id = -1;
@@ -110,8 +90,8 @@ struct Pool {
   int block = 256, grid = 0;
   int ordering = LBM_ORDER_REFERENCE;
   double fp16_scale = 1.0;
-  Buf x_fields;  // field export
-  Buf pop, table, rows, tile_inst, inst, state, partials, active_tiles, n_active, work, slot_off;
+  DevBuf x_fields;  // field export
+  DevBuf pop, table, rows, tile_inst, inst, state, partials, active_tiles, n_active, work, slot_off;
   SetupScratch setup;
   std::vector<InstParams> h_inst;
   InstState* h_state = nullptr;  // pinned
@@ -450,7 +430,7 @@ struct Pool {
     if (x_fields.bytes < need) LBM_CUDA_TRY(x_fields.alloc(need));
     double* r = x_fields.as<double>();
     double* v = r + rows;
-    Buf ref;  // reference order: internal index p is reference id p + 1
+    DevBuf ref;  // reference order: internal index p is reference id p + 1
     if (!j.geo.ref_of.empty()) {
       LBM_CUDA_TRY(ref.alloc(sizeof(int32_t) * n));
       LBM_CUDA_TRY(cudaMemcpyAsync(ref.p, j.geo.ref_of.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream));

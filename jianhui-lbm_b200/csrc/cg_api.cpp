@@ -17,24 +17,6 @@ lbm_status read_mask_file(const char* path, int nx, int ny, int nz, int decbin, 
 
 namespace {
 
-struct Dev {
-  void* p = nullptr;
-  size_t bytes = 0;
-  ~Dev() {
-    if (p) lbm::dev_free(p);
-  }
-  cudaError_t alloc(size_t b) {
-    if (p) lbm::dev_free(p);
-    p = nullptr;
-    bytes = b;
-    return b ? lbm::dev_alloc(&p, b) : cudaSuccess;
-  }
-  template <typename T>
-  T* as() const {
-    return static_cast<T*>(p);
-  }
-};
-
 constexpr int kCgGraphSteps = 16;
 
 // Draw k (0-based) of the seeded generator that stands in for the
@@ -69,11 +51,11 @@ struct lbm_cg_handle {
   Geometry geo;
   double MI[kQ][kQ];
   CgParams cp{};
-  Dev f[2], gr, gb, rec, table, corder, psi, rho_r, rho_b, ref_of, partials, result;
-  Dev u_prev, axis, partials2, result2;  // Error's u0 and the saturation position sums
-  Dev win;                                // permeability window flags, or none
-  Dev face_nodes, face_psi0;              // phase-face nodes and their constant values
-  Dev face_src, face_tmp;                 // copied-phase faces: source node per entry (-1: constant), values
+  DevBuf f[2], gr, gb, rec, table, corder, psi, rho_r, rho_b, ref_of, partials, result;
+  DevBuf u_prev, axis, partials2, result2;  // Error's u0 and the saturation position sums
+  DevBuf win;                                // permeability window flags, or none
+  DevBuf face_nodes, face_psi0;              // phase-face nodes and their constant values
+  DevBuf face_src, face_tmp;                 // copied-phase faces: source node per entry (-1: constant), values
   bool face_copy = false;                 // some face node copies another node's phase
   // psi / rho_r / rho_b already hold the pending macro step's colour pass
   // (a reader ran it); the next step uses them instead of running it again,
@@ -82,8 +64,8 @@ struct lbm_cg_handle {
   bool colour_done = false;
   double rand_sat = -1.0;                 // ini_Sat: threshold of the random phase faces
   unsigned long long rand_seed = 0;       // seed of the random phase faces
-  Dev x_fields;                           // field export, kept between calls
-  Dev zero_sigma;                         // zero-surface-tension layer flags, or none
+  DevBuf x_fields;                           // field export, kept between calls
+  DevBuf zero_sigma;                         // zero-surface-tension layer flags, or none
   int nface = 0;
   std::vector<double> psi0;               // initial phase per node (internal order), as read
   long long window_volume = 0;            // divisor of the fluxes and the saturation
@@ -94,7 +76,7 @@ struct lbm_cg_handle {
   // set between steps acts on the step just run, as the reference changes
   // p_* between collision and boundary_pressure.
   lbm_boundary bc{};
-  Dev bc_nodes, bc_off, bc_ops, bc_snap, bc_rec;
+  DevBuf bc_nodes, bc_off, bc_ops, bc_snap, bc_rec;
   int bc_nface = 0, bc_nsnap = 0;
   bool faces_pending = false;
   int perdir = 1;
@@ -661,7 +643,7 @@ lbm_status lbm_cg_get_fields(lbm_cg_handle* h, double* rho, double* u, double* p
   if (rho) LBM_CUDA_TRY(d2h_staged(rho, rref, rows * sizeof(double), h->stream));
   if (u) LBM_CUDA_TRY(d2h_staged(u, uref, 3 * rows * sizeof(double), h->stream));
   double* outs[3] = {psi, rho_r, rho_b};
-  const Dev* srcs[3] = {&h->psi, &h->rho_r, &h->rho_b};
+  const DevBuf* srcs[3] = {&h->psi, &h->rho_r, &h->rho_b};
   for (int i = 0; i < 3; i++) {
     if (!outs[i]) continue;
     LBM_CUDA_TRY(launch_export_scalar(h->f64, srcs[i]->p, h->ref_of.as<int32_t>(), n, rref, h->stream));
@@ -677,7 +659,7 @@ lbm_status lbm_cg_get_populations(lbm_cg_handle* h, double* f) {
   if (!f) return fail(LBM_ERR_ARG, "lbm_cg_get_populations: null output");
   LBM_CUDA_TRY(resolve_faces(h));
   const int n = h->geo.count;
-  Dev o;
+  DevBuf o;
   LBM_CUDA_TRY(o.alloc((size_t)(n + 1) * kQ * sizeof(double)));
   LBM_CUDA_TRY(cudaMemsetAsync(o.p, 0, o.bytes, h->stream));
   LBM_CUDA_TRY(cg_export_f(h->f64, h->f[h->cur].p, h->table.as<int32_t>(), h->ref_of.as<int32_t>(), n, h->geo.npad,
@@ -947,7 +929,7 @@ lbm_status lbm_cg_set_state(lbm_cg_handle* h, const double* f, const double* psi
   if (st != LBM_OK) return st;
   if (!f || !psi || !rho_r || !rho_b) return fail(LBM_ERR_ARG, "lbm_cg_set_state: null argument");
   const int n = h->geo.count, npad = h->geo.npad;
-  Dev in;
+  DevBuf in;
   const size_t fbytes = (size_t)(n + 1) * kQ * sizeof(double);
   LBM_CUDA_TRY(in.alloc(fbytes));
   LBM_CUDA_TRY(cudaMemcpyAsync(in.p, f, fbytes, cudaMemcpyHostToDevice, h->stream));
@@ -955,7 +937,7 @@ lbm_status lbm_cg_set_state(lbm_cg_handle* h, const double* f, const double* psi
                            in.as<double>(), h->stream));
   // scalar fields: internal order equals reference order - 1 for this solver
   const double* srcs[3] = {psi, rho_r, rho_b};
-  Dev* dsts[3] = {&h->psi, &h->rho_r, &h->rho_b};
+  DevBuf* dsts[3] = {&h->psi, &h->rho_r, &h->rho_b};
   std::vector<double> d(npad, 0.0);
   std::vector<float> fl(npad, 0.f);
   for (int i = 0; i < 3; i++) {

@@ -209,6 +209,36 @@ void dev_free(void* p);
 // Returns the memory freed solvers left in the pools to the driver.
 cudaError_t dev_pool_trim();
 
+// A device buffer of a solver.  After an allocation that failed it is empty
+// (p null, bytes 0), so a caller that decides by either allocates again.
+struct DevBuf {
+  void* p = nullptr;
+  size_t bytes = 0;
+  DevBuf() = default;
+  DevBuf(const DevBuf&) = delete;
+  DevBuf& operator=(const DevBuf&) = delete;
+  ~DevBuf() { release(); }
+  void release() {
+    if (p) dev_free(p);
+    p = nullptr;
+    bytes = 0;
+  }
+  cudaError_t alloc(size_t b) {
+    release();
+    if (b == 0) return cudaSuccess;
+    const cudaError_t e = dev_alloc(&p, b);
+    if (e == cudaSuccess)
+      bytes = b;
+    else
+      p = nullptr;
+    return e;
+  }
+  template <typename T>
+  T* as() const {
+    return static_cast<T*>(p);
+  }
+};
+
 // Mask and box of a single-phase handle (for solvers coupled to it).
 const uint8_t* lbm_internal_mask(lbm_handle* h, int* nx, int* ny, int* nz);
 extern "C" const uint8_t* lbm_cg_internal_mask(lbm_cg_handle* h, int* nx, int* ny, int* nz);

@@ -13,20 +13,6 @@
 namespace lbm {
 namespace {
 
-struct Mem {
-  void* p = nullptr;
-  size_t bytes = 0;
-  ~Mem() {
-    if (p) lbm::dev_free(p);
-  }
-  cudaError_t alloc(size_t b) {
-    if (p) lbm::dev_free(p);
-    p = nullptr;
-    bytes = b;
-    return b ? lbm::dev_alloc(&p, b) : cudaSuccess;
-  }
-};
-
 // Slab-solver ids at one rank run over pore cells with i outer, k fastest
 // (SP:1168-1180), i.e. ascending coor = i*ny*nz + j*nz + k.  Returns, for each
 // slab id s (0-based), the library's reference id (1-based).
@@ -52,7 +38,7 @@ struct lbm_st7_handle {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   Geometry geo;
-  Mem g, table, rows, u, c0, ref_of, x_conc;
+  DevBuf g, table, rows, u, c0, ref_of, x_conc;
   int cur = kPull;  // phase of g
   bool rows_on = false;
   // captured step chains, one per starting phase
@@ -129,7 +115,7 @@ lbm_status solute_graph(lbm_st7_handle* h, int c0) {
   return LBM_OK;
 }
 
-lbm_status upload_as(lbm_st7_handle* h, Mem& m, const std::vector<double>& v) {
+lbm_status upload_as(lbm_st7_handle* h, DevBuf& m, const std::vector<double>& v) {
   if (h->f64) {
     LBM_CUDA_TRY(cudaMemcpyAsync(m.p, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice, h->stream));
     LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -183,7 +169,7 @@ lbm_status create_solute(const lbm_st7_params* p, const uint8_t* mask, int nx, i
                                h->stream));
   LBM_CUDA_TRY(cudaMemcpyAsync(h->ref_of.p, g.ref_of.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, h->stream));
   if (nq == kQ && rows_large(n, (kQ + 3LL) * (long long)s)) {
-    Mem marked;
+    DevBuf marked;
     int count = 0;
     LBM_CUDA_TRY(h->rows.alloc((size_t)9 * npad * sizeof(int32_t)));
     LBM_CUDA_TRY(marked.alloc(sizeof(int)));
@@ -316,7 +302,7 @@ lbm_status lbm_st7_get_populations(lbm_st7_handle* h, double* g) {
   if (!h || !g) return fail(LBM_ERR_ARG, "lbm_st7_get_populations: bad argument");
   LBM_CUDA_TRY(cudaSetDevice(h->device));
   const int n = h->geo.count;
-  Mem out;
+  DevBuf out;
   const size_t bytes = sizeof(double) * (size_t)(n + 1) * h->nq;
   LBM_CUDA_TRY(out.alloc(bytes));
   LBM_CUDA_TRY(cudaMemsetAsync(out.p, 0, bytes, h->stream));
@@ -330,7 +316,7 @@ lbm_status lbm_st7_set_state(lbm_st7_handle* h, const double* g, const double* c
   if (!h || !g || !c) return fail(LBM_ERR_ARG, "lbm_st7_set_state: bad argument");
   LBM_CUDA_TRY(cudaSetDevice(h->device));
   const int n = h->geo.count, npad = h->geo.npad;
-  Mem in;
+  DevBuf in;
   const size_t bytes = sizeof(double) * (size_t)(n + 1) * h->nq;
   LBM_CUDA_TRY(in.alloc(bytes));
   LBM_CUDA_TRY(cudaMemcpyAsync(in.p, g, bytes, cudaMemcpyHostToDevice, h->stream));

@@ -158,9 +158,13 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
     }
   }
   e = cudaMallocAsync(p, bytes, 0);
+  if (e != cudaSuccess) {
+    *p = nullptr;
+    cudaGetLastError();  // the caller has it: a later launch must not report it again
+    return e;
+  }
   // usable on every stream once the allocation on the legacy stream is done
-  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
-  return e;
+  return cudaStreamSynchronize(0);
 }
 
 void dev_free(void* p) {
