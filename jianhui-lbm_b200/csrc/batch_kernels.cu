@@ -58,9 +58,9 @@ __global__ void __launch_bounds__(BS, 640 / BS) batch_step_kernel(BatchStepArgs 
     F2 f[kQ];
     if constexpr (LOCAL) {
       step_wait();
-      load_row<K>(pop + p, inv_scale, f[0]);
+      load_row<K>(pop + p, inv_scale, true, f[0]);  // a tile's padding is its own
 #pragma unroll
-      for (int q = 1; q < kQ; q++) load_row<K>(pop + (size_t)opp(q) * cap + p, inv_scale, f[q]);
+      for (int q = 1; q < kQ; q++) load_row<K>(pop + (size_t)opp(q) * cap + p, inv_scale, true, f[q]);
     } else {
       int32_t s0[kQ], s1[kQ];
       if constexpr (ROWS) {

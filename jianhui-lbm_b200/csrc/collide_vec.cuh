@@ -117,13 +117,19 @@ __host__ __device__ constexpr bool first_moment(int k, int q) {
 }
 
 // Populations of one node, or of the nodes p and p + 1 of a row (p even).
+// both: node p + 1 is the launch's; else its slot may be another kernel's (the
+// face kernel's beside the step kernel) and is left alone, the first node's
+// value standing in for it.
 template <Store K>
-__device__ __forceinline__ void load_row(const typename Traits<K>::T* p, float inv_scale, float& v) {
+__device__ __forceinline__ void load_row(const typename Traits<K>::T* p, float inv_scale, bool, float& v) {
   v = load_pop_rw<K>(p, inv_scale);
 }
 template <Store K>
-__device__ __forceinline__ void load_row(const typename Traits<K>::T* p, float inv_scale, F2& v) {
-  if constexpr (K == Store::F16) {
+__device__ __forceinline__ void load_row(const typename Traits<K>::T* p, float inv_scale, bool both, F2& v) {
+  if (!both) {
+    const float first = load_pop_rw<K>(p, inv_scale);
+    v = make_f2(first, first);
+  } else if constexpr (K == Store::F16) {
     const float2 a = __half22float2(*reinterpret_cast<const __half2*>(p));
     v = vmul(make_f2(a.x, a.y), make_f2(inv_scale, inv_scale));
   } else {

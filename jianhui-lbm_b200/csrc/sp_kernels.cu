@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(BS, vec_min_blocks<V>(BS)) step_vec_kernel(Ste
   if constexpr (SL == Slots::Local) {
     step_wait();
 #pragma unroll
-    for (int q = 1; q < kQ; q++) load_row<K>(pop + (size_t)opp(q) * a.npad + p, inv_scale, f[q]);
+    for (int q = 1; q < kQ; q++) load_row<K>(pop + (size_t)opp(q) * a.npad + p, inv_scale, both, f[q]);
   } else if constexpr (N == 1) {
     int32_t slot[kQ];  // slot[q] holds f_q on entry and takes f*_opp(q)
     read_slots<SL>(cb, a, p, ow, slot);
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(BS, vec_min_blocks<V>(BS)) step_vec_kernel(Ste
   }
 
   if constexpr (N == 1 || PAIR)
-    load_row<K>(pop + p, inv_scale, f[0]);
+    load_row<K>(pop + p, inv_scale, both, f[0]);
   else
     f[0] = make_f2(load_pop_rw<K>(pop + p, inv_scale), load_pop_rw<K>(pop + p1, inv_scale));
 
