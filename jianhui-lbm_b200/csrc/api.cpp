@@ -142,14 +142,17 @@ struct lbm_handle {
   int last_p = -1;
   double fp16_scale = 1.0;
   double last_ms = 0.0;
-  cudaGraphExec_t graph = nullptr;  // captured step chain, from a kPull state
+  // captured step chains by starting phase; single_steps: steps launched one
+  // by one that a chain from a kLocal state would have covered
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};
+  int single_steps = 0;
   // false when the layout was built on the device and the host copies of the
   // compaction / node order (needed only for exports and re-layouts) are not
   // built yet
   bool host_geo = true;
 
   ~lbm_handle() {
-    if (graph) cudaGraphExecDestroy(graph);
+    drop_graphs();
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (ev_fork) cudaEventDestroy(ev_fork);
@@ -159,8 +162,10 @@ struct lbm_handle {
   }
   size_t mac_bytes() const { return (kind == Store::F64 || kind == Store::F64D) ? 8 : 4; }
   void drop_graphs() {
-    if (graph) cudaGraphExecDestroy(graph);
-    graph = nullptr;
+    for (auto& g : graph) {
+      if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
   }
 };
 
@@ -445,15 +450,14 @@ lbm_status one_step(lbm_handle* h, bool write) {
 }
 
 constexpr int kGraphSteps = 16;  // even: a replay leaves the phase unchanged
+constexpr int kCaptureSteps = 128;
 
-// The chain of kGraphSteps steps from a kPull state (a caller in the other
-// phase steps once first: capturing and instantiating a second chain costs
-// more than that step).
-lbm_status ensure_graph(lbm_handle* h) {
-  if (h->graph) return LBM_OK;
+// The chain of kGraphSteps steps from a state of phase c0.
+lbm_status ensure_graph(lbm_handle* h, int c0) {
+  if (h->graph[c0]) return LBM_OK;
   cudaGraph_t g = nullptr;
   LBM_CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  int c = kPull;
+  int c = c0;
   cudaError_t err = cudaSuccess;
   // (with faces the steps are joined by events)
   const bool chain = !h->bc.active && chain_pays(h->geo.count, h->mac_bytes() == 8 ? 148 * 256 : 148 * 1024);
@@ -472,7 +476,7 @@ lbm_status ensure_graph(lbm_handle* h) {
     return fail(LBM_ERR_CUDA, std::string("graph capture failed: ") +
                                   cudaGetErrorString(err != cudaSuccess ? err : end));
   }
-  const cudaError_t inst = cudaGraphInstantiate(&h->graph, g, 0);
+  const cudaError_t inst = cudaGraphInstantiate(&h->graph[c0], g, 0);
   cudaGraphDestroy(g);
   LBM_CUDA_TRY(inst);
   return LBM_OK;
@@ -485,19 +489,31 @@ lbm_status run_steps(lbm_handle* h, int nsteps) {
   // one, and the last of the call, which writes the pre-collision macro
   // fields (the velocity one step before the new state)
   int left = nsteps;
-  const bool lead_given = h->given_macro;
-  const int after_given = lead_given ? kLocal : h->cur;
-  const int lead = (lead_given ? 1 : 0) + (after_given == kLocal ? 1 : 0);
+  int lead = h->given_macro ? 1 : 0, from = lead ? kLocal : h->cur;
+  if (from == kLocal) {
+    // A chain from here, or one step and a chain from the kPull state after
+    // it: the same as long as the call has a step to spare.  Where it has not
+    // (every second call of 16 k + 1 steps), a chain's worth of steps would be
+    // launched one by one, 5 to 35 us a call (33 steps at 24^3 | 64^3 in FP32:
+    // 80 | 165 us, one by one 114 | 189); the other chain, about 160 us, is
+    // captured after kCaptureSteps such steps.
+    const int spare = nsteps - lead - 1;
+    if (!h->graph[kLocal] && spare / kGraphSteps > (spare - 1) / kGraphSteps) h->single_steps += kGraphSteps;
+    if (h->single_steps < kCaptureSteps) {
+      lead++;
+      from = kPull;
+    }
+  }
   const bool chains = nsteps - lead - 1 >= kGraphSteps;
   // capture before the start event: capture and instantiation are host work
   // and must not count as step time
-  if (chains && (st = ensure_graph(h)) != LBM_OK) return st;
+  if (chains && (st = ensure_graph(h, from)) != LBM_OK) return st;
   LBM_CUDA_TRY(cudaEventRecord(h->ev0, h->stream));
   if (chains) {
     for (int i = 0; i < lead; i++, left--)
       if ((st = one_step(h, false)) != LBM_OK) return st;
     for (; left - 1 >= kGraphSteps; left -= kGraphSteps) {
-      LBM_CUDA_TRY(cudaGraphLaunch(h->graph, h->stream));
+      LBM_CUDA_TRY(cudaGraphLaunch(h->graph[from], h->stream));
       h->step += kGraphSteps;
     }
   }
