@@ -105,7 +105,8 @@ typedef struct lbm_params {
   double u_init[3];   /* initial velocity inivx..inivz (SP3:1331-1333) */
   int precision;      /* lbm_precision */
   int ordering;       /* lbm_ordering (LBM_ORDER_AUTO allowed) */
-  int block_size;     /* threads per block; 0 = default, autotune may change */
+  int block_size;     /* nodes per thread block of the step: 64, 128, 256 or 512;
+                         0 = chosen by precision and size; autotune may change */
   int perdir;         /* PerDir 1..3: permeability direction (SP3:3560-3570) */
   int window[6];      /* per_xn,per_xp,per_yn,per_yp,per_zn,per_zp; all -1 = whole box */
   double fp16_scale;  /* LBM_PREC_F16 storage scale; 0 = derived from nu and |g| */
@@ -715,8 +716,10 @@ typedef struct lbm_batch lbm_batch;
  * contiguous tile-aligned node range, its pull table pointing only into its
  * own range) stepped by one persistent kernel per step inside CUDA graphs.
  * precision: LBM_PREC_F32 or LBM_PREC_F16; ordering: node order inside each
- * instance; block: 128/256/512 (0 = 256).  Replaces running the reference
- * binary once per subsample. */
+ * instance; block: nodes per pass of a step over a 512-node tile, 128, 256 or
+ * 512; 0 = autotuned at creation (lbm_batch_autotune), negative = chosen by the
+ * number of stepping tiles.  Replaces running the reference binary once per
+ * subsample. */
 LBM_API lbm_status lbm_batch_create(int n, const lbm_instance* inst, int precision, int ordering, int block,
                                     int device, lbm_batch** out);
 /* Runs every instance to convergence (or max_steps); instances that converge
@@ -750,7 +753,8 @@ typedef struct lbm_server_config {
   int max_active;            /* slots: solves resident at once */
   int precision;             /* LBM_PREC_F32 or LBM_PREC_F16 */
   int ordering;              /* node order inside each solve */
-  int block;                 /* step block size (0 = 256) */
+  int block;                 /* nodes per pass of a step, 128, 256 or 512; 0 = chosen
+                                by the number of stepping tiles */
   double tol;                /* stop test tolerance */
   int check_every;           /* steps per device chain between admissions */
   long long max_steps;       /* per-solve step cap */

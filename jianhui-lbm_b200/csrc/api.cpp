@@ -137,7 +137,7 @@ struct lbm_handle {
   bool uprev_valid = false;
   double perm_prev[3] = {0, 0, 0};
   int overspeed = 0;
-  int block = 256;
+  int block = 0;  // nodes per block asked for or autotuned; 0 = default_block
   int ordering = LBM_ORDER_REFERENCE;
   int last_p = -1;
   double fp16_scale = 1.0;
@@ -412,7 +412,7 @@ BcArgs bc_args(lbm_handle* h, const StepArgs& s, int c) {
 // runs on the side stream beside the step kernel and the step ends when both
 // have.
 cudaError_t launch_full_step(lbm_handle* h, const StepArgs& a, int c) {
-  const int block = h->block == 256 ? default_block(h->kind, a.n_main) : h->block;
+  const int block = h->block ? h->block : default_block(h->kind, a.n_main);
   if (!h->bc.active) return launch_step(h->kind, a, block, h->stream);
   cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
@@ -632,7 +632,7 @@ void lbm_params_default(lbm_params* p) {
   p->gx = 1e-6;
   p->precision = LBM_PREC_F32;
   p->ordering = LBM_ORDER_REFERENCE;
-  p->block_size = 256;
+  p->block_size = 0;
   p->perdir = 1;
   for (int i = 0; i < 6; i++) p->window[i] = -1;
   p->fp16_scale = 0.0;
@@ -661,7 +661,7 @@ lbm_status lbm_create(const lbm_params* p, const uint8_t* mask, int nx, int ny, 
   h->kind = store_of(p->precision);
   h->block = (p->block_size == 64 || p->block_size == 128 || p->block_size == 256 || p->block_size == 512)
                  ? p->block_size
-                 : 256;
+                 : 0;
   LBM_CUDA_TRY(cudaSetDevice(h->device));
   LBM_CUDA_TRY(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
   LBM_CUDA_TRY(cudaEventCreate(&h->ev0));
@@ -1079,7 +1079,7 @@ lbm_status lbm_autotune(lbm_handle* h, int trial_steps, int* ordering_out, int* 
   std::sort(cands.begin(), cands.end(), [](const Cand& x, const Cand& y) { return x.ml > y.ml; });
   if (cands.size() > 3) cands.resize(3);
   double best = -1.0;
-  int best_o = h->ordering, best_b = h->block;
+  int best_o = h->ordering, best_b = default_block(h->kind, n);
   bool best_ct = h->ct_on;
   for (Cand& c : cands) {
     if ((st = layout(h, c.o)) != LBM_OK) return st;

@@ -87,7 +87,7 @@ struct Pool {
   };
   std::vector<ChainRecord> trace;
   int cap = 0, ntiles = 0, nslots = 0;
-  int block = 256, grid = 0;
+  int block = 0, grid = 0;  // nodes per pass of the step asked for or autotuned (0: batch_block)
   int ordering = LBM_ORDER_REFERENCE;
   double fp16_scale = 1.0;
   DevBuf x_fields;  // field export
@@ -137,7 +137,7 @@ struct Pool {
   lbm_status init(Store k, long long cap_nodes, int slots, int blk, int dev, int order, double f16) {
     kind = k;
     device = dev;
-    block = (blk == 128 || blk == 512) ? blk : 256;
+    block = (blk == 128 || blk == 256 || blk == 512) ? blk : 0;
     ordering = order;
     fp16_scale = f16;
     const long long c = ((cap_nodes + kTile - 1) / kTile) * kTile;
@@ -349,7 +349,7 @@ struct Pool {
     cudaError_t err = launch_batch_list(reduce_args(c0), step_grid, block, stream);
     int c = c0;
     for (int s = 0; s < chain && err == cudaSuccess; s++) {
-      err = launch_batch_step(kind, step_args(c, step_grid), block, step_grid, s, stream);
+      err = launch_batch_step(kind, step_args(c, step_grid), block ? block : batch_block(step_grid), step_grid, s, stream);
       c = 1 - c;
     }
     if (err == cudaSuccess) err = launch_batch_check(kind, reduce_args(c), chain, tol, max_steps, stream);
@@ -647,7 +647,7 @@ lbm_status lbm_batch_autotune(lbm_batch* b, int trial_steps, int* ordering_out, 
   const int orders[2] = {LBM_ORDER_REFERENCE, LBM_ORDER_HILBERT};
   const int blocks[3] = {128, 256, 512};
   double best = -1;
-  int best_o = P.ordering, best_b = P.block;
+  int best_o = P.ordering, best_b = batch_block(P.ntiles);
   lbm_status st;
   for (int o : orders) {
     P.ordering = o;
@@ -679,7 +679,8 @@ lbm_status lbm_batch_autotune(lbm_batch* b, int trial_steps, int* ordering_out, 
     }
   }
   P.ordering = best_o;
-  P.block = best_b;
+  // the pool's own choice where it is that: it follows the grid as solves stop
+  P.block = best_b == batch_block(P.ntiles) ? 0 : best_b;
   P.grid = batch_step_grid(P.ntiles, best_b);
   if ((st = batch_layout(b)) != LBM_OK) return st;
   if ((st = batch_reset(b)) != LBM_OK) return st;
@@ -731,7 +732,7 @@ void lbm_server_config_default(lbm_server_config* c) {
   c->max_active = 256;
   c->precision = LBM_PREC_F32;
   c->ordering = LBM_ORDER_REFERENCE;
-  c->block = 256;
+  c->block = 0;
   c->tol = 1e-6;
   c->check_every = 100;
   c->max_steps = 1000000;

@@ -87,6 +87,11 @@ cudaError_t launch_batch_export_macro(Store kind, const void* pop, int phase, co
                                       cudaStream_t st);
 cudaError_t launch_batch_init(Store kind, void* pop, int phase, const int32_t* table, int cap, int begin, int n,
                               const InstParams& ip, cudaStream_t st);
+// Nodes per pass of the step where none was asked for: a tile in one pass
+// where there are too few tiles to fill the chip in two (one | two passes: 3.50
+// | 3.98 us per step at 5.5 K nodes, 4.25 | 4.73 at 44 K, 5.58 | 5.75 at 88 K,
+// 7.93 | 7.17 at 177 K, a grid of 512).
+constexpr int batch_block(int grid) { return grid <= 256 ? 512 : 256; }
 // Largest step grid of a pool: one block per tile of the pool (a block steps
 // its tile in kTile / block passes).
 int batch_step_grid(int ntiles, int block);

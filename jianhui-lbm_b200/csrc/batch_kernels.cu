@@ -334,13 +334,9 @@ static cudaError_t step_bs(const BatchStepArgs& a, int grid, int chain_step, cud
     return launch_chained(batch_step_kernel<K, BS, false, true>, grid, BS, st, chained, a, chain_step);
   return launch_chained(batch_step_kernel<K, BS, false, false>, grid, BS, st, chained, a, chain_step);
 }
-// `block` nodes a pass, two per thread; a tile in one pass where there are
-// too few tiles to fill the chip in two (one | two passes: 3.50 | 3.98 us per
-// step at 5.5 K nodes, 4.25 | 4.73 at 44 K, 5.58 | 5.75 at 88 K, 7.93 | 7.17 at
-// 177 K, a grid of 512).
+// `block` nodes a pass, two per thread.
 template <Store K>
 static cudaError_t step_k(const BatchStepArgs& a, int block, int grid, int chain_step, cudaStream_t st) {
-  if (grid <= 256) block = 512;
   switch (block) {
     case 128: return step_bs<K, 64>(a, grid, chain_step, st);
     case 512: return step_bs<K, 256>(a, grid, chain_step, st);

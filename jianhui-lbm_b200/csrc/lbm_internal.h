@@ -307,10 +307,11 @@ struct StepArgs {
   // written times lat_c)
   Lattice lat;
 };
-// Threads per block of the step where the caller left the default of 256: 64
-// for small solves, whose few large blocks leave SMs idle or give some twice
-// the work of others, and for the bit-exact FP64 step, whose blocks keep the
-// FP64 pipe busier when they end one by one.  us per step, 64 | 256 threads:
+// Nodes per block of the step where the caller asked for no size: 64 for small
+// solves, whose few large blocks leave SMs idle or give some twice the work of
+// others, and for the bit-exact FP64 step, whose blocks keep the FP64 pipe
+// busier when they end one by one.  (One thread per node; half as many threads
+// where a thread takes two nodes.)  us per step, 64 | 256 threads:
 // FP64 5 K nodes 4.28 | 5.66, 92 K 11.5 | 12.3, 310 K 28.2 | 30.9, 5.9 M 504 | 529;
 // FP64 deviation 5 K 2.15 | 3.00, 310 K 13.3 | 14.3, 734 K 45.5 | 43.8; FP32 5 K
 // 1.85 | 2.32, 49 K 3.12 | 3.51, 131 K 4.79 | 5.30 (above that two nodes per

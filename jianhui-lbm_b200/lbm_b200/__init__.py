@@ -640,9 +640,10 @@ def _instance(mask, nu, g):
 class Batch:
     """Many independent single-phase solves in one node pool on one GPU.
 
-    ``solves`` is a list of (mask, nu, g) tuples."""
+    ``solves`` is a list of (mask, nu, g) tuples.  ``block``: nodes per pass
+    of a step (128, 256, 512), -1 for the pool's own choice, 0 to autotune."""
 
-    def __init__(self, solves, precision="f32", ordering="reference", block=256, device=0):
+    def __init__(self, solves, precision="f32", ordering="reference", block=-1, device=0):
         keep = []
         arr = (Instance * len(solves))()
         for i, (mask, nu, g) in enumerate(solves):
@@ -712,10 +713,11 @@ class Batch:
 
 
 class Server:
-    """Continuous-batching permeability solve server on one GPU."""
+    """Continuous-batching permeability solve server on one GPU.  ``block``: nodes per pass of a step (128, 256,
+    512), 0 for the pool's own choice."""
 
     def __init__(self, capacity_nodes=64 * 1024 * 1024, max_active=256, precision="f32", ordering="reference",
-                 block=256, tol=1e-6, check_every=100, max_steps=1_000_000, device=0, target_active_nodes=0,
+                 block=0, tol=1e-6, check_every=100, max_steps=1_000_000, device=0, target_active_nodes=0,
                  policy="fifo"):
         c = ServerConfig()
         lib().lbm_server_config_default(C.byref(c))
@@ -868,10 +870,12 @@ class SinglePhase:
 
     ``mask`` is a (nz, ny, nx) uint8 array, 0 = pore.  ``g`` is the body
     force (acceleration), ``nu`` the kinematic viscosity (tau = 3 nu + 1/2).
+    ``block_size``: nodes per thread block (64, 128, 256, 512), 0 for the
+    solver's own choice.
     """
 
     def __init__(self, mask, nu, g=(1e-6, 0.0, 0.0), precision="f32", ordering="reference",
-                 block_size=256, u_init=(0.0, 0.0, 0.0), perdir=1, window=None, fp16_scale=0.0, device=0,
+                 block_size=0, u_init=(0.0, 0.0, 0.0), perdir=1, window=None, fp16_scale=0.0, device=0,
                  bc=None, _handle=None):
         self._h = None
         if _handle is not None:
