@@ -411,9 +411,15 @@ BcArgs bc_args(lbm_handle* h, const StepArgs& s, int c) {
 // face kernel the rest), and the previous step's record, so the face kernel
 // runs on the side stream beside the step kernel and the step ends when both
 // have.
-cudaError_t launch_full_step(lbm_handle* h, const StepArgs& a, int c) {
-  const int block = h->block ? h->block : default_block(h->kind, a.n_main);
+cudaError_t launch_full_step(lbm_handle* h, StepArgs a, int c) {
+  const int block = h->block ? h->block : default_block(h->kind, a.n_main, h->bc.active);
   if (!h->bc.active) return launch_step(h->kind, a, block, h->stream);
+  // One split of L1 and shared memory for the steps of both phases and the
+  // face kernel of small solves: left to the driver, an SM that a block of one
+  // of them runs on takes no block of another.  us per step, without | with
+  // it: FP64 44^3 20.4 | 19.3, 56^3 22.4 | 20.5, FP32 44^3 4.1 | 3.8, 56^3
+  // 5.0 | 4.6 (128^3 25.0 | 26.0: not there).
+  if (a.n_main < 148 * 1024) a.carveout = 50;
   cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
   if (e == cudaSuccess) e = launch_boundary(h->kind, bc_args(h, a, c), h->side);

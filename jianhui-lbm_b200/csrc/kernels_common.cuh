@@ -67,24 +67,44 @@ struct Traits<Store::F16> {
 __device__ __forceinline__ void step_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+//
+// carveout: percent of an SM's L1 that the launch asks for as shared memory
+// (0: the driver's choice by kernel).  An SM changes the split only when it is
+// empty, so kernels that run beside each other have to ask for the same.
 template <typename Args, typename... More>
-cudaError_t launch_chained(void (*kernel)(Args, More...), int grid, int block, cudaStream_t st, bool chained,
-                           const Args& a, More... more) {
-  if (!chained) {
-    kernel<<<grid, block, 0, st>>>(a, more...);
-    return cudaGetLastError();
-  }
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
+cudaError_t launch_with(void (*kernel)(Args, More...), int grid, int block, cudaStream_t st, bool chained,
+                        int carveout, const Args& a, More... more) {
+  cudaLaunchAttribute at[2];
   cudaLaunchConfig_t c{};
   c.gridDim = dim3((unsigned)grid);
   c.blockDim = dim3((unsigned)block);
   c.stream = st;
-  c.attrs = &at;
-  c.numAttrs = 1;
+  c.attrs = at;
+  if (chained) {
+    at[c.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[c.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (carveout > 0) {
+    at[c.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at[c.numAttrs++].val.sharedMemCarveout = (unsigned)carveout;
+  }
   return cudaLaunchKernelEx(&c, kernel, a, more...);
 }
+template <typename Args, typename... More>
+cudaError_t launch_chained(void (*kernel)(Args, More...), int grid, int block, cudaStream_t st, bool chained,
+                           const Args& a, More... more) {
+  return launch_with(kernel, grid, block, st, chained, 0, a, more...);
+}
+inline cudaError_t launch_step_kernel(void (*kernel)(StepArgs), int grid, int block, cudaStream_t st,
+                                      const StepArgs& a) {
+  return launch_with(kernel, grid, block, st, a.chained != 0, a.carveout, a);
+}
+// Threads per block of a face kernel over nb nodes: few enough blocks that
+// most SMs are left to the step beside it, and no more threads than that, as
+// the threads of a block wait for one FP64 unit.  us per FP64 step with
+// pressure faces at x, 32 | 64 | 128 threads: 820 face nodes (32^3) 18.1 | 18.3
+// | 18.7, 2.5 K (56^3) 24.3 | 19.0 | 20.6, 3.3 K (64^3) 28.2 | 24.6 | 22.5.
+constexpr int face_block(int nb) { return nb <= 1024 ? 32 : nb <= 3000 ? 64 : 128; }
 
 // Read-only (non-coherent) loads, for the table and for populations that the
 // launch does not write.

@@ -271,6 +271,7 @@ struct StepArgs {
   const int32_t* rows;   // [9][npad] row form of the table (row_table.cuh), or null
   int ahead;             // nodes ahead that a block prefetches into L2, 0 = none
   int chained;           // launched as a programmatic dependent of the step before it
+  int carveout;          // percent of an SM's L1 to ask for as shared memory, 0 = the driver's choice
   int n;                 // fluid nodes
   int npad;
   // macro input for a step that must use given rho/u (first step after init
@@ -316,7 +317,15 @@ struct StepArgs {
 // FP64 deviation 5 K 2.15 | 3.00, 310 K 13.3 | 14.3, 734 K 45.5 | 43.8; FP32 5 K
 // 1.85 | 2.32, 49 K 3.12 | 3.51, 131 K 4.79 | 5.30 (above that two nodes per
 // thread, 310 K 7.99 | 7.82).
-constexpr int default_block(Store kind, long long n) {
+//
+// Beside a face kernel (faces) the FP64 step's smaller blocks would spread over
+// the face kernel's SMs as well: 256 | 128 | 64, FP64 with pressure faces, 70 K
+// nodes 19.0 | 19.2 | 20.4, 105 K 22.5 | 23.4 | 23.4, 149 K 25.4 | 24.4 | 24.6,
+// 354 K 49.9 | 46.6 | 48.4; FP32 (256 | 128 | 64) 34 K 4.0 | 3.9 | 3.85, 105 K
+// 5.7 | 5.6 | 5.9, 149 K 6.8 | 6.7 | 6.9.
+constexpr int default_block(Store kind, long long n, bool faces = false) {
+  if (faces && kind == Store::F64) return n < 148 * 850 ? 256 : 128;
+  if (faces && (kind == Store::F32 || kind == Store::F16) && n >= 148 * 512 && n < 148 * 1024) return 128;
   return kind == Store::F64 || n < (kind == Store::F64D ? 400000 : 148 * 1024) ? 64 : 256;
 }
 

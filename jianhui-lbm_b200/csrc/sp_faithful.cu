@@ -478,13 +478,24 @@ __global__ void __launch_bounds__(BS, f64_min_blocks(BS)) step_f64_faithful(Step
 // a.bnd_f set: only the populations after the rules (current state).  LAT:
 // a self-defined lattice (the rules' equilibria, the macro step and the
 // collision on it).
-template <bool GIVEN, bool FINAL, bool LAT, bool LOCAL>
-__global__ void __launch_bounds__(128) bc_f64_faithful(BcArgs a) {
-  const int b = blockIdx.x * 128 + threadIdx.x;
+// One kernel for both phases: the few warps of a face run their thousands of
+// instructions once, so what they wait for is instructions, and a second
+// kernel would take the first one's place in the caches every step.
+template <int BS, bool GIVEN, bool FINAL, bool LAT>
+__global__ void __launch_bounds__(BS, GIVEN ? 1 : 512 / BS) bc_f64_faithful(BcArgs a) {
+  const int b = blockIdx.x * BS + threadIdx.x;
   const int p = a.s.n_main + b;
   if (p >= a.s.n) return;
+  __shared__ int32_t keep[FINAL ? 1 : kQ - 1][FINAL ? 1 : BS];  // slot of f_q, which takes f*_opp(q) in both phases
+  const double* pop = static_cast<const double*>(a.s.pop);
   double f[kQ];
-  pull_f64<LOCAL>(a.s, p, f);
+  f[0] = pop[p];
+#pragma unroll
+  for (int q = 1; q < kQ; q++) {
+    const int32_t s = state_slot(a.s.phase, a.s.table, a.s.npad, p, q);
+    f[q] = pop[s];
+    if constexpr (!FINAL) keep[q - 1][threadIdx.x] = s;
+  }
   if (!GIVEN) bc_apply(a, b, f, a.s.lat);
   if (FINAL) {
     const size_t nb = (size_t)(a.s.n - a.s.n_main);
@@ -497,32 +508,29 @@ __global__ void __launch_bounds__(128) bc_f64_faithful(BcArgs a) {
   snap_write(a.s.snap_dst, a.s.nsnap, p - a.s.snap_begin, f, rho, ux, uy, uz);
   double m[kQ];
   moments_by_column(m, f, QSeq{});
-  collide_moments<false, LAT, LOCAL>(m, rho, ux, uy, uz, a.s, p, [&](int q) {
-    return __ldg(a.s.table + (size_t)(q - 1) * a.s.npad + p);
-  });
+  if constexpr (!FINAL)
+    collide_moments<false, LAT, false>(m, rho, ux, uy, uz, a.s, p, [&](int q) { return keep[q - 1][threadIdx.x]; });
 }
 
-template <bool LAT, bool LOCAL>
-static void launch_bc_f64(const BcArgs& a, int grid, cudaStream_t st) {
-  if (a.bnd_f)
-    bc_f64_faithful<false, true, LAT, LOCAL><<<grid, 128, 0, st>>>(a);
-  else if (a.s.rho_in != nullptr)
-    bc_f64_faithful<true, false, LAT, false><<<grid, 128, 0, st>>>(a);  // a given state is a kPull state
-  else
-    bc_f64_faithful<false, false, LAT, LOCAL><<<grid, 128, 0, st>>>(a);
+template <bool LAT>
+static cudaError_t launch_bc_f64(const BcArgs& a, int nb, cudaStream_t st) {
+  auto run = [&](void (*kernel)(BcArgs), int bs) {
+    return launch_with(kernel, (nb + bs - 1) / bs, bs, st, false, a.s.carveout, a);
+  };
+  if (a.bnd_f) return run(bc_f64_faithful<128, false, true, LAT>, 128);
+  if (a.s.rho_in != nullptr) return run(bc_f64_faithful<128, true, false, LAT>, 128);
+  switch (face_block(nb)) {
+    case 32: return run(bc_f64_faithful<32, false, false, LAT>, 32);
+    case 64: return run(bc_f64_faithful<64, false, false, LAT>, 64);
+    default: return run(bc_f64_faithful<128, false, false, LAT>, 128);
+  }
 }
 
 cudaError_t launch_boundary_f64(const BcArgs& a, cudaStream_t st) {
   const int nb = a.s.n - a.s.n_main;
   if (nb <= 0) return cudaSuccess;
-  const int grid = (nb + 127) / 128;
-  const bool local = a.s.phase == kLocal;
-  if (local && a.s.rho_in != nullptr) return cudaErrorInvalidValue;
-  if (a.s.lat.on)
-    local ? launch_bc_f64<true, true>(a, grid, st) : launch_bc_f64<true, false>(a, grid, st);
-  else
-    local ? launch_bc_f64<false, true>(a, grid, st) : launch_bc_f64<false, false>(a, grid, st);
-  return cudaGetLastError();
+  if (a.s.phase == kLocal && a.s.rho_in != nullptr) return cudaErrorInvalidValue;  // a given state is a kPull state
+  return a.s.lat.on ? launch_bc_f64<true>(a, nb, st) : launch_bc_f64<false>(a, nb, st);
 }
 
 // final pass of the diagnostics reduction (shared by all kinds)
@@ -543,18 +551,18 @@ static cudaError_t launch_f64_bs(const StepArgs& a, cudaStream_t st) {
   if (a.phase == kLocal) {
     if (given) return cudaErrorInvalidValue;  // a given state is a kPull state
     if (write)
-      return launch_chained(step_f64_faithful<BS, false, true, GX, LAT, true, false>, grid, BS, st, a.chained != 0, a);
-    return launch_chained(step_f64_faithful<BS, false, false, GX, LAT, true, false>, grid, BS, st, a.chained != 0, a);
+      return launch_step_kernel(step_f64_faithful<BS, false, true, GX, LAT, true, false>, grid, BS, st, a);
+    return launch_step_kernel(step_f64_faithful<BS, false, false, GX, LAT, true, false>, grid, BS, st, a);
   } else if (given && write) {
-    return launch_chained(step_f64_faithful<BS, true, true, GX, LAT, false, false>, grid, BS, st, a.chained != 0, a);
+    return launch_step_kernel(step_f64_faithful<BS, true, true, GX, LAT, false, false>, grid, BS, st, a);
   } else if (given) {
-    return launch_chained(step_f64_faithful<BS, true, false, GX, LAT, false, false>, grid, BS, st, a.chained != 0, a);
+    return launch_step_kernel(step_f64_faithful<BS, true, false, GX, LAT, false, false>, grid, BS, st, a);
   } else if (write) {
-    return a.rows ? launch_chained(step_f64_faithful<BS, false, true, GX, LAT, false, true>, grid, BS, st, a.chained != 0, a)
-           : launch_chained(step_f64_faithful<BS, false, true, GX, LAT, false, false>, grid, BS, st, a.chained != 0, a);
+    return a.rows ? launch_step_kernel(step_f64_faithful<BS, false, true, GX, LAT, false, true>, grid, BS, st, a)
+           : launch_step_kernel(step_f64_faithful<BS, false, true, GX, LAT, false, false>, grid, BS, st, a);
   } else {
-    return a.rows ? launch_chained(step_f64_faithful<BS, false, false, GX, LAT, false, true>, grid, BS, st, a.chained != 0, a)
-           : launch_chained(step_f64_faithful<BS, false, false, GX, LAT, false, false>, grid, BS, st, a.chained != 0, a);
+    return a.rows ? launch_step_kernel(step_f64_faithful<BS, false, false, GX, LAT, false, true>, grid, BS, st, a)
+           : launch_step_kernel(step_f64_faithful<BS, false, false, GX, LAT, false, false>, grid, BS, st, a);
   }
 }
 

@@ -339,24 +339,32 @@ __global__ void __launch_bounds__(BS, vec_min_blocks<V>(BS)) step_vec_kernel(Ste
 }
 
 // Face nodes in deviation storage: the rules act on full populations in
-// double, the macro step and collision are the step kernel's.
-template <Store K, bool GIVEN, bool FINAL>
-__global__ void __launch_bounds__(128) bc_dev_kernel(BcArgs a) {
+// double, the macro step and collision are the step kernel's.  The slots are
+// kept for the stores, as in the step: read from the table again they are 18
+// more loads in a row.
+template <Store K, int BS, bool GIVEN, bool FINAL>
+__global__ void __launch_bounds__(BS, 512 / BS) bc_dev_kernel(BcArgs a) {
   using T = typename Traits<K>::T;
   using A = typename Traits<K>::A;
   using Mac = typename Traits<K>::Mac;
-  const int b = blockIdx.x * 128 + threadIdx.x;
+  const int b = blockIdx.x * BS + threadIdx.x;
   const int p = a.s.n_main + b;
   if (p >= a.s.n) return;
   const StepArgs& s = a.s;
   T* pop = static_cast<T*>(s.pop);
   const float scale = (float)s.fp16_scale;
-  const float inv_scale = (float)(1.0 / s.fp16_scale);
+  const float inv_scale = s.fp16_inv;
+  __shared__ SlotKeep<FINAL ? 1 : BS, 1> keep;  // slot[q] holds f_q and takes f*_opp(q), in both phases
   double F[kQ];
-  F[0] = to_full<K>(load_pop_rw<K>(pop + p, inv_scale), 0);
+  {
+    int32_t slot[kQ];
 #pragma unroll
-  for (int q = 1; q < kQ; q++)
-    F[q] = to_full<K>(load_pop_rw<K>(pop + state_slot(s.phase, s.table, s.npad, p, q), inv_scale), q);
+    for (int q = 1; q < kQ; q++) slot[q] = state_slot(s.phase, s.table, s.npad, p, q);
+    F[0] = to_full<K>(load_pop_rw<K>(pop + p, inv_scale), 0);
+#pragma unroll
+    for (int q = 1; q < kQ; q++) F[q] = to_full<K>(load_pop_rw<K>(pop + slot[q], inv_scale), q);
+    if constexpr (!FINAL) keep_slots(keep, threadIdx.x, [&](int q) { return slot[q]; });
+  }
   // the rules on the default lattice: velocities here are in units of lat_c
   if (!GIVEN) bc_apply(a, b, F, Lattice{});
   if (FINAL) {
@@ -401,23 +409,24 @@ __global__ void __launch_bounds__(128) bc_dev_kernel(BcArgs a) {
   else
     mrt_collide_dev<A>(f, ps, drho, rho, ux, uy, uz, A(s.gx), A(s.gy), A(s.gz), A(s.s_v), A(s.s_o));
   store_pop<K>(pop + p, f[0], scale);
-#pragma unroll
-  for (int q = 1; q < kQ; q++)
-    store_pop<K>(pop + state_slot(s.phase, s.table, s.npad, p, opp(q)), f[q], scale);
+  if constexpr (!FINAL)
+    for_kept_slots(keep, threadIdx.x, [&](int q, int32_t slot) { store_pop<K>(pop + slot, f[opp(q)], scale); });
 }
 
 template <Store K>
 static cudaError_t launch_bc_dev(const BcArgs& a, cudaStream_t st) {
   const int nb = a.s.n - a.s.n_main;
   if (nb <= 0) return cudaSuccess;
-  const int grid = (nb + 127) / 128;
-  if (a.bnd_f)
-    bc_dev_kernel<K, false, true><<<grid, 128, 0, st>>>(a);
-  else if (a.s.rho_in != nullptr)
-    bc_dev_kernel<K, true, false><<<grid, 128, 0, st>>>(a);
-  else
-    bc_dev_kernel<K, false, false><<<grid, 128, 0, st>>>(a);
-  return cudaGetLastError();
+  auto run = [&](void (*kernel)(BcArgs), int bs) {
+    return launch_with(kernel, (nb + bs - 1) / bs, bs, st, false, a.s.carveout, a);
+  };
+  if (a.bnd_f) return run(bc_dev_kernel<K, 128, false, true>, 128);
+  if (a.s.rho_in != nullptr) return run(bc_dev_kernel<K, 128, true, false>, 128);
+  switch (face_block(nb)) {
+    case 32: return run(bc_dev_kernel<K, 32, false, false>, 32);
+    case 64: return run(bc_dev_kernel<K, 64, false, false>, 64);
+    default: return run(bc_dev_kernel<K, 128, false, false>, 128);
+  }
 }
 
 cudaError_t launch_boundary(Store kind, const BcArgs& a, cudaStream_t st) {
@@ -435,22 +444,22 @@ static cudaError_t launch_f64d(const StepArgs& a, int grid, cudaStream_t st) {
   const bool given = a.rho_in != nullptr, write = a.rho_out != nullptr;
   if constexpr (SL != Slots::Local) {
     if (given)
-      return write ? launch_chained(step_dev_kernel<BS, true, true, SL>, grid, BS, st, a.chained != 0, a)
-                   : launch_chained(step_dev_kernel<BS, true, false, SL>, grid, BS, st, a.chained != 0, a);
+      return write ? launch_step_kernel(step_dev_kernel<BS, true, true, SL>, grid, BS, st, a)
+                   : launch_step_kernel(step_dev_kernel<BS, true, false, SL>, grid, BS, st, a);
   }
-  return write ? launch_chained(step_dev_kernel<BS, false, true, SL>, grid, BS, st, a.chained != 0, a)
-        : launch_chained(step_dev_kernel<BS, false, false, SL>, grid, BS, st, a.chained != 0, a);
+  return write ? launch_step_kernel(step_dev_kernel<BS, false, true, SL>, grid, BS, st, a)
+        : launch_step_kernel(step_dev_kernel<BS, false, false, SL>, grid, BS, st, a);
 }
 template <Store K, int BS, typename V, Slots SL>
 static cudaError_t launch_vec(const StepArgs& a, int grid, cudaStream_t st) {
   const bool given = a.rho_in != nullptr, write = a.rho_out != nullptr;
   if constexpr (SL != Slots::Local && VecOf<V>::kNodes == 1) {
     if (given)
-      return write ? launch_chained(step_vec_kernel<K, BS, V, true, true, SL>, grid, BS, st, a.chained != 0, a)
-                   : launch_chained(step_vec_kernel<K, BS, V, true, false, SL>, grid, BS, st, a.chained != 0, a);
+      return write ? launch_step_kernel(step_vec_kernel<K, BS, V, true, true, SL>, grid, BS, st, a)
+                   : launch_step_kernel(step_vec_kernel<K, BS, V, true, false, SL>, grid, BS, st, a);
   }
-  return write ? launch_chained(step_vec_kernel<K, BS, V, false, true, SL>, grid, BS, st, a.chained != 0, a)
-        : launch_chained(step_vec_kernel<K, BS, V, false, false, SL>, grid, BS, st, a.chained != 0, a);
+  return write ? launch_step_kernel(step_vec_kernel<K, BS, V, false, true, SL>, grid, BS, st, a)
+        : launch_step_kernel(step_vec_kernel<K, BS, V, false, false, SL>, grid, BS, st, a);
 }
 
 template <Store K, int BS>
