@@ -411,7 +411,7 @@ BcArgs bc_args(lbm_handle* h, const StepArgs& s, int c) {
 // face kernel the rest), and the previous step's record, so the face kernel
 // runs on the side stream beside the step kernel and the step ends when both
 // have.
-cudaError_t launch_full_step(lbm_handle* h, StepArgs a, int c) {
+cudaError_t launch_full_step(lbm_handle* h, StepArgs& a, int c) {
   const int block = h->block ? h->block : default_block(h->kind, a.n_main, h->bc.active);
   if (!h->bc.active) return launch_step(h->kind, a, block, h->stream);
   // One split of L1 and shared memory for the steps of both phases and the
@@ -446,8 +446,13 @@ lbm_status finalize_faces(lbm_handle* h, int* n_main, const double** bnd_f) {
   return LBM_OK;
 }
 
-lbm_status one_step(lbm_handle* h, bool write) {
-  const StepArgs a = step_args(h, write);
+// With faces the steps are joined by events.
+bool chained_steps(const lbm_handle* h) { return !h->bc.active && chain_pays(h->kind, h->geo.count); }
+
+// follows: launched right after another step.
+lbm_status one_step(lbm_handle* h, bool write, bool follows) {
+  StepArgs a = step_args(h, write);
+  a.chained = follows && chained_steps(h);
   LBM_CUDA_TRY(launch_full_step(h, a, h->cur));
   h->cur = 1 - h->cur;
   h->given_macro = false;
@@ -465,12 +470,10 @@ lbm_status ensure_graph(lbm_handle* h, int c0) {
   LBM_CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   int c = c0;
   cudaError_t err = cudaSuccess;
-  // (with faces the steps are joined by events)
-  const bool chain = !h->bc.active && chain_pays(h->geo.count, h->mac_bytes() == 8 ? 148 * 256 : 148 * 1024);
   for (int s = 0; s < kGraphSteps && err == cudaSuccess; s++) {
     StepArgs a = step_args(h, false);
     a.phase = c;
-    a.chained = s > 0 && chain;
+    a.chained = s > 0 && chained_steps(h);
     a.rho_in = a.u_in = nullptr;
     if (h->bc.active) a.snap_dst = h->snap[1 - c].as<double>();
     err = launch_full_step(h, a, c);
@@ -517,16 +520,14 @@ lbm_status run_steps(lbm_handle* h, int nsteps) {
   LBM_CUDA_TRY(cudaEventRecord(h->ev0, h->stream));
   if (chains) {
     for (int i = 0; i < lead; i++, left--)
-      if ((st = one_step(h, false)) != LBM_OK) return st;
+      if ((st = one_step(h, false, i > 0)) != LBM_OK) return st;
     for (; left - 1 >= kGraphSteps; left -= kGraphSteps) {
       LBM_CUDA_TRY(cudaGraphLaunch(h->graph[from], h->stream));
       h->step += kGraphSteps;
     }
   }
-  while (left > 0) {
-    if ((st = one_step(h, left == 1)) != LBM_OK) return st;
-    left--;
-  }
+  for (bool follows = false; left > 0; left--, follows = true)
+    if ((st = one_step(h, left == 1, follows)) != LBM_OK) return st;
   h->uprev_valid = true;
   LBM_CUDA_TRY(cudaEventRecord(h->ev1, h->stream));
   LBM_CUDA_TRY(cudaEventSynchronize(h->ev1));

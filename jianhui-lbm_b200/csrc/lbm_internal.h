@@ -364,17 +364,23 @@ constexpr int prefetch_ahead(long long n, long long pop_bytes, long long table_b
   return n * (pop_bytes + table_bytes) > (120LL << 20) ? 148 * 640 : 0;
 }
 
-// Whether the steps of a chain are launched as programmatic dependents
-// (kernels_common.cuh), for n nodes and `full` nodes from which the chip is
-// full.  The next step's blocks then start in the slots the running one
-// leaves, which saves a launch gap per step, but where the two together
-// neither leave SMs free nor fill them they land unevenly.  us per step,
-// chained | not, cubes at porosity 0.35:
-//   FP32  5 K nodes 2.27 | 2.72, 22 K 2.85 | 2.82, 49 K 4.00 | 3.47, 101 K
-//         5.07 | 4.23, 131 K 5.25 | 5.25, 179 K 5.14 | 5.52, 310 K 7.83 | 8.21,
-//         734 K 17.0 | 18.1, 5.9 M 161 | 164
-//   FP64  11 K 5.82 | 6.17, 22 K 7.49 | 6.29, 39 K 8.57 | 8.72, 92 K 12.2 | 12.6
-constexpr bool chain_pays(long long n, long long full) { return n <= 74 * 256 || n >= full; }
+// Whether successive steps are launched as programmatic dependents
+// (kernels_common.cuh), for n nodes.  The next step's blocks then start in the
+// slots the running one leaves, which saves a launch gap per step, but where
+// the two together neither leave SMs free nor fill them they land unevenly.  us
+// per step at the default block size, chained | not, porosity 0.35:
+//   FP32  10 K nodes 1.93 | 2.38, 21 K 2.19 | 2.63, 37 K 2.63 | 3.00, 49 K 3.30 | 3.26,
+//         71 K 4.03 | 3.66, 102 K 4.99 | 4.43, 126 K 5.25 | 4.96, 157 K 5.39 | 5.58, 310 K
+//         7.78 | 8.09, 734 K 17.3 | 18.1 (FP16 the same within 6 %)
+//   FP64  10 K 5.30 | 5.84, 18 K 5.91 | 6.23, 22 K 6.90 | 6.13, 32 K 7.87 | 6.48, 53 K
+//         8.79 | 7.62, 66 K 8.95 | 8.78, 71 K 8.46 | 9.15, 126 K 13.2 | 13.8, 734 K
+//         65.8 | 67.6
+// FP64 deviation storage gains 2 to 20 % and loses up to 3 % about 20 K; the
+// solutes (st7_api.cpp) gain at every size.
+constexpr bool chain_pays(Store kind, long long n) {
+  return kind == Store::F64D ||
+         (kind == Store::F64 ? n <= 148 * 128 || n >= 148 * 480 : n <= 148 * 256 || n >= 148 * 1024);
+}
 
 constexpr int kSnapRows = kQ + 4;  // per-step record of a node: f_0..f_18, rho, ux, uy, uz
 

@@ -99,7 +99,10 @@ constexpr int kSoluteGraphSteps = 16;  // even: a replay leaves the phase unchan
 constexpr int kSoluteCaptureSteps = 128;
 
 // A chain of steps from phase c0, captured once (launched one by one, steps
-// of small solves wait on the host: 4.1 us per step at 48^3).
+// of small solves wait on the host: 4.1 us per step at 48^3).  Steps that follow
+// one another are programmatic dependents (kernels_common.cuh) at every size:
+// us per step, chained | not, D3Q7 FP32 24^3 1.66 | 2.18, 48^3 2.43 | 2.82, 96^3 4.37
+// | 4.77, 160^3 13.8 | 14.3, D3Q19 FP64 24^3 3.33 | 3.71, 128^3 50.6 | 52.9.
 lbm_status solute_graph(lbm_st7_handle* h, int c0) {
   if (h->graph[c0]) return LBM_OK;
   cudaGraph_t g = nullptr;
@@ -108,7 +111,7 @@ lbm_status solute_graph(lbm_st7_handle* h, int c0) {
   St7Args a = st7_args(h, false);
   for (int s = 0; s < kSoluteGraphSteps && err == cudaSuccess; s++) {
     a.phase = (c0 + s) & 1;
-    a.chained = s > 0 && chain_pays(h->geo.count, 148 * 1024);
+    a.chained = s > 0;
     err = st7_launch_step(h->f64, a, h->stream);
   }
   const cudaError_t end = cudaStreamEndCapture(h->stream, &g);
@@ -279,13 +282,18 @@ lbm_status lbm_st7_step(lbm_st7_handle* h, int nsteps) {
     }
   }
   LBM_CUDA_TRY(cudaEventRecord(h->ev0, h->stream));
+  bool follows = false;  // the launch before was a single step
   for (int left = nsteps; left > 0;) {
     if (!h->given && left >= kSoluteGraphSteps && h->graph[c]) {
       LBM_CUDA_TRY(cudaGraphLaunch(h->graph[c], h->stream));
       left -= kSoluteGraphSteps;
+      follows = false;
       continue;
     }
-    LBM_CUDA_TRY(st7_launch_step(h->f64, st7_args(h, h->given), h->stream));
+    St7Args a = st7_args(h, h->given);
+    a.chained = follows;
+    LBM_CUDA_TRY(st7_launch_step(h->f64, a, h->stream));
+    follows = true;
     h->cur = 1 - h->cur;
     h->given = false;
     left--;

@@ -37,3 +37,26 @@ def test_faces_with_two_nodes_per_thread(precision, bar, odd):
         assert np.array_equal(a, b)
     _, _, u64 = run("f64", 0)
     assert np.abs(got[2] - u64).max() <= bar * np.abs(u64).max()
+
+
+# Cubes in, below and above the sizes whose steps are not chained (19 K to 71 K
+# nodes in FP64, 38 K to 152 K in FP32 and FP16), and boxes above 120 MiB of
+# populations and table, where blocks prefetch (1.1 M nodes in FP16, 0.85 M in
+# FP32, 0.56 M in FP64).
+@pytest.mark.parametrize("shape,phi", [((17, 16, 19), 0.8), ((33, 35, 39), 0.8), ((45, 47, 51), 0.9),
+                                       ((128, 121, 119), 0.7)])
+@pytest.mark.parametrize("precision", ["f32", "f16", "f64", "f64fast"])
+def test_a_call_equals_its_steps_one_by_one(precision, shape, phi):
+    """Captured chains, single steps that follow one another and lone steps
+    give the same bits."""
+    mask = spheres(shape, phi, 4.5, seed=8)
+    kw = dict(g=(1e-5, 4e-6, -3e-6), precision=precision)
+    with L.SinglePhase(mask, 0.1, **kw) as a, L.SinglePhase(mask, 0.1, **kw) as b:
+        for n in (37, 15, 33):
+            a.step(n)
+        for _ in range(85):
+            b.step(1)
+        assert np.array_equal(a.populations(), b.populations())
+        for x, y in zip(a.fields(), b.fields()):
+            assert np.array_equal(x, y)
+        assert a.reduce() == b.reduce()
