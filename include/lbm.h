@@ -302,8 +302,8 @@ LBM_API lbm_status lbm_release_cached_memory(void);
 
 /* Form of the pull table the step kernel reads (the reference's nei_loc,
  * SP3:1099-1151, as a pull table).  compact = 0 (default): the int32 table,
- * which large solves in the reference's node order read in a 36-byte row
- * form of their own choice.
+ * which large FP32 solves in the reference's node order read in a 36-byte
+ * row form of their own choice.
  * compact = 1: per aligned group of 32 nodes and direction one int32 base
  * and per node a 16-bit offset from it, 18*2 + 18*4/32 bytes per node
  * instead of 18*4; groups whose sources spread wider than the offsets reach

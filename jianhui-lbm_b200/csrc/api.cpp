@@ -121,12 +121,11 @@ struct lbm_handle {
   bool ct_ok = false;
   bool ct_on = false;  // the int32 table unless chosen (lbm_set_table_mode, lbm_autotune)
   double ct_wide_frac = 1.0;
-  // row form of the pull table, built with every layout of a solve that is
-  // large enough; read instead of the int32 table when few enough nodes are
-  // marked
-  DevBuf rows, rows_marked;
+  // row form of the pull table, built with every layout of an FP32 solve that
+  // is large enough and kept when few enough nodes are marked; read instead of
+  // the int32 table
+  DevBuf rows;
   int marked = 0;
-  bool rows_on() const { return rows.p != nullptr && rows_pay(marked, geo.count); }
   // field export: device buffers kept between calls
   DevBuf x_rint, x_uint, x_rref, x_uref;
   // phase of the populations (kPull / kLocal); with faces also the record of
@@ -201,18 +200,18 @@ lbm_status build_compact_table(lbm_handle* h) {
   return LBM_OK;
 }
 
-// Builds the row form of the table; h->marked is set when the stream has
-// been waited for.
+// Builds the row form of the table, and keeps it where it pays.
 lbm_status build_rows(lbm_handle* h) {
-  if (!rows_large(h->geo.count, kQ * (long long)store_bytes(h->kind))) return LBM_OK;
-  if (!h->rows.p) {
-    LBM_CUDA_TRY(h->rows.alloc((size_t)9 * h->geo.npad * sizeof(int32_t)));
-    LBM_CUDA_TRY(h->rows_marked.alloc(sizeof(int)));
-  }
-  LBM_CUDA_TRY(cudaMemsetAsync(h->rows_marked.p, 0, sizeof(int), h->stream));
-  LBM_CUDA_TRY(launch_row_table(h->table.as<int32_t>(), h->geo.npad, 0, h->geo.count, h->rows.as<int32_t>(),
-                                h->rows_marked.as<int>(), h->stream));
-  LBM_CUDA_TRY(cudaMemcpyAsync(&h->marked, h->rows_marked.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  if (h->kind != Store::F32 || !rows_large(h->geo.count, kQ * (long long)store_bytes(h->kind))) return LBM_OK;
+  DevBuf marked;
+  if (!h->rows.p) LBM_CUDA_TRY(h->rows.alloc((size_t)9 * h->geo.npad * sizeof(int32_t)));
+  LBM_CUDA_TRY(marked.alloc(sizeof(int)));
+  LBM_CUDA_TRY(cudaMemsetAsync(marked.p, 0, sizeof(int), h->stream));
+  LBM_CUDA_TRY(launch_row_table(h->table.as<int32_t>(), h->geo.npad, h->geo.count, h->rows.as<int32_t>(),
+                                marked.as<int>(), h->stream));
+  LBM_CUDA_TRY(cudaMemcpyAsync(&h->marked, marked.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
+  if (!rows_pay(h->marked, h->geo.count)) h->rows.release();
   return LBM_OK;
 }
 
@@ -225,7 +224,7 @@ double table_bytes_per_node(const lbm_handle* h) {
 // Table bytes a step reads per node: those of the row form where the int32
 // mode reads it, by every second step (the others read none).
 double step_table_bytes(const lbm_handle* h) {
-  if (!(h->ct_ok && h->ct_on) && h->rows_on())
+  if (!(h->ct_ok && h->ct_on) && h->rows.p)
     return 0.5 * (9.0 * 4.0 + 5.0 * 4.0 * h->marked / std::max(h->geo.count, 1));
   return 0.5 * table_bytes_per_node(h);
 }
@@ -244,7 +243,7 @@ lbm_status upload_layout(lbm_handle* h) {
   h->last_p = g.count > 0 ? g.int_of[g.count] : -1;
   lbm_status rst = build_rows(h);
   if (rst != LBM_OK) return rst;
-  LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));  // h->marked
+  LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
   h->drop_graphs();
   h->cell_idx_valid = false;
   // the compact form is built when it is first chosen (lbm_set_table_mode,
@@ -376,8 +375,8 @@ StepArgs step_args(lbm_handle* h, bool write) {
     a.ct_off = h->ct_off.as<uint16_t>();
     a.nwarps = h->geo.npad / 32;
   }
-  if (h->rows_on()) a.rows = h->rows.as<int32_t>();
-  a.ahead = prefetch_ahead(n, kQ * (long long)store_bytes(h->kind), a.rows ? 36 : 72);
+  a.rows = h->rows.as<int32_t>();
+  a.ahead = prefetch_ahead(n, kQ * (long long)store_bytes(h->kind), a.ct_base ? 39 : a.rows ? 36 : 72);
   a.snap_begin = h->bc.active ? h->bc.snap_begin : n;
   a.nsnap = std::max(n - a.snap_begin, 1);
   a.snap_dst = h->bc.active ? h->snap[1 - h->cur].as<double>() : nullptr;

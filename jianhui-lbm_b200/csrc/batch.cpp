@@ -91,7 +91,7 @@ struct Pool {
   int ordering = LBM_ORDER_REFERENCE;
   double fp16_scale = 1.0;
   DevBuf x_fields;  // field export
-  DevBuf pop, table, rows, tile_inst, inst, state, partials, active_tiles, n_active, work, slot_off;
+  DevBuf pop, table, tile_inst, inst, state, partials, active_tiles, n_active, work, slot_off;
   SetupScratch setup;
   std::vector<InstParams> h_inst;
   InstState* h_state = nullptr;  // pinned
@@ -155,9 +155,6 @@ struct Pool {
     const size_t s = store_bytes(kind);
     LBM_CUDA_TRY(pop.alloc((size_t)kQ * cap * s));
     LBM_CUDA_TRY(table.alloc((size_t)18 * cap * sizeof(int32_t)));
-    // the row form of the table, for pools whose chains may exceed L2
-    if (ordering == LBM_ORDER_REFERENCE && rows_large(cap, kQ * (long long)s))
-      LBM_CUDA_TRY(rows.alloc((size_t)9 * cap * sizeof(int32_t)));
     LBM_CUDA_TRY(tile_inst.alloc((size_t)ntiles * sizeof(int)));
     LBM_CUDA_TRY(inst.alloc((size_t)nslots * sizeof(InstParams)));
     LBM_CUDA_TRY(state.alloc((size_t)nslots * sizeof(InstState)));
@@ -254,9 +251,6 @@ struct Pool {
                                      cudaMemcpyHostToDevice, stream));
       LBM_CUDA_TRY(cudaStreamSynchronize(stream));  // rows is a host temporary
     }
-    if (rows.p)
-      LBM_CUDA_TRY(launch_row_table(table.as<int32_t>(), cap, ip.begin, j.geo.count, rows.as<int32_t>(), nullptr,
-                                    stream));
     for (int t = ip.tile_begin; t < ip.tile_end; t++) h_tile_inst[t] = slot;
     LBM_CUDA_TRY(cudaMemcpyAsync(tile_inst.as<int>() + ip.tile_begin, h_tile_inst.data() + ip.tile_begin,
                                  sizeof(int) * (ip.tile_end - ip.tile_begin), cudaMemcpyHostToDevice, stream));
@@ -302,16 +296,12 @@ struct Pool {
     return LBM_OK;
   }
 
-  // A step from phase c over step_grid tiles; the row form of the table where
-  // they exceed L2 (its marked nodes are the x wraps in reference order).
-  BatchStepArgs step_args(int c, int step_grid) const {
+  // A step from phase c.
+  BatchStepArgs step_args(int c) const {
     BatchStepArgs a{};
     a.pop = pop.p;
     a.phase = c;
     a.table = table.as<int32_t>();
-    if (rows.p && ordering == LBM_ORDER_REFERENCE &&
-        rows_large((long long)step_grid * kTile, kQ * (long long)store_bytes(kind)))
-      a.rows = rows.as<int32_t>();
     a.cap = cap;
     a.ntiles = ntiles;
     a.tile_inst = tile_inst.as<int>();
@@ -349,7 +339,7 @@ struct Pool {
     cudaError_t err = launch_batch_list(reduce_args(c0), step_grid, block, stream);
     int c = c0;
     for (int s = 0; s < chain && err == cudaSuccess; s++) {
-      err = launch_batch_step(kind, step_args(c, step_grid), block ? block : batch_block(step_grid), step_grid, s, stream);
+      err = launch_batch_step(kind, step_args(c), block ? block : batch_block(step_grid), step_grid, s, stream);
       c = 1 - c;
     }
     if (err == cudaSuccess) err = launch_batch_check(kind, reduce_args(c), chain, tol, max_steps, stream);
@@ -658,12 +648,12 @@ lbm_status lbm_batch_autotune(lbm_batch* b, int trial_steps, int* ordering_out, 
       if ((st = batch_reset(b)) != LBM_OK) return st;
       LBM_CUDA_TRY(launch_batch_list(P.reduce_args(P.cur), P.grid, P.block, P.stream));
       for (int s = 0; s < 2; s++) {  // warm-up
-        LBM_CUDA_TRY(launch_batch_step(P.kind, P.step_args(P.cur, P.grid), P.block, P.grid, s, P.stream));
+        LBM_CUDA_TRY(launch_batch_step(P.kind, P.step_args(P.cur), P.block, P.grid, s, P.stream));
         P.cur = 1 - P.cur;
       }
       LBM_CUDA_TRY(cudaEventRecord(P.ev0, P.stream));
       for (int s = 0; s < trial_steps; s++) {
-        LBM_CUDA_TRY(launch_batch_step(P.kind, P.step_args(P.cur, P.grid), P.block, P.grid, 1, P.stream));
+        LBM_CUDA_TRY(launch_batch_step(P.kind, P.step_args(P.cur), P.block, P.grid, 1, P.stream));
         P.cur = 1 - P.cur;
       }
       LBM_CUDA_TRY(cudaEventRecord(P.ev1, P.stream));

@@ -46,7 +46,6 @@ struct BatchStepArgs {
   void* pop;   // [19][cap], updated in place (kernels_common.cuh)
   int phase;   // Phase of the pool's state
   const int32_t* table;
-  const int32_t* rows;  // [9][cap] row form of the table, or null (read `table`)
   int cap;     // pool nodes (row stride)
   int ntiles;  // cap / kTile
   const int* tile_inst;

@@ -20,7 +20,6 @@
 // (SP:812-816, u_ave from Comput_Perm SP3:3634-3638) per instance.
 #include "batch.h"
 #include "collide_vec.cuh"
-#include "row_table.cuh"
 
 namespace lbm {
 
@@ -34,7 +33,7 @@ namespace lbm {
 // A thread takes two nodes (collide_vec.cuh), neighbours on the node's own
 // slots and 32 apart through the table, as the single-domain step; BS threads
 // step 2 BS nodes a pass, 5 blocks of 128 threads per SM in 96 registers.
-template <Store K, int BS, bool LOCAL, bool ROWS>
+template <Store K, int BS, bool LOCAL>
 __global__ void __launch_bounds__(BS, 640 / BS) batch_step_kernel(BatchStepArgs a, int chain_step) {
   using T = typename Traits<K>::T;
   constexpr int kSub = kTile / (2 * BS);
@@ -63,15 +62,10 @@ __global__ void __launch_bounds__(BS, 640 / BS) batch_step_kernel(BatchStepArgs 
       for (int q = 1; q < kQ; q++) load_row<K>(pop + (size_t)opp(q) * cap + p, inv_scale, true, f[q]);
     } else {
       int32_t s0[kQ], s1[kQ];
-      if constexpr (ROWS) {
-        row_slots(a.rows, a.table, cap, p, s0);
-        row_slots(a.rows, a.table, cap, p1, s1);
-      } else {
 #pragma unroll
-        for (int q = 1; q < kQ; q++) {
-          s0[q] = __ldg(a.table + (size_t)(q - 1) * cap + p);
-          s1[q] = __ldg(a.table + (size_t)(q - 1) * cap + p1);
-        }
+      for (int q = 1; q < kQ; q++) {
+        s0[q] = __ldg(a.table + (size_t)(q - 1) * cap + p);
+        s1[q] = __ldg(a.table + (size_t)(q - 1) * cap + p1);
       }
       step_wait();
       f[0] = make_f2(load_pop_rw<K>(pop + p, inv_scale), load_pop_rw<K>(pop + p1, inv_scale));
@@ -333,11 +327,8 @@ static cudaError_t step_bs(const BatchStepArgs& a, int grid, int chain_step, cud
   // 5.50, 137 K (512) 8.79 | 6.07, 205 K (512) 9.10 | 7.20, 273 K (1024) 9.43 |
   // 8.68, 376 K (1024) 9.75 | 10.3, 562 K (2048) 14.5 | 14.8, 2.8 M 94.0 | 95.6.
   const bool chained = chain_step > 0 && (grid <= 32 || grid >= 1024 || (grid == 256 && BS == 256));
-  if (a.phase == kLocal)
-    return launch_chained(batch_step_kernel<K, BS, true, false>, grid, BS, st, chained, a, chain_step);
-  if (a.rows != nullptr)
-    return launch_chained(batch_step_kernel<K, BS, false, true>, grid, BS, st, chained, a, chain_step);
-  return launch_chained(batch_step_kernel<K, BS, false, false>, grid, BS, st, chained, a, chain_step);
+  if (a.phase == kLocal) return launch_chained(batch_step_kernel<K, BS, true>, grid, BS, st, chained, a, chain_step);
+  return launch_chained(batch_step_kernel<K, BS, false>, grid, BS, st, chained, a, chain_step);
 }
 // `block` nodes a pass, two per thread.
 template <Store K>

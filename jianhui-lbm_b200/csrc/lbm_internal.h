@@ -268,7 +268,7 @@ struct StepArgs {
   void* pop;             // [19][npad] populations, updated in place
   int phase;             // Phase of the state the step starts from
   const int32_t* table;  // [18][npad]
-  const int32_t* rows;   // [9][npad] row form of the table (row_table.cuh), or null
+  const int32_t* rows;   // FP32: [9][npad] row form of the table (row_table.cuh), or null
   int ahead;             // nodes ahead that a block prefetches into L2, 0 = none
   int chained;           // launched as a programmatic dependent of the step before it
   int carveout;          // percent of an SM's L1 to ask for as shared memory, 0 = the driver's choice
@@ -335,25 +335,30 @@ cudaError_t launch_step(Store kind, const StepArgs& a, int block, cudaStream_t s
 cudaError_t launch_compact_table(const int32_t* table, int n, int npad, int32_t* ct_base, uint16_t* ct_off,
                                  unsigned long long* wide, cudaStream_t st);
 
-// Row form of the table entries of nodes [begin, begin + n) of a table of row
-// stride `stride`, at rows + i * stride + begin; adds the marked nodes to
-// *marked (device) when it is not null.
-cudaError_t launch_row_table(const int32_t* table, int stride, int begin, int n, int32_t* rows, int* marked,
-                             cudaStream_t st);
-// Whether the row form is the better one to read, for n nodes with pop_bytes
-// of populations per node (rows_large: whether to build it), `marked` of
-// them marked (rows_pay: whether to read it).
-//  * It reads 36 bytes per node against 72, and each marked node up to five
-//    table entries in 32-byte sectors of their own: the two meet where 160
-//    bytes x the marked share are 36, at 0.22.  Reference order marks 2 / nx
-//    of the nodes, the curve orders most of them.
+// Row form of a table of row stride `stride`, its first n nodes; adds the
+// marked nodes to *marked (device).
+cudaError_t launch_row_table(const int32_t* table, int stride, int n, int32_t* rows, int* marked, cudaStream_t st);
+// Where the row form is the better one to read: in the FP32 single-phase step
+// and the D3Q19 solutes, for n nodes with pop_bytes of populations per node
+// (rows_large: whether to build it), `marked` of them marked (rows_pay: whether
+// to keep and read it).
+//  * It reads 36 bytes per node against 72, for arithmetic that the other
+//    steps have no room for.  us per step, rows | int32, 256^3, porosity 0.35:
+//    FP32 166 | 173, FP16 129 | 125 (0.6: 226 | 216), FP64 717 | 671, FP64
+//    deviation 323 | 317 (0.6: 562 | 544); D3Q19 solute 192^3 FP32 111 | 113,
+//    FP64 211 | 220; pools of 96^3 to 200^3 1 to 8 % slower with rows.
+//  * A warp with a marked node waits for up to five table entries more, and
+//    about every warp has one where a row of cells holds fewer than 32 nodes.
+//    Reference order marks 2 / nx of the nodes, the curve orders most of them.
+//    FP32 us, rows | int32, nx = 64, 96, 128, 256: porosity 0.35 (1.1 M nodes) 34.8 |
+//    34.5, 33.6 | 34.4, 32.7 | 34.8, 31.0 | 34.3; 0.6 (1.9 M) 63.9 | 59.6, 60.0 | 59.9,
+//    60.2 | 61.4, 58.1 | 59.3: the line is drawn at nx = 100.
 //  * Its arithmetic costs more than the bytes it saves while the solve lives
-//    in the 126 MB L2 with either form: FP32 steps of cubes at porosity 0.35
-//    took (int32 | rows) 4.28 | 4.62 us at 64^3, 9.12 | 9.51 at 96^3 and
-//    12.8 | 13.4 at 112^3 (73 MB with the int32 table), 21.1 | 19.4 at 128^3
-//    (109 MB); the line is drawn between the last two.
+//    in the 126 MB L2 with either form: FP32 cubes at porosity 0.35 took (int32
+//    | rows) 9.12 | 9.51 us at 96^3, 12.8 | 13.4 at 112^3 (73 MB with the int32
+//    table), 21.1 | 19.4 at 128^3 (109 MB).
 constexpr bool rows_large(long long n, long long pop_bytes) { return n * (pop_bytes + 72) > (90LL << 20); }
-constexpr bool rows_pay(long long marked, long long n) { return marked * 8 <= n; }
+constexpr bool rows_pay(long long marked, long long n) { return marked * 50 <= n; }
 // Nodes ahead of its own that a block prefetches into L2 (half a wave of
 // resident threads), or 0 for a solve that stays in L2.  A step waits on two
 // loads in a row, table then populations; asked for half a wave early, both

@@ -48,12 +48,11 @@ __global__ void pull_table_kernel(const int32_t* __restrict__ coor_x, const int3
   }
 }
 
-__global__ void __launch_bounds__(256) row_table_kernel(const int32_t* __restrict__ table, int stride, int begin, int n,
+__global__ void __launch_bounds__(256) row_table_kernel(const int32_t* __restrict__ table, int stride, int n,
                                                         int32_t* __restrict__ rows, int* __restrict__ marked) {
-  const int i = blockIdx.x * 256 + threadIdx.x;
-  const int p = begin + i;
+  const int p = blockIdx.x * 256 + threadIdx.x;
   bool mark = false;
-  if (i < n) {
+  if (p < n) {
     int32_t m[kQ];
     uint32_t bits = 0;
 #pragma unroll
@@ -78,10 +77,8 @@ __global__ void __launch_bounds__(256) row_table_kernel(const int32_t* __restric
     rows[(size_t)8 * stride + p] = (int32_t)bits;
     mark = (bits & (kRowLo | kRowHi)) != 0;
   }
-  if (marked != nullptr) {
-    const int c = __popc(__ballot_sync(0xffffffffu, mark));
-    if ((threadIdx.x & 31) == 0 && c > 0) atomicAdd(marked, c);
-  }
+  const int c = __popc(__ballot_sync(0xffffffffu, mark));
+  if ((threadIdx.x & 31) == 0 && c > 0) atomicAdd(marked, c);
 }
 
 __global__ void iota_kernel(int32_t* __restrict__ out, int n, int first) {
@@ -193,9 +190,8 @@ lbm_status device_index_reference(const uint8_t* host_mask, int nx, int ny, int 
   return LBM_OK;
 }
 
-cudaError_t launch_row_table(const int32_t* table, int stride, int begin, int n, int32_t* rows, int* marked,
-                             cudaStream_t st) {
-  if (n > 0) row_table_kernel<<<(n + 255) / 256, 256, 0, st>>>(table, stride, begin, n, rows, marked);
+cudaError_t launch_row_table(const int32_t* table, int stride, int n, int32_t* rows, int* marked, cudaStream_t st) {
+  if (n > 0) row_table_kernel<<<(n + 255) / 256, 256, 0, st>>>(table, stride, n, rows, marked);
   return cudaGetLastError();
 }
 

@@ -31,7 +31,6 @@
 #include <utility>
 
 #include "bc_kernels.cuh"
-#include "row_table.cuh"
 #include "mi_pattern.h"  // generated at build time from mrt.cpp's M^-1
 
 namespace lbm {
@@ -364,14 +363,12 @@ __device__ __forceinline__ void collide_moments(double (&m)[kQ], double rho, dou
 
 // Post-streaming populations of node p; got(q, slot) sees the slots they were
 // read from.
-template <bool LOCAL, bool ROWS, typename Got>
+template <bool LOCAL, typename Got>
 __device__ __forceinline__ void pull_f64(const StepArgs& a, int p, double (&f)[kQ], Got&& got) {
   const double* pop = static_cast<const double*>(a.pop);
   int32_t s[kQ];
-  if constexpr (ROWS) row_slots(a.rows, a.table, a.npad, p, s);
 #pragma unroll
-  for (int q = 1; q < kQ; q++)
-    if constexpr (!ROWS) s[q] = LOCAL ? opp(q) * a.npad + p : __ldg(a.table + (size_t)(q - 1) * a.npad + p);
+  for (int q = 1; q < kQ; q++) s[q] = LOCAL ? opp(q) * a.npad + p : __ldg(a.table + (size_t)(q - 1) * a.npad + p);
   step_wait();
   f[0] = pop[p];
 #pragma unroll
@@ -382,7 +379,7 @@ __device__ __forceinline__ void pull_f64(const StepArgs& a, int p, double (&f)[k
 }
 template <bool LOCAL>
 __device__ __forceinline__ void pull_f64(const StepArgs& a, int p, double (&f)[kQ]) {
-  pull_f64<LOCAL, false>(a, p, f, [](int, int32_t) {});
+  pull_f64<LOCAL>(a, p, f, [](int, int32_t) {});
 }
 
 __device__ __forceinline__ void macro_in_out(const StepArgs& a, int p, bool given, bool write, const double (&f)[kQ],
@@ -418,11 +415,10 @@ constexpr int f64_min_blocks(int bs) { return 512 / bs; }
 // from the accumulated moments; with a self-defined lattice (LAT) j sums the
 // products e_a lat_c f_q, each rounded, in direction order, which the kernel
 // accumulates beside the moments.
-template <int BS, bool GIVEN, bool WRITE, bool GX, bool LAT, bool LOCAL, bool ROWS>
+template <int BS, bool GIVEN, bool WRITE, bool GX, bool LAT, bool LOCAL>
 __global__ void __launch_bounds__(BS, f64_min_blocks(BS)) step_f64_faithful(StepArgs a) {
   const int p = blockIdx.x * BS + threadIdx.x;
-  prefetch_block<BS, BS, ROWS ? 9 : LOCAL ? 0 : 18>(static_cast<const double*>(a.pop), ROWS ? a.rows : a.table, a.npad,
-                                                a.ahead);
+  prefetch_block<BS, BS, LOCAL ? 0 : 18>(static_cast<const double*>(a.pop), a.table, a.npad, a.ahead);
   step_begin();
   if (p >= a.n_main) return;
   // the slots of a kPull state's gathers, for the stores after the collision
@@ -432,7 +428,7 @@ __global__ void __launch_bounds__(BS, f64_min_blocks(BS)) step_f64_faithful(Step
   double jx = 0.0, jy = 0.0, jz = 0.0;
   {
     double f[kQ];
-    pull_f64<LOCAL, ROWS>(a, p, f, [&](int q, int32_t s) {
+    pull_f64<LOCAL>(a, p, f, [&](int q, int32_t s) {
       if constexpr (!LOCAL) keep[q - 1][threadIdx.x] = s;
     });
     moments_by_column(m, f, QSeq{});
@@ -550,20 +546,14 @@ static cudaError_t launch_f64_bs(const StepArgs& a, cudaStream_t st) {
   const bool given = a.rho_in != nullptr, write = a.rho_out != nullptr;
   if (a.phase == kLocal) {
     if (given) return cudaErrorInvalidValue;  // a given state is a kPull state
-    if (write)
-      return launch_step_kernel(step_f64_faithful<BS, false, true, GX, LAT, true, false>, grid, BS, st, a);
-    return launch_step_kernel(step_f64_faithful<BS, false, false, GX, LAT, true, false>, grid, BS, st, a);
-  } else if (given && write) {
-    return launch_step_kernel(step_f64_faithful<BS, true, true, GX, LAT, false, false>, grid, BS, st, a);
-  } else if (given) {
-    return launch_step_kernel(step_f64_faithful<BS, true, false, GX, LAT, false, false>, grid, BS, st, a);
-  } else if (write) {
-    return a.rows ? launch_step_kernel(step_f64_faithful<BS, false, true, GX, LAT, false, true>, grid, BS, st, a)
-           : launch_step_kernel(step_f64_faithful<BS, false, true, GX, LAT, false, false>, grid, BS, st, a);
-  } else {
-    return a.rows ? launch_step_kernel(step_f64_faithful<BS, false, false, GX, LAT, false, true>, grid, BS, st, a)
-           : launch_step_kernel(step_f64_faithful<BS, false, false, GX, LAT, false, false>, grid, BS, st, a);
+    return write ? launch_step_kernel(step_f64_faithful<BS, false, true, GX, LAT, true>, grid, BS, st, a)
+                 : launch_step_kernel(step_f64_faithful<BS, false, false, GX, LAT, true>, grid, BS, st, a);
   }
+  if (given)
+    return write ? launch_step_kernel(step_f64_faithful<BS, true, true, GX, LAT, false>, grid, BS, st, a)
+                 : launch_step_kernel(step_f64_faithful<BS, true, false, GX, LAT, false>, grid, BS, st, a);
+  return write ? launch_step_kernel(step_f64_faithful<BS, false, true, GX, LAT, false>, grid, BS, st, a)
+               : launch_step_kernel(step_f64_faithful<BS, false, false, GX, LAT, false>, grid, BS, st, a);
 }
 
 template <int BS>

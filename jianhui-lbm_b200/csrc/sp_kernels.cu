@@ -73,8 +73,8 @@ cudaError_t launch_compact_table(const int32_t* table, int n, int npad, int32_t*
 static bool two_nodes(int n) { return n >= 148 * 1024; }
 
 // Where a step reads and writes: the node's own slots (a kLocal state), or
-// the slots of the int32 table, of its row form or of its compact form (a
-// kPull state).
+// the slots of the int32 table, of its row form (FP32) or of its compact form
+// (a kPull state).
 enum class Slots { Local, Table, Rows, Compact };
 
 // The block's warp bases of the compact table, in shared memory, and this
@@ -112,14 +112,12 @@ __device__ __forceinline__ void compact_slots(const CompactBlock<BS>& cb, const 
     slot[q] = b < 0 ? t : c;
   }
 }
-// slot[q] of node p through the int32 table, its row form or its compact form
+// slot[q] of node p through the int32 table or its compact form
 template <Slots SL, int BS>
 __device__ __forceinline__ void read_slots(const CompactBlock<BS>& cb, const StepArgs& a, int p,
                                            const uint32_t (&ow)[9], int32_t (&slot)[kQ]) {
   if constexpr (SL == Slots::Compact) {
     compact_slots(cb, a, p, ow, slot);
-  } else if constexpr (SL == Slots::Rows) {
-    row_slots(a.rows, a.table, a.npad, p, slot);
   } else {
 #pragma unroll
     for (int q = 1; q < kQ; q++) slot[q] = __ldg(a.table + (size_t)(q - 1) * a.npad + p);
@@ -136,8 +134,7 @@ __global__ void __launch_bounds__(BS, BS == 256 ? 2 : 1) step_dev_kernel(StepArg
   __shared__ CompactBlock<SL == Slots::Compact ? BS : 32> cb;
   uint32_t ow[9] = {};
   if constexpr (SL == Slots::Compact) compact_load(cb, a, p, ow);
-  prefetch_block<BS, BS, SL == Slots::Rows ? 9 : SL == Slots::Table ? 18 : 0>(
-      static_cast<const double*>(a.pop), SL == Slots::Rows ? a.rows : a.table, a.npad, a.ahead);
+  prefetch_block<BS, BS, SL == Slots::Table ? 18 : 0>(static_cast<const double*>(a.pop), a.table, a.npad, a.ahead);
   step_begin();
   if (p >= a.n_main) return;
   double* pop = static_cast<double*>(a.pop);
@@ -214,6 +211,7 @@ __global__ void __launch_bounds__(BS, vec_min_blocks<V>(BS)) step_vec_kernel(Ste
   using T = typename Traits<K>::T;
   constexpr int N = VecOf<V>::kNodes;
   static_assert(N == 1 || (!GIVEN && SL != Slots::Compact), "given states and the compact table: one node per thread");
+  static_assert(N == 2 || SL != Slots::Rows, "the row form: two nodes per thread");
   constexpr bool PAIR = N == 2 && SL == Slots::Local;  // p, p + 1
   const int p = N == 1 ? blockIdx.x * BS + threadIdx.x
                 : PAIR ? (blockIdx.x * BS + threadIdx.x) * 2
@@ -467,27 +465,26 @@ static cudaError_t launch_dev_bs(const StepArgs& a, cudaStream_t st) {
   if (a.n_main <= 0) return cudaSuccess;
   const bool local = a.phase == kLocal;
   if (local && a.rho_in != nullptr) return cudaErrorInvalidValue;  // a given state is a kPull state
-  const Slots sl = local ? Slots::Local : a.ct_base ? Slots::Compact : a.rows ? Slots::Rows : Slots::Table;
+  const Slots sl = local ? Slots::Local : a.ct_base ? Slots::Compact : Slots::Table;
   const int grid = (a.n_main + BS - 1) / BS;  // BS nodes per block, by BS or BS / 2 threads
   if constexpr (K == Store::F64D) {
     switch (sl) {
       case Slots::Local: return launch_f64d<BS, Slots::Local>(a, grid, st);
       case Slots::Table: return launch_f64d<BS, Slots::Table>(a, grid, st);
-      case Slots::Rows: return launch_f64d<BS, Slots::Rows>(a, grid, st);
       case Slots::Compact: return launch_f64d<BS, Slots::Compact>(a, grid, st);
+      case Slots::Rows: break;
     }
   } else if (a.rho_in == nullptr && sl != Slots::Compact && two_nodes(a.n_main)) {
-    switch (sl) {
-      case Slots::Local: return launch_vec<K, BS / 2, F2, Slots::Local>(a, grid, st);
-      case Slots::Rows: return launch_vec<K, BS / 2, F2, Slots::Rows>(a, grid, st);
-      default: return launch_vec<K, BS / 2, F2, Slots::Table>(a, grid, st);
-    }
+    if (local) return launch_vec<K, BS / 2, F2, Slots::Local>(a, grid, st);
+    if constexpr (K == Store::F32)
+      if (a.rows) return launch_vec<K, BS / 2, F2, Slots::Rows>(a, grid, st);
+    return launch_vec<K, BS / 2, F2, Slots::Table>(a, grid, st);
   } else {
     switch (sl) {
       case Slots::Local: return launch_vec<K, BS, float, Slots::Local>(a, grid, st);
       case Slots::Table: return launch_vec<K, BS, float, Slots::Table>(a, grid, st);
-      case Slots::Rows: return launch_vec<K, BS, float, Slots::Rows>(a, grid, st);
       case Slots::Compact: return launch_vec<K, BS, float, Slots::Compact>(a, grid, st);
+      case Slots::Rows: break;
     }
   }
   return cudaErrorInvalidValue;

@@ -40,7 +40,6 @@ struct lbm_st7_handle {
   Geometry geo;
   DevBuf g, table, rows, u, c0, ref_of, x_conc;
   int cur = kPull;  // phase of g
-  bool rows_on = false;
   // captured step chains, one per starting phase, and the steps launched one
   // by one that each would have covered
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -73,8 +72,8 @@ St7Args st7_args(lbm_st7_handle* h, bool given) {
   a.phase = h->cur;
   a.table = static_cast<const int32_t*>(h->table.p);
   const long long bytes = (long long)(h->nq == kQ ? kQ : 6) * (h->f64 ? 8 : 4), ub = 3LL * (h->f64 ? 8 : 4);
-  a.rows = h->rows_on ? static_cast<const int32_t*>(h->rows.p) : nullptr;
-  a.ahead = prefetch_ahead(h->geo.count, bytes + ub, h->nq == kQ ? (h->rows_on ? 36 : 72) : 24);
+  a.rows = h->rows.as<int32_t>();
+  a.ahead = prefetch_ahead(h->geo.count, bytes + ub, h->nq == kQ ? (h->rows.p ? 36 : 72) : 24);
   a.u = h->u.p;
   a.c_given = given ? h->c0.p : nullptr;
   a.n = h->geo.count;
@@ -184,11 +183,10 @@ lbm_status create_solute(const lbm_st7_params* p, const uint8_t* mask, int nx, i
     LBM_CUDA_TRY(h->rows.alloc((size_t)9 * npad * sizeof(int32_t)));
     LBM_CUDA_TRY(marked.alloc(sizeof(int)));
     LBM_CUDA_TRY(cudaMemsetAsync(marked.p, 0, sizeof(int), h->stream));
-    LBM_CUDA_TRY(launch_row_table(static_cast<const int32_t*>(h->table.p), npad, 0, n, static_cast<int32_t*>(h->rows.p),
-                                  static_cast<int*>(marked.p), h->stream));
+    LBM_CUDA_TRY(launch_row_table(h->table.as<int32_t>(), npad, n, h->rows.as<int32_t>(), marked.as<int>(), h->stream));
     LBM_CUDA_TRY(cudaMemcpyAsync(&count, marked.p, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    h->rows_on = rows_pay(count, n);
+    if (!rows_pay(count, n)) h->rows.release();
   }
   std::vector<double> uu((size_t)3 * npad, 0.0), cc((size_t)npad, 0.0);
   for (int x = 0; x < n; x++) {

@@ -23,7 +23,7 @@ cudaError_t launch_init_uniform(Store, void*, const int32_t*, int, int, double, 
   return last();
 }
 cudaError_t launch_fill_macro(Store, void*, void*, int, int, double, const double*, cudaStream_t) { return last(); }
-cudaError_t launch_row_table(const int32_t*, int, int, int, int32_t*, int*, cudaStream_t) { return last(); }
+cudaError_t launch_row_table(const int32_t*, int, int, int32_t*, int*, cudaStream_t) { return last(); }
 cudaError_t launch_compact_table(const int32_t*, int, int, int32_t*, uint16_t*, unsigned long long*, cudaStream_t) {
   return last();
 }

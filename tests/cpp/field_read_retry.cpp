@@ -23,7 +23,7 @@ int batch_step_grid(int ntiles, int) { return ntiles; }
 cudaError_t launch_init_uniform(Store, void*, const int32_t*, int, int, double, const double*, cudaStream_t) {
   return last();
 }
-cudaError_t launch_row_table(const int32_t*, int, int, int, int32_t*, int*, cudaStream_t) { return last(); }
+cudaError_t launch_row_table(const int32_t*, int, int, int32_t*, int*, cudaStream_t) { return last(); }
 void SetupScratch::release() {}
 lbm_status device_index_reference(const uint8_t*, int, int, int, int, int32_t*, long long, int, int32_t*,
                                   SetupScratch&, cudaStream_t) {

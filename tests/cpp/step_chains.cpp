@@ -19,7 +19,7 @@ cudaError_t launch_init_uniform(Store, void*, const int32_t*, int, int, double, 
   return last();
 }
 cudaError_t launch_fill_macro(Store, void*, void*, int, int, double, const double*, cudaStream_t) { return last(); }
-cudaError_t launch_row_table(const int32_t*, int, int, int, int32_t*, int*, cudaStream_t) { return last(); }
+cudaError_t launch_row_table(const int32_t*, int, int, int32_t*, int*, cudaStream_t) { return last(); }
 bool SetupScratch::borrow(void*, size_t, long long, int) { return true; }
 void SetupScratch::release() {}
 lbm_status device_index_reference(const uint8_t*, int, int, int, int, int32_t*, long long, int, int32_t*,

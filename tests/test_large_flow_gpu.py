@@ -60,3 +60,17 @@ def test_a_call_equals_its_steps_one_by_one(precision, shape, phi):
         for x, y in zip(a.fields(), b.fields()):
             assert np.array_equal(x, y)
         assert a.reduce() == b.reduce()
+
+
+# FP32 reads the row form above 90 MiB (0.64 M nodes) where rows of cells are
+# 100 cells or longer; other storages and curve orders read the int32 table.
+@pytest.mark.parametrize("precision,ordering,shape,rows", [
+    ("f32", "reference", (128, 101, 97), True), ("f32", "reference", (90, 128, 109), False),
+    ("f32", "hilbert", (128, 101, 97), False), ("f32", "reference", (101, 80, 80), False),
+    ("f16", "reference", (128, 121, 119), False), ("f64", "reference", (128, 101, 97), False),
+    ("f64fast", "reference", (128, 101, 97), False)])
+def test_where_the_row_form_is_read(precision, ordering, shape, rows):
+    mask = spheres(shape, 0.8, 4.5, seed=2)
+    with L.SinglePhase(mask, 0.1, (1e-6, 0.0, 0.0), precision=precision, ordering=ordering) as s:
+        per_step = s.memory()["bytes_per_lu"] - 38 * {"f16": 2, "f32": 4}.get(precision, 8)
+        assert per_step == 36 if not rows else 18 <= per_step < 19
