@@ -74,8 +74,10 @@ static bool two_nodes(int n) { return n >= 148 * 1024; }
 
 // Where a step reads and writes: the node's own slots (a kLocal state), or
 // the slots of the int32 table, of its row form (FP32) or of its compact form
-// (a kPull state).
-enum class Slots { Local, Table, Rows, Compact };
+// (a kPull state).  LocalOdd: the node's own slots, of an odd number of nodes
+// that face nodes follow: the last pair's second slot is the face kernel's,
+// which runs beside the step (asking everywhere costs 0.5 to 3 % in L2).
+enum class Slots { Local, LocalOdd, Table, Rows, Compact };
 
 // The block's warp bases of the compact table, in shared memory, and this
 // node's offset words: the words are loaded before the barrier so that their
@@ -212,12 +214,12 @@ __global__ void __launch_bounds__(BS, vec_min_blocks<V>(BS)) step_vec_kernel(Ste
   constexpr int N = VecOf<V>::kNodes;
   static_assert(N == 1 || (!GIVEN && SL != Slots::Compact), "given states and the compact table: one node per thread");
   static_assert(N == 2 || SL != Slots::Rows, "the row form: two nodes per thread");
-  constexpr bool PAIR = N == 2 && SL == Slots::Local;  // p, p + 1
+  constexpr bool LOCAL = SL == Slots::Local || SL == Slots::LocalOdd, PAIR = N == 2 && LOCAL;  // p, p + 1
   const int p = N == 1 ? blockIdx.x * BS + threadIdx.x
                 : PAIR ? (blockIdx.x * BS + threadIdx.x) * 2
                        : blockIdx.x * BS * 2 + (threadIdx.x >> 5) * 64 + (threadIdx.x & 31);
   const int second = p + (PAIR ? 1 : 32);
-  __shared__ SlotKeep<SL == Slots::Local ? 1 : BS, N> keep;
+  __shared__ SlotKeep<LOCAL ? 1 : BS, N> keep;
   __shared__ CompactBlock<SL == Slots::Compact ? BS : 32> cb;
   uint32_t ow[9] = {};
   if constexpr (SL == Slots::Compact) compact_load(cb, a, p, ow);
@@ -227,14 +229,15 @@ __global__ void __launch_bounds__(BS, vec_min_blocks<V>(BS)) step_vec_kernel(Ste
   if (p >= a.n_main) return;
   const bool both = N == 2 && second < a.n_main;
   const int p1 = both ? second : p;  // a missing second node is worked on as the first and not stored
+  const bool load_both = SL != Slots::LocalOdd || both;
   T* pop = static_cast<T*>(a.pop);
   const float scale = (float)a.fp16_scale;
   const float inv_scale = a.fp16_inv;
   V f[kQ];
-  if constexpr (SL == Slots::Local) {
+  if constexpr (LOCAL) {
     step_wait();
 #pragma unroll
-    for (int q = 1; q < kQ; q++) load_row<K>(pop + (size_t)opp(q) * a.npad + p, inv_scale, both, f[q]);
+    for (int q = 1; q < kQ; q++) load_row<K>(pop + (size_t)opp(q) * a.npad + p, inv_scale, load_both, f[q]);
   } else if constexpr (N == 1) {
     int32_t slot[kQ];  // slot[q] holds f_q on entry and takes f*_opp(q)
     read_slots<SL>(cb, a, p, ow, slot);
@@ -270,7 +273,7 @@ __global__ void __launch_bounds__(BS, vec_min_blocks<V>(BS)) step_vec_kernel(Ste
   }
 
   if constexpr (N == 1 || PAIR)
-    load_row<K>(pop + p, inv_scale, both, f[0]);
+    load_row<K>(pop + p, inv_scale, load_both, f[0]);
   else
     f[0] = make_f2(load_pop_rw<K>(pop + p, inv_scale), load_pop_rw<K>(pop + p1, inv_scale));
 
@@ -322,7 +325,7 @@ __global__ void __launch_bounds__(BS, vec_min_blocks<V>(BS)) step_vec_kernel(Ste
     store_pop<K>(pop + p, lane(f[0], 0), scale);
     if (both) store_pop<K>(pop + p1, lane(f[0], 1), scale);
   }
-  if constexpr (SL == Slots::Local) {
+  if constexpr (LOCAL) {
 #pragma unroll
     for (int q = 1; q < kQ; q++) store_row<K>(pop + (size_t)q * a.npad + p, f[q], scale, both);
   } else if constexpr (N == 1) {
@@ -472,9 +475,10 @@ static cudaError_t launch_dev_bs(const StepArgs& a, cudaStream_t st) {
       case Slots::Local: return launch_f64d<BS, Slots::Local>(a, grid, st);
       case Slots::Table: return launch_f64d<BS, Slots::Table>(a, grid, st);
       case Slots::Compact: return launch_f64d<BS, Slots::Compact>(a, grid, st);
-      case Slots::Rows: break;
+      default: break;
     }
   } else if (a.rho_in == nullptr && sl != Slots::Compact && two_nodes(a.n_main)) {
+    if (local && a.n_main < a.n && (a.n_main & 1)) return launch_vec<K, BS / 2, F2, Slots::LocalOdd>(a, grid, st);
     if (local) return launch_vec<K, BS / 2, F2, Slots::Local>(a, grid, st);
     if constexpr (K == Store::F32)
       if (a.rows) return launch_vec<K, BS / 2, F2, Slots::Rows>(a, grid, st);
@@ -484,7 +488,7 @@ static cudaError_t launch_dev_bs(const StepArgs& a, cudaStream_t st) {
       case Slots::Local: return launch_vec<K, BS, float, Slots::Local>(a, grid, st);
       case Slots::Table: return launch_vec<K, BS, float, Slots::Table>(a, grid, st);
       case Slots::Compact: return launch_vec<K, BS, float, Slots::Compact>(a, grid, st);
-      case Slots::Rows: break;
+      default: break;
     }
   }
   return cudaErrorInvalidValue;
