@@ -359,14 +359,20 @@ cudaError_t launch_row_table(const int32_t* table, int stride, int n, int32_t* r
 //    table), 21.1 | 19.4 at 128^3 (109 MB).
 constexpr bool rows_large(long long n, long long pop_bytes) { return n * (pop_bytes + 72) > (90LL << 20); }
 constexpr bool rows_pay(long long marked, long long n) { return marked * 50 <= n; }
-// Nodes ahead of its own that a block prefetches into L2 (half a wave of
-// resident threads), or 0 for a solve that stays in L2.  A step waits on two
-// loads in a row, table then populations; asked for half a wave early, both
-// come from L2.  256^3, porosity 0.35, rows: 184 -> 169 us per FP32 step,
-// 347 -> 319 in 64-bit deviation storage; at 128^3, in L2, 19.4 -> 20.3.
-// (A whole wave ahead 174, two waves 192 us: the lines are evicted again.)
+// Nodes ahead of its own that a block prefetches into L2, or 0 for a solve that
+// stays in L2, for pop_bytes of rows and table_bytes of table per node.  A step
+// waits on two loads in a row, table then populations; asked for early, both
+// come from L2.  What matters is how much is on its way: too little and the
+// lines arrive late, too much and they are evicted again.  The best distance
+// was about 44 KB per SM for every step (a multiple of 64 nodes per SM).  us per
+// step without | at that | at 640 nodes per SM, cubes at porosity 0.35: FP32 256^3
+// (112 bytes) 174 | 161 | 161, FP16 256^3 (110) 136 | 128 | 128, FP64 deviation 256^3
+// (224) 335 | 299 | 314, D3Q7 FP32 192^3 (60) 33.1 | 27.6 | 27.6, FP64 192^3 (96) 60.4
+// | 48.0 | 48.0, D3Q19 FP32 192^3 (124) 94.4 | 77.6 | 78.3, FP64 128^3 (212) 53.2 | 44.7
+// | 48.5.  The bit-exact FP64 step is bound by its FP64 pipe: 484 to 491 at any.
 constexpr int prefetch_ahead(long long n, long long pop_bytes, long long table_bytes) {
-  return n * (pop_bytes + table_bytes) > (120LL << 20) ? 148 * 640 : 0;
+  const long long bytes = pop_bytes + table_bytes;
+  return n * bytes > (120LL << 20) ? 148 * 64 * (int)((44000 / bytes + 32) / 64) : 0;
 }
 
 // Whether successive steps are launched as programmatic dependents

@@ -10,8 +10,8 @@
 //
 // Both solutes step in place (kernels_common.cuh): every second step works on
 // the node's own slots and reads no table, and a solve needs one array.  They
-// are bound by their bytes; a block prefetches the rows of nodes half a wave
-// ahead into L2 when the solve exceeds it, as the flow step does.
+// are bound by their bytes; a block prefetches the rows of nodes further on
+// into L2 when the solve exceeds it, as the flow step does (prefetch_ahead).
 #pragma once
 
 #include "cg_basis.h"
