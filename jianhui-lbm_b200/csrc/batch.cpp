@@ -90,7 +90,6 @@ struct Pool {
   int block = 0, grid = 0;  // nodes per pass of the step asked for or autotuned (0: batch_block)
   int ordering = LBM_ORDER_REFERENCE;
   double fp16_scale = 1.0;
-  DevBuf x_fields;  // field export
   DevBuf pop, table, tile_inst, inst, state, partials, active_tiles, n_active, work, slot_off;
   SetupScratch setup;
   std::vector<InstParams> h_inst;
@@ -414,22 +413,22 @@ struct Pool {
     const Job& j = *slot_job[slot];
     const InstParams& ip = h_inst[slot];
     const int n = j.geo.count;
-    // rho [n + 1] and u [n + 1][3]; kept between calls, grown to the largest
-    // instance read
-    const size_t rows = (size_t)n + 1, need = 4 * rows * sizeof(double);
-    if (x_fields.bytes < need) LBM_CUDA_TRY(x_fields.alloc(need));
-    double* r = x_fields.as<double>();
+    const size_t rows = (size_t)n + 1;
+    DevBuf buf;  // rho [n + 1] and u [n + 1][3]
+    LBM_CUDA_TRY(buf.alloc(4 * rows * sizeof(double)));
+    double* r = buf.as<double>();
     double* v = r + rows;
     DevBuf ref;  // reference order: internal index p is reference id p + 1
     if (!j.geo.ref_of.empty()) {
       LBM_CUDA_TRY(ref.alloc(sizeof(int32_t) * n));
       LBM_CUDA_TRY(cudaMemcpyAsync(ref.p, j.geo.ref_of.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream));
     }
-    LBM_CUDA_TRY(cudaMemsetAsync(r, 0, need, stream));
+    LBM_CUDA_TRY(cudaMemsetAsync(r, 0, buf.bytes, stream));
     LBM_CUDA_TRY(launch_batch_export_macro(kind, pop.p, slot_phase[slot], table.as<int32_t>(), cap, ip.begin, n,
                                            ref.as<int32_t>(), ip, r, v, stream));
-    if (rho) LBM_CUDA_TRY(d2h_staged(rho, r, rows * sizeof(double), stream));
-    if (u) LBM_CUDA_TRY(d2h_staged(u, v, 3 * rows * sizeof(double), stream));
+    const HostPart out[2] = {{rho, rows * sizeof(double)}, {u, 3 * rows * sizeof(double)}};
+    if (rho) LBM_CUDA_TRY(d2h_staged(out, u ? 2 : 1, r, stream));
+    if (!rho && u) LBM_CUDA_TRY(d2h_staged(out + 1, 1, v, stream));
     LBM_CUDA_TRY(cudaStreamSynchronize(stream));
     return LBM_OK;
   }

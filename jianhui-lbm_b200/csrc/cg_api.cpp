@@ -64,7 +64,6 @@ struct lbm_cg_handle {
   bool colour_done = false;
   double rand_sat = -1.0;                 // ini_Sat: threshold of the random phase faces
   unsigned long long rand_seed = 0;       // seed of the random phase faces
-  DevBuf x_fields;                           // field export, kept between calls
   DevBuf zero_sigma;                         // zero-surface-tension layer flags, or none
   int nface = 0;
   std::vector<double> psi0;               // initial phase per node (internal order), as read
@@ -627,27 +626,34 @@ lbm_status lbm_cg_get_fields(lbm_cg_handle* h, double* rho, double* u, double* p
   lbm_status st = cg_check(h);
   if (st != LBM_OK) return st;
   const int n = h->geo.count, npad = h->geo.npad;
-  // internal-order rho and u, then the fields in the reference's order; kept
-  // between calls, and filled and ordered on the device: the host only copies
+  // internal-order rho and u, then the fields in the reference's order, filled
+  // and ordered on the device: the host only copies
   const size_t rows = (size_t)n + 1;
-  const size_t need = ((size_t)4 * npad + 4 * rows) * sizeof(double);
-  if (h->x_fields.bytes != need) LBM_CUDA_TRY(h->x_fields.alloc(need));
-  double* rint = h->x_fields.as<double>();
+  DevBuf buf;
+  LBM_CUDA_TRY(buf.alloc(((size_t)4 * npad + 7 * rows) * sizeof(double)));
+  double* rint = buf.as<double>();
   double* uint_ = rint + npad;
-  double* rref = uint_ + (size_t)3 * npad;
-  double* uref = rref + rows;
+  double* ref = uint_ + (size_t)3 * npad;  // rho, u [rows][3], psi, rho_r, rho_b
   double r[8];
   if ((st = cg_reduce_raw(h, r, rint, uint_)) != LBM_OK) return st;
-  LBM_CUDA_TRY(cudaMemsetAsync(rref, 0, 4 * rows * sizeof(double), h->stream));
-  LBM_CUDA_TRY(launch_export_macro(rint, uint_, h->ref_of.as<int32_t>(), n, npad, rref, uref, h->stream));
-  if (rho) LBM_CUDA_TRY(d2h_staged(rho, rref, rows * sizeof(double), h->stream));
-  if (u) LBM_CUDA_TRY(d2h_staged(u, uref, 3 * rows * sizeof(double), h->stream));
-  double* outs[3] = {psi, rho_r, rho_b};
+  LBM_CUDA_TRY(cudaMemsetAsync(ref, 0, 4 * rows * sizeof(double), h->stream));
+  LBM_CUDA_TRY(launch_export_macro(rint, uint_, h->ref_of.as<int32_t>(), n, npad, ref, ref + rows, h->stream));
+  const HostPart out[5] = {{rho, rows * sizeof(double)}, {u, 3 * rows * sizeof(double)}, {psi, rows * sizeof(double)},
+                           {rho_r, rows * sizeof(double)}, {rho_b, rows * sizeof(double)}};
   const DevBuf* srcs[3] = {&h->psi, &h->rho_r, &h->rho_b};
-  for (int i = 0; i < 3; i++) {
-    if (!outs[i]) continue;
-    LBM_CUDA_TRY(launch_export_scalar(h->f64, srcs[i]->p, h->ref_of.as<int32_t>(), n, rref, h->stream));
-    LBM_CUDA_TRY(d2h_staged(outs[i], rref, rows * sizeof(double), h->stream));
+  for (int i = 0; i < 3; i++)
+    if (out[2 + i].dst)
+      LBM_CUDA_TRY(launch_export_scalar(h->f64, srcs[i]->p, h->ref_of.as<int32_t>(), n, ref + (4 + i) * rows, h->stream));
+  // each run of fields that are asked for as one copy
+  const double* src = ref;
+  for (int i = 0; i < 5;) {
+    int k = i;
+    size_t bytes = 0;
+    for (; k < 5 && out[k].dst; k++) bytes += out[k].bytes;
+    LBM_CUDA_TRY(d2h_staged(out + i, k - i, src, h->stream));
+    if (k < 5) bytes += out[k].bytes;
+    src += bytes / sizeof(double);
+    i = k + 1;
   }
   LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
   return LBM_OK;

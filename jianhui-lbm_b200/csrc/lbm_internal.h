@@ -194,7 +194,16 @@ struct PinnedStage {
 // Copies `bytes` from device memory `src` to host memory `dst` in order on
 // `st` (a stream of the current device) and returns when the host copy is
 // complete.
-cudaError_t d2h_staged(void* dst, const void* src, size_t bytes, cudaStream_t st);
+struct HostPart {
+  void* dst;
+  size_t bytes;
+};
+// (several destinations: their sources follow one another at src)
+cudaError_t d2h_staged(const HostPart* parts, int nparts, const void* src, cudaStream_t st);
+inline cudaError_t d2h_staged(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  const HostPart one{dst, bytes};
+  return d2h_staged(&one, 1, src, st);
+}
 // Pins one stage for the current device if its pool has none yet (so that
 // the process's first field read does not pay for it).
 cudaError_t stage_pool_prime();

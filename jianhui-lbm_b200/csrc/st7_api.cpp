@@ -38,7 +38,7 @@ struct lbm_st7_handle {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   Geometry geo;
-  DevBuf g, table, rows, u, c0, ref_of, x_conc;
+  DevBuf g, table, rows, u, c0, ref_of;
   int cur = kPull;  // phase of g
   // captured step chains, one per starting phase, and the steps launched one
   // by one that each would have covered
@@ -309,9 +309,9 @@ lbm_status lbm_st7_get_concentration(lbm_st7_handle* h, double* c) {
   if (!h || !c) return fail(LBM_ERR_ARG, "lbm_st7_get_concentration: bad argument");
   LBM_CUDA_TRY(cudaSetDevice(h->device));
   const int n = h->geo.count;
-  const size_t need = sizeof(double) * ((size_t)h->geo.npad + n + 1);
-  if (h->x_conc.bytes != need) LBM_CUDA_TRY(h->x_conc.alloc(need));  // kept between calls
-  double* inner = static_cast<double*>(h->x_conc.p);
+  DevBuf buf;  // C in internal order, then in the reference's
+  LBM_CUDA_TRY(buf.alloc(sizeof(double) * ((size_t)h->geo.npad + n + 1)));
+  double* inner = buf.as<double>();
   double* ref = inner + h->geo.npad;
   LBM_CUDA_TRY(st7_launch_conc(h->f64, st7_args(h, h->given), inner, h->stream));
   LBM_CUDA_TRY(launch_export_scalar(true, inner, static_cast<const int32_t*>(h->ref_of.p), n, ref, h->stream));

@@ -101,20 +101,28 @@ cudaError_t stage_pool_prime() {
 // chunk i runs while the host copies chunk i-1 out of the other buffer, so
 // the transfer takes about the longer of the two instead of a pageable copy
 // (which the driver stages through a small bounce buffer, chunk by chunk,
-// without overlap).
-cudaError_t d2h_staged(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+// without overlap).  Several destinations are one copy, so that the fields of a
+// read fill the chunks together: the five of a two-phase read at 0.5 M nodes,
+// 4 to 13 MB each, took 5.0 to 6.5 ms one after the other.
+cudaError_t d2h_staged(const HostPart* parts, int nparts, const void* src, cudaStream_t st) {
+  std::vector<host_copy::Piece> pieces;
+  size_t bytes = 0;
+  for (int i = 0; i < nparts; i++) {
+    if (parts[i].bytes == 0) continue;
+    pieces.push_back({static_cast<char*>(parts[i].dst), parts[i].bytes});
+    bytes += parts[i].bytes;
+  }
   if (bytes == 0) return cudaSuccess;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  advise_huge(dst, bytes);
+  for (const auto& p : pieces) advise_huge(p.dst, p.bytes);
   PinnedStage* sp = borrow_stage(dev);
   PinnedStage& s = *sp;
   e = fill_stage(s);
   const size_t n = (bytes + PinnedStage::kChunk - 1) / PinnedStage::kChunk;
   auto len = [&](size_t i) { return i + 1 < n ? PinnedStage::kChunk : bytes - i * PinnedStage::kChunk; };
   const char* s8 = static_cast<const char*>(src);
-  char* d8 = static_cast<char*>(dst);
   for (size_t i = 0; i <= n && e == cudaSuccess; i++) {
     if (i < n) {
       // buffer i&1 was emptied by the host copy of chunk i-2 (previous iteration)
@@ -126,7 +134,7 @@ cudaError_t d2h_staged(void* dst, const void* src, size_t bytes, cudaStream_t st
       const size_t j = i - 1;
       e = cudaEventSynchronize(s.ev[j & 1]);
       if (e != cudaSuccess) break;
-      host_copy::copy_parallel(d8 + j * PinnedStage::kChunk, static_cast<const char*>(s.buf[j & 1]), len(j));
+      host_copy::copy_parallel(pieces.data(), j * PinnedStage::kChunk, len(j), static_cast<const char*>(s.buf[j & 1]));
     }
   }
   // no DMA into the stage may be in flight when another copy borrows it

@@ -128,6 +128,22 @@ static void retry(const char* name, size_t nvalues, Create create, Read read, De
   check(failures > 0, "the read allocates");
 }
 
+// Every subset of the five two-phase fields is the plain read's values.
+static void subsets(lbm_cg_handle* h, size_t r) {
+  std::vector<double> all(7 * r);
+  const size_t at[5] = {0, r, 4 * r, 5 * r, 6 * r}, len[5] = {r, 3 * r, r, r, r};
+  check(lbm_cg_get_fields(h, &all[0], &all[r], &all[4 * r], &all[5 * r], &all[6 * r]) == LBM_OK, "all fields");
+  for (int m = 0; m < 32; m++) {
+    std::vector<double> v(7 * r, -1.0);
+    double* p[5];
+    for (int i = 0; i < 5; i++) p[i] = (m >> i & 1) ? &v[at[i]] : nullptr;
+    check(lbm_cg_get_fields(h, p[0], p[1], p[2], p[3], p[4]) == LBM_OK, "some fields");
+    for (int i = 0; i < 5; i++)
+      for (size_t k = 0; k < len[i]; k++)
+        check(v[at[i] + k] == ((m >> i & 1) ? all[at[i] + k] : -1.0), "values of some fields");
+  }
+}
+
 int main() {
   const int nx = 9, ny = 7, nz = 6;
   std::vector<uint8_t> mask(nx * ny * nz, 0);
@@ -157,6 +173,18 @@ int main() {
           return lbm_cg_get_fields(h, v, v + r, v + 4 * r, v + 5 * r, v + 6 * r);
         },
         lbm_cg_destroy);
+    {
+      lbm_cg_params p{};
+      p.nu_l = p.nu_g = 0.1;
+      p.psi_solid = 0.7;
+      p.cap_a = 1e-3;
+      p.perdir = 1;
+      p.precision = precision;
+      lbm_cg_handle* h = nullptr;
+      check(lbm_cg_create(&p, mask.data(), psi.data(), nx, ny, nz, &h) == LBM_OK, "lbm_cg_create");
+      subsets(h, r);
+      lbm_cg_destroy(h);
+    }
     for (int lattice : {7, 19})
       retry(
           "solute concentration", r,
