@@ -731,7 +731,7 @@ lbm_status lbm_create(const lbm_params* p, const uint8_t* mask, int nx, int ny, 
   }
   if ((st = init_state(h.get())) != LBM_OK) return st;
   // the process's staging memory for field reads (pinned once per device)
-  LBM_CUDA_TRY(stage_pool_prime());
+  stage_pool_prime();
   LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
   *out = h.release();
   if (p->ordering == LBM_ORDER_AUTO) {

@@ -176,7 +176,7 @@ struct Pool {
     LBM_CUDA_TRY(cudaMemcpyAsync(state.p, h_state, (size_t)nslots * sizeof(InstState), cudaMemcpyHostToDevice,
                                  stream));
     grid = batch_step_grid(ntiles, block);
-    LBM_CUDA_TRY(stage_pool_prime());  // the process's staging memory for field reads
+    stage_pool_prime();  // the process's staging memory for field reads
     return LBM_OK;
   }
 

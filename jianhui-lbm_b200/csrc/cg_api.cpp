@@ -519,7 +519,7 @@ lbm_status lbm_cg_create_bc(const lbm_cg_params* p, const lbm_boundary* bc, cons
     LBM_CUDA_TRY(cudaMemcpyAsync(h->rho_b.p, c.data(), sizeof(float) * npad, cudaMemcpyHostToDevice, h->stream));
     LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
   }
-  LBM_CUDA_TRY(stage_pool_prime());  // the process's staging memory for field reads
+  stage_pool_prime();  // the process's staging memory for field reads
   if (h->gr.p) LBM_CUDA_TRY(cudaMemsetAsync(h->gr.p, 0, h->gr.bytes, h->stream));
   if (h->gb.p) LBM_CUDA_TRY(cudaMemsetAsync(h->gb.p, 0, h->gb.bytes, h->stream));
   if (h->rec.p) LBM_CUDA_TRY(cudaMemsetAsync(h->rec.p, 0, h->rec.bytes, h->stream));

@@ -205,8 +205,9 @@ inline cudaError_t d2h_staged(void* dst, const void* src, size_t bytes, cudaStre
   return d2h_staged(&one, 1, src, st);
 }
 // Pins one stage for the current device if its pool has none yet (so that
-// the process's first field read does not pay for it).
-cudaError_t stage_pool_prime();
+// the process's first field read does not pay for it).  Where no memory can be
+// pinned the reads go without.
+void stage_pool_prime();
 
 // Device memory of the solvers, from the current device's default memory
 // pool with its release threshold raised: what a destroyed solver frees

@@ -202,7 +202,7 @@ lbm_status create_solute(const lbm_st7_params* p, const uint8_t* mask, int nx, i
   LBM_CUDA_TRY(cudaMemsetAsync(h->g.p, 0, h->g.bytes, h->stream));
   const St7Args a = st7_args(h.get(), true);  // the initial state is the pre-image of the first pull
   LBM_CUDA_TRY(st7_launch_init(h->f64, a, h->stream));
-  LBM_CUDA_TRY(stage_pool_prime());  // the process's staging memory for field reads
+  stage_pool_prime();  // the process's staging memory for field reads
   LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
   *out = h.release();
   return LBM_OK;

@@ -83,18 +83,16 @@ void advise_huge(void* dst, size_t bytes) {
 
 }  // namespace
 
-cudaError_t stage_pool_prime() {
+void stage_pool_prime() {
   int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
   {
     std::lock_guard<std::mutex> lk(g_stage_mu);
-    if (!free_stages()[dev].empty()) return cudaSuccess;
+    if (!free_stages()[dev].empty()) return;
   }
   PinnedStage* s = new PinnedStage();
-  e = fill_stage(*s);
+  if (fill_stage(*s) != cudaSuccess) cudaGetLastError();
   return_stage(dev, s);  // kept even when incomplete: the next copy retries
-  return e;
 }
 
 // Chunks of kChunk bytes alternate between two pinned buffers: the DMA of
@@ -119,10 +117,21 @@ cudaError_t d2h_staged(const HostPart* parts, int nparts, const void* src, cudaS
   for (const auto& p : pieces) advise_huge(p.dst, p.bytes);
   PinnedStage* sp = borrow_stage(dev);
   PinnedStage& s = *sp;
-  e = fill_stage(s);
+  const char* s8 = static_cast<const char*>(src);
+  if (fill_stage(s) != cudaSuccess) {
+    // no host memory to pin (a limit on locked memory): the driver's own staging
+    cudaGetLastError();
+    return_stage(dev, sp);
+    for (const auto& p : pieces) {
+      e = cudaMemcpyAsync(p.dst, s8, p.bytes, cudaMemcpyDeviceToHost, st);
+      if (e != cudaSuccess) break;
+      s8 += p.bytes;
+    }
+    const cudaError_t done = cudaStreamSynchronize(st);
+    return e != cudaSuccess ? e : done;
+  }
   const size_t n = (bytes + PinnedStage::kChunk - 1) / PinnedStage::kChunk;
   auto len = [&](size_t i) { return i + 1 < n ? PinnedStage::kChunk : bytes - i * PinnedStage::kChunk; };
-  const char* s8 = static_cast<const char*>(src);
   for (size_t i = 0; i <= n && e == cudaSuccess; i++) {
     if (i < n) {
       // buffer i&1 was emptied by the host copy of chunk i-2 (previous iteration)

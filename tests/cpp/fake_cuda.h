@@ -15,6 +15,7 @@
 static std::map<const char*, size_t> g_live;
 [[maybe_unused]] static bool g_capturing = false;
 [[maybe_unused]] static int g_captures = 0, g_replays = 0;
+[[maybe_unused]] static bool g_fail_pin = false;  // no MB of host memory can be pinned
 static int g_fail_in = 0;  // 1: the next device allocation fails
 static cudaError_t g_last = cudaSuccess;
 
@@ -48,6 +49,7 @@ cudaError_t cudaFreeAsync(void* p, cudaStream_t) {
   return cudaSuccess;
 }
 cudaError_t cudaMallocHost(void** p, size_t n) {
+  if (g_fail_pin && n >= size_t(1) << 20) return g_last = cudaErrorMemoryAllocation;
   *p = std::calloc(n, 1);
   return cudaSuccess;
 }

@@ -144,7 +144,8 @@ static void subsets(lbm_cg_handle* h, size_t r) {
   }
 }
 
-int main() {
+int main(int argc, char** argv) {
+  g_fail_pin = argc > 1 && !std::strcmp(argv[1], "nopin");
   const int nx = 9, ny = 7, nz = 6;
   std::vector<uint8_t> mask(nx * ny * nz, 0);
   std::vector<double> psi(mask.size());
