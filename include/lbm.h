@@ -286,7 +286,8 @@ LBM_API lbm_status lbm_autotune(lbm_handle* h, int trial_steps, int* ordering_ou
 /* Kernel timing of the last lbm_step call (CUDA events on the handle's stream). */
 LBM_API lbm_status lbm_last_step_ms(lbm_handle* h, double* ms);
 
-/* Memory facts: bytes of device memory the handle holds and the algorithmic
+/* Memory facts: bytes of device memory the handle holds (64 per node more from
+ * the first lbm_get_fields on, whose buffers it keeps) and the algorithmic
  * bytes one fluid-node update moves on average (2*19*s populations + half
  * the table bytes per node that the step reads: every second step reads no
  * table). */

@@ -983,7 +983,8 @@ lbm_status lbm_memory(lbm_handle* h, size_t* device_bytes, double* bytes_per_lu)
     size_t b = 0;
     for (const DevBuf* d : {&h->pop, &h->table, &h->ref_of, &h->window, &h->rho_given, &h->u_given,
                             &h->rho_prev, &h->u_prev, &h->partials, &h->result, &h->snap[0], &h->snap[1],
-                            &h->bc_ops, &h->bc_off, &h->bc_mi, &h->bnd_f, &h->ct_base, &h->ct_off, &h->rows})
+                            &h->bc_ops, &h->bc_off, &h->bc_mi, &h->bnd_f, &h->ct_base, &h->ct_off, &h->rows,
+                            &h->x_rint, &h->x_uint, &h->x_rref, &h->x_uref})
       b += d->bytes;
     *device_bytes = b;
   }

@@ -74,3 +74,12 @@ def test_where_the_row_form_is_read(precision, ordering, shape, rows):
     with L.SinglePhase(mask, 0.1, (1e-6, 0.0, 0.0), precision=precision, ordering=ordering) as s:
         per_step = s.memory()["bytes_per_lu"] - 38 * {"f16": 2, "f32": 4}.get(precision, 8)
         assert per_step == 36 if not rows else 18 <= per_step < 19
+
+
+def test_memory_counts_what_a_field_read_keeps():
+    mask = spheres((33, 21, 18), 0.55, 3.0, seed=9)
+    with L.SinglePhase(mask, 0.1, (1e-6, 0.0, 0.0)) as s:
+        before = s.memory()["device_bytes"]
+        s.fields()
+        npad, rows = -(-s.count // 256) * 256, s.count + 1
+        assert s.memory()["device_bytes"] - before == 8 * 4 * (npad + rows)
