@@ -2,8 +2,9 @@
 //
 // Blackwell's packed FP32 instructions (add / mul / fma .rn.f32x2) do two
 // independent FP32 operations per issued instruction.  The step is bound by
-// issue slots as soon as its bytes come from L2 (about 490 instructions per
-// node, 69 % of the issue slots at 256^3, 75 % with 16-bit storage), so a
+// issue slots as soon as its bytes come from L2 (one node per thread: 665
+// instructions per node through the table and 540 on its own slots, 69 % of the
+// issue slots at 256^3, 75 % with 16-bit storage), so a
 // thread works on two neighbouring nodes, one per half of each pair.
 //
 // The operator is mrt_collide_dev's (kernels_common.cuh).  Every operation

@@ -59,7 +59,7 @@ struct Traits<Store::F16> {
   static constexpr bool kDev = true;
 };
 
-// Programmatic dependent launch between the steps of a chain.  A step lets
+// Programmatic dependent launch between steps that follow one another.  A step lets
 // the next one launch as soon as its own blocks run (step_begin); the next
 // reads what no step writes, the table, and waits for the previous step's end
 // before it touches populations (step_wait).  A kernel that was launched

@@ -405,8 +405,9 @@ __device__ __forceinline__ void macro_in_out(const StepArgs& a, int p, bool give
   }
 }
 
-// Resident blocks per SM asked of the register allocator: 16 warps (128
-// registers, no spills).
+// Resident blocks per SM asked of the register allocator: 16 warps, 128
+// registers.  No spills on the default lattice but 40 bytes in the given state
+// of a general force; 128 to 160 bytes on a self-defined lattice.
 constexpr int f64_min_blocks(int bs) { return 512 / bs; }
 
 // One node per thread.  The macro step of the reference (comput_macro_variables,

@@ -194,7 +194,8 @@ __global__ void __launch_bounds__(BS, BS == 256 ? 2 : 1) step_dev_kernel(StepArg
 }
 
 // Resident blocks per SM asked of the register allocator: one node per
-// thread fits 1280 threads (48 registers), two nodes 640 (96 registers; 512
+// thread fits 1280 threads (48 registers; given states and the compact table
+// spill 4 to 88 bytes), two nodes 640 (96 registers; 512
 // threads and 128 registers: 19.6 against 18.4 us at 128^3; 768 threads spill
 // 150-230 bytes: 22.9 us).
 template <typename V>
