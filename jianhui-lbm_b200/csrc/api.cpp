@@ -446,7 +446,10 @@ lbm_status finalize_faces(lbm_handle* h, int* n_main, const double** bnd_f) {
 }
 
 // With faces the steps are joined by events.
-bool chained_steps(const lbm_handle* h) { return !h->bc.active && chain_pays(h->kind, h->geo.count); }
+bool chained_steps(const lbm_handle* h) {
+  const int n = h->geo.count;
+  return !h->bc.active && chain_pays(h->kind, n, h->block ? h->block : default_block(h->kind, n));
+}
 
 // follows: launched right after another step.
 lbm_status one_step(lbm_handle* h, bool write, bool follows) {

@@ -321,12 +321,12 @@ __global__ void batch_init_kernel(typename Traits<K>::T* __restrict__ pop, int p
 template <Store K, int BS>
 static cudaError_t step_bs(const BatchStepArgs& a, int grid, int chain_step, cudaStream_t st) {
   // The chain's first step follows the list kernels, the others are dependents
-  // (launch_with) by the grid, a power of two of tiles.  us per FP32 step,
-  // chained | not: 13 K nodes (grid 32) 3.78 | 4.11, 26 K (64) 4.31 | 4.12, 52 K
-  // (128) 4.57 | 4.25, in one pass 70 K (256) 4.49 | 4.48 and 105 K (256) 4.85 |
-  // 5.50, 137 K (512) 8.79 | 6.07, 205 K (512) 9.10 | 7.20, 273 K (1024) 9.43 |
-  // 8.68, 376 K (1024) 9.75 | 10.3, 562 K (2048) 14.5 | 14.8, 2.8 M 94.0 | 95.6.
-  const bool chained = chain_step > 0 && (grid <= 32 || grid >= 1024 || (grid == 256 && BS == 256));
+  // (launch_with) by the grid: a power of two of tiles, or all the pool's.  us
+  // per FP32 step, chained | not: 13 K nodes (26 tiles) 3.78 | 4.11, 26 K (52) 4.31 |
+  // 4.12, 44 K (87) 4.46 | 4.21, in one pass 86 K (169) 5.10 | 5.38, 115 K (225) 4.99 |
+  // 5.59, 137 K (268) 8.79 | 6.07, 205 K (400) 9.10 | 7.20, 273 K (533) 9.43 | 8.68, 311
+  // K (609) 9.65 | 9.90, 376 K (736) 9.75 | 10.3, 562 K 14.5 | 14.8, 2.8 M 94.0 | 95.6.
+  const bool chained = chain_step > 0 && (grid <= 32 || grid >= 600 || (grid > 128 && grid <= 256 && BS == 256));
   if (a.phase == kLocal) return launch_chained(batch_step_kernel<K, BS, true>, grid, BS, st, chained, a, chain_step);
   return launch_chained(batch_step_kernel<K, BS, false>, grid, BS, st, chained, a, chain_step);
 }

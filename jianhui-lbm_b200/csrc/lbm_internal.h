@@ -397,9 +397,10 @@ constexpr int prefetch_ahead(long long n, long long pop_bytes, long long table_b
 //         8.79 | 7.62, 66 K 8.95 | 8.78, 71 K 8.46 | 9.15, 126 K 13.2 | 13.8, 734 K
 //         65.8 | 67.6
 // FP64 deviation storage gains 2 to 20 % and loses up to 3 % about 20 K; the
-// solutes (st7_api.cpp) gain at every size.
-constexpr bool chain_pays(Store kind, long long n) {
-  return kind == Store::F64D ||
+// solutes (st7_api.cpp) gain at every size.  Larger blocks that were asked for
+// gain nearly everywhere (256 nodes, FP64 39 K 8.40 | 8.65, FP32 92 K 3.92 | 4.31).
+constexpr bool chain_pays(Store kind, long long n, int block) {
+  return kind == Store::F64D || block >= 256 ||
          (kind == Store::F64 ? n <= 148 * 128 || n >= 148 * 480 : n <= 148 * 256 || n >= 148 * 1024);
 }
 
