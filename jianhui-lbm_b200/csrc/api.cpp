@@ -127,7 +127,7 @@ struct lbm_handle {
   DevBuf rows;
   int marked = 0;
   // field export: device buffers kept between calls
-  DevBuf x_rint, x_uint, x_rref, x_uref;
+  DevBuf x_rint, x_uint, x_ref;
   // phase of the populations (kPull / kLocal); with faces also the record of
   // the state, snap[cur]
   int cur = kPull;
@@ -888,21 +888,23 @@ lbm_status lbm_get_fields(lbm_handle* h, double* rho, double* u) {
   lbm_status st = check_handle(h);
   if (st != LBM_OK) return st;
   const int n = h->geo.count, npad = h->geo.npad;
-  DevBuf &rint = h->x_rint, &uint_ = h->x_uint, &rref = h->x_rref, &uref = h->x_uref;
+  const size_t rows = (size_t)n + 1;
+  DevBuf &rint = h->x_rint, &uint_ = h->x_uint, &ref = h->x_ref;
   if (!rint.p) LBM_CUDA_TRY(rint.alloc((size_t)npad * sizeof(double)));
   if (!uint_.p) LBM_CUDA_TRY(uint_.alloc((size_t)3 * npad * sizeof(double)));
-  if (!rref.p) LBM_CUDA_TRY(rref.alloc((size_t)(n + 1) * sizeof(double)));
-  if (!uref.p) LBM_CUDA_TRY(uref.alloc((size_t)(n + 1) * 3 * sizeof(double)));
+  if (!ref.p) LBM_CUDA_TRY(ref.alloc(4 * rows * sizeof(double)));
+  double* rref = ref.as<double>();
+  double* uref = rref + rows;
   double r[8];
   const double pp[3] = {h->perm_prev[0], h->perm_prev[1], h->perm_prev[2]};
   if ((st = reduce_raw(h, r, rint.as<double>(), uint_.as<double>())) != LBM_OK) return st;
   for (int i = 0; i < 3; i++) h->perm_prev[i] = pp[i];
-  LBM_CUDA_TRY(cudaMemsetAsync(rref.p, 0, rref.bytes, h->stream));
-  LBM_CUDA_TRY(cudaMemsetAsync(uref.p, 0, uref.bytes, h->stream));
-  LBM_CUDA_TRY(launch_export_macro(rint.as<double>(), uint_.as<double>(), h->ref_of.as<int32_t>(), n, npad,
-                                   rref.as<double>(), uref.as<double>(), h->stream));
-  if (rho) LBM_CUDA_TRY(d2h_staged(rho, rref.p, rref.bytes, h->stream));
-  if (u) LBM_CUDA_TRY(d2h_staged(u, uref.p, uref.bytes, h->stream));
+  LBM_CUDA_TRY(cudaMemsetAsync(ref.p, 0, ref.bytes, h->stream));
+  LBM_CUDA_TRY(launch_export_macro(rint.as<double>(), uint_.as<double>(), h->ref_of.as<int32_t>(), n, npad, rref, uref,
+                                   h->stream));
+  const HostPart out[2] = {{rho, rows * sizeof(double)}, {u, 3 * rows * sizeof(double)}};
+  if (rho) LBM_CUDA_TRY(d2h_staged(out, u ? 2 : 1, rref, h->stream));
+  if (!rho && u) LBM_CUDA_TRY(d2h_staged(out + 1, 1, uref, h->stream));
   LBM_CUDA_TRY(cudaStreamSynchronize(h->stream));
   return LBM_OK;
 }
@@ -987,7 +989,7 @@ lbm_status lbm_memory(lbm_handle* h, size_t* device_bytes, double* bytes_per_lu)
     for (const DevBuf* d : {&h->pop, &h->table, &h->ref_of, &h->window, &h->rho_given, &h->u_given,
                             &h->rho_prev, &h->u_prev, &h->partials, &h->result, &h->snap[0], &h->snap[1],
                             &h->bc_ops, &h->bc_off, &h->bc_mi, &h->bnd_f, &h->ct_base, &h->ct_off, &h->rows,
-                            &h->x_rint, &h->x_uint, &h->x_rref, &h->x_uref})
+                            &h->x_rint, &h->x_uint, &h->x_ref})
       b += d->bytes;
     *device_bytes = b;
   }

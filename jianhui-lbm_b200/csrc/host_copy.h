@@ -110,12 +110,12 @@ inline void copy_range(const Piece* pieces, size_t off, size_t len, const char* 
 
 // copy_range out of the staging buffer split over up to 16 threads: one
 // thread writes fresh pageable memory (page faults, the kernel zeroing each
-// page) at well under the DMA's rate.  A thread per MB for full chunks, per 2 MB
-// below: where the pages are there already or few, more threads wait for each
+// page) at well under the DMA's rate.  A thread per MB in copies of a full
+// chunk or more, per 2 MB below: where the pages are there already or few, more threads wait for each
 // other (a two-phase read of 15 MB into pages used before 1.8 ms with 2 MB | 2.2
 // with 1, into fresh pages 1.9 | 1.9; 3.9 MB 0.54 | 1.1).
-inline void copy_parallel(const Piece* pieces, size_t off, size_t bytes, const char* src) {
-  const size_t min_split = size_t(bytes < (size_t(16) << 20) ? 2 : 1) << 20;
+inline void copy_parallel(const Piece* pieces, size_t off, size_t bytes, const char* src, bool long_copy) {
+  const size_t min_split = size_t(long_copy ? 1 : 2) << 20;
   const int nt = (int)std::min<size_t>((size_t)copy_threads(), std::max<size_t>(1, bytes / min_split));
   if (nt == 1) {
     copy_range(pieces, off, bytes, src);
@@ -130,7 +130,7 @@ inline void copy_parallel(const Piece* pieces, size_t off, size_t bytes, const c
 }
 inline void copy_parallel(char* dst, const char* src, size_t bytes) {
   const Piece one{dst, bytes};
-  copy_parallel(&one, 0, bytes, src);
+  copy_parallel(&one, 0, bytes, src, bytes >= size_t(16) << 20);
 }
 
 }  // namespace host_copy

@@ -143,7 +143,8 @@ cudaError_t d2h_staged(const HostPart* parts, int nparts, const void* src, cudaS
       const size_t j = i - 1;
       e = cudaEventSynchronize(s.ev[j & 1]);
       if (e != cudaSuccess) break;
-      host_copy::copy_parallel(pieces.data(), j * PinnedStage::kChunk, len(j), static_cast<const char*>(s.buf[j & 1]));
+      host_copy::copy_parallel(pieces.data(), j * PinnedStage::kChunk, len(j), static_cast<const char*>(s.buf[j & 1]),
+                               bytes >= PinnedStage::kChunk);
     }
   }
   // no DMA into the stage may be in flight when another copy borrows it

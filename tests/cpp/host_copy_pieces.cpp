@@ -26,7 +26,7 @@ int main() {
     for (size_t i = 0; i < total; i++) src[i] = (char)(i * 131 + round + 1);
     const size_t chunk = 1 + rng() % (total + 1);
     for (size_t o = 0; o < total; o += chunk)
-      lbm::host_copy::copy_parallel(pieces.data(), o, std::min(chunk, total - o), src.data() + o);
+      lbm::host_copy::copy_parallel(pieces.data(), o, std::min(chunk, total - o), src.data() + o, round % 2);
     size_t at = 0;
     for (int i = 0; i < n; i++) {
       for (size_t b = 0; b < pieces[i].bytes; b++) bad += dst[i][b] != src[at + b];
