@@ -415,10 +415,11 @@ cudaError_t launch_full_step(lbm_handle* h, StepArgs& a, int c) {
   if (!h->bc.active) return launch_step(h->kind, a, block, h->stream);
   // One split of L1 and shared memory for the steps of both phases and the
   // face kernel of small solves: left to the driver, an SM that a block of one
-  // of them runs on takes no block of another.  us per step, without | with
-  // it: FP64 44^3 20.4 | 19.3, 56^3 22.4 | 20.5, FP32 44^3 4.1 | 3.8, 56^3
-  // 5.0 | 4.6 (128^3 25.0 | 26.0: not there).
-  if (a.n_main < 148 * 1024) a.carveout = 50;
+  // of them runs on takes no block of another.  us per step, driver's choice |
+  // 50 % | 70 %: FP64 44^3 20.4 | 18.4 | 18.5, 64^3 (105 K nodes) 23.5 | 22.5 | 20.6, 72^3
+  // (149 K) 25.4 | 24.7 | 25.1, FP32 44^3 4.1 | 3.8 | 3.8, 64^3 5.8 | 5.7 | 5.5, 72^3 6.6 |
+  // 6.7 | 6.8, 128^3 25.0 | 26.0.
+  if (a.n_main < 148 * 1024) a.carveout = a.n_main < 148 * 900 ? 70 : 50;
   cudaError_t e = cudaEventRecord(h->ev_fork, h->stream);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side, h->ev_fork, 0);
   if (e == cudaSuccess) e = launch_boundary(h->kind, bc_args(h, a, c), h->side);
