@@ -330,7 +330,7 @@ struct StepArgs {
 //
 // Beside a face kernel (faces) the FP64 step's smaller blocks would spread over
 // the face kernel's SMs as well: 256 | 128 | 64, FP64 with pressure faces, 70 K
-// nodes 19.0 | 19.2 | 20.4, 105 K 22.5 | 23.4 | 23.4, 149 K 25.4 | 24.4 | 24.6,
+// nodes 19.0 | 19.2 | 20.4, 105 K 20.7 | 21.7 | 22.3, 149 K 25.4 | 24.4 | 24.6,
 // 354 K 49.9 | 46.6 | 48.4; FP32 (256 | 128 | 64) 34 K 4.0 | 3.9 | 3.85, 105 K
 // 5.7 | 5.6 | 5.9, 149 K 6.8 | 6.7 | 6.9.
 constexpr int default_block(Store kind, long long n, bool faces = false) {

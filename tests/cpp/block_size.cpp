@@ -62,8 +62,11 @@ cudaError_t launch_batch_step(Store, const BatchStepArgs&, int block, int, int, 
   g_blocks.push_back(block);
   return last();
 }
+// captured once per chain graph: ends all solves but the first g_keep
+static int g_keep = 0;
 cudaError_t launch_batch_check(Store, const BatchReduceArgs& a, int, double, long long, cudaStream_t) {
-  for (int i = 0; i < a.nslots; i++) a.state[i].active = 0, a.state[i].done = 1;  // captured: every chain ends the run
+  for (int i = g_keep; i < a.nslots; i++) a.state[i].active = 0, a.state[i].done = 1;
+  g_keep = 0;
   return last();
 }
 }  // namespace lbm
@@ -134,6 +137,16 @@ int main() {
         g_blocks.clear();
         check(lbm_batch_run(b, 1e-6, 10, 1000, nullptr) == LBM_OK, "lbm_batch_run");
         for (int s : g_blocks) check(s == best, "pool block after autotuning", best, s);
+        if (count == 8) {  // 568 tiles, then the 71 of the solve that is left
+          check(best == 128, "equal times: the first size", best);
+          check(lbm_batch_autotune(b, 4, &order, &best, &ml) == LBM_OK, "lbm_batch_autotune");
+          g_blocks.clear();
+          g_keep = 1;
+          check(lbm_batch_run(b, 1e-6, 10, 1000, nullptr) == LBM_OK, "lbm_batch_run");
+          check(g_blocks.size() == 20, "two chains", g_blocks.size());
+          for (size_t i = 0; i < g_blocks.size(); i++)
+            check(g_blocks[i] == (i < 10 ? best : 512), "tuned block as solves stop", i, g_blocks[i]);
+        }
       }
       lbm_batch_destroy(b);
     }
