@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(BS, 640 / BS) batch_step_kernel(BatchStepArgs 
     } else {
       macro_vec<F2>(f, 0.5f * w.g[0], 0.5f * w.g[1], 0.5f * w.g[2], drho, rho, ux, uy, uz);
     }
-    collide_vec<F2>(f, drho, rho, ux, uy, uz, cs);
+    collide_vec<F2, true>(f, drho, rho, ux, uy, uz, cs);
     if constexpr (LOCAL) {
       store_row<K>(pop + p, f[0], scale, both);
 #pragma unroll

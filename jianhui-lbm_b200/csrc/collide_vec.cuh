@@ -210,8 +210,11 @@ __device__ __forceinline__ CollideScalars collide_scalars(float gx, float gy, fl
 }
 
 // MRT collision with Guo forcing of the deviations f, in place; the operator
-// and the closed forms of mrt_collide_dev.
-template <typename V>
+// and the closed forms of mrt_collide_dev.  POOL: the node pool's rounding of
+// moment 2, which keeps the force term's product and fuses the relaxation's;
+// the single-domain steps do it the other way round.  A solve in 16-bit storage
+// stops by noise of this size, so each keeps its own bits.
+template <typename V, bool POOL = false>
 __device__ __forceinline__ void collide_vec(V (&f)[kQ], V drho, V rho, V ux, V uy, V uz, const CollideScalars& c) {
   using O = VecOf<V>;
   auto S = [](float x) { return O::splat(x); };
@@ -251,8 +254,11 @@ __device__ __forceinline__ void collide_vec(V (&f)[kQ], V drho, V rho, V ux, V u
   V a[kQ];
   a[1] = vmul(vfma(S(c.hv38), ug, vmul(nsv, vsub(m[1], vfma(vmul(S(19.f), rho), usq, vmul(S(-11.f), drho))))),
               S(kInvNorm<1>));
-  a[2] = vmul(vfma(S(c.nhv11), ug, vmul(nsv, vsub(m[2], vfma(S(3.f), drho, vmul(vmul(S(-5.5f), rho), usq))))),
-              S(kInvNorm<2>));
+  const V x2 = vsub(m[2], vfma(S(3.f), drho, vmul(vmul(S(-5.5f), rho), usq)));
+  if constexpr (POOL)
+    a[2] = vmul(vfma(nsv, x2, vmul(S(c.nhv11), ug)), S(kInvNorm<2>));
+  else
+    a[2] = vmul(vfma(S(c.nhv11), ug, vmul(nsv, x2)), S(kInvNorm<2>));
   a[3] = S(__fmul_rn(c.gx, kInvNorm<3>));
   a[5] = S(__fmul_rn(c.gy, kInvNorm<5>));
   a[7] = S(__fmul_rn(c.gz, kInvNorm<7>));
