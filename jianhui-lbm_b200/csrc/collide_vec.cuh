@@ -210,9 +210,10 @@ __device__ __forceinline__ CollideScalars collide_scalars(float gx, float gy, fl
 }
 
 // MRT collision with Guo forcing of the deviations f, in place; the operator
-// and the closed forms of mrt_collide_dev.  POOL: the node pool's rounding of
-// moment 2, which keeps the force term's product and fuses the relaxation's;
-// the single-domain steps do it the other way round.  A solve in 16-bit storage
+// and the closed forms of mrt_collide_dev.  POOL: the node pool's rounding, which
+// rounds the force term's product of moment 2 and fuses the relaxation's, and
+// fuses the first product of the cross terms of moments 13 to 15; the
+// single-domain steps do both the other way round.  A solve in 16-bit storage
 // stops by noise of this size, so each keeps its own bits.
 template <typename V, bool POOL = false>
 __device__ __forceinline__ void collide_vec(V (&f)[kQ], V drho, V rho, V ux, V uy, V uz, const CollideScalars& c) {
@@ -250,6 +251,12 @@ __device__ __forceinline__ void collide_vec(V (&f)[kQ], V drho, V rho, V ux, V u
   const V usq = vfma(uz, uz, vfma(ux, ux, vmul(uy, uy)));
   const V ug = vfma(uz, gz, vfma(ux, gx, vmul(uy, gy)));
   const V nsv = S(c.nsv), nso = S(c.nso), hv = S(c.hv);
+  auto cross = [](V x, V y, V px, V py) {  // x py + y px
+    if constexpr (POOL)
+      return vfma(x, py, vmul(y, px));
+    else
+      return vfma(y, px, vmul(x, py));
+  };
   // a_k = [ -S_k (m_k - m_eq,k) + (1 - S_k/2) (M G)_k ] / |row k|^2
   V a[kQ];
   a[1] = vmul(vfma(S(c.hv38), ug, vmul(nsv, vsub(m[1], vfma(vmul(S(19.f), rho), usq, vmul(S(-11.f), drho))))),
@@ -278,9 +285,9 @@ __device__ __forceinline__ void collide_vec(V (&f)[kQ], V drho, V rho, V ux, V u
   const V x11 = vfma(hv, f11, vmul(nsv, vsub(m[11], p11)));  // a_11 |row 11|^2: its product is part of the sums below
   a[12] = vmul(vfma(nsv, vfma(S(0.5f), p11, m[12]), vmul(S(c.nhv5), f11)), S(kInvNorm<12>));
   const V nrx = vmul(rho, nux), nry = vmul(rho, nuy);
-  a[13] = vmul(vfma(hv, vfma(ux, gy, vmul(uy, gx)), vmul(nsv, vfma(nrx, uy, m[13]))), S(kInvNorm<13>));
-  a[14] = vmul(vfma(hv, vfma(uy, gz, vmul(uz, gy)), vmul(nsv, vfma(nry, uz, m[14]))), S(kInvNorm<14>));
-  a[15] = vmul(vfma(hv, vfma(ux, gz, vmul(uz, gx)), vmul(nsv, vfma(nrx, uz, m[15]))), S(kInvNorm<15>));
+  a[13] = vmul(vfma(hv, cross(ux, uy, gx, gy), vmul(nsv, vfma(nrx, uy, m[13]))), S(kInvNorm<13>));
+  a[14] = vmul(vfma(hv, cross(uy, uz, gy, gz), vmul(nsv, vfma(nry, uz, m[14]))), S(kInvNorm<14>));
+  a[15] = vmul(vfma(hv, cross(ux, uz, gx, gz), vmul(nsv, vfma(nrx, uz, m[15]))), S(kInvNorm<15>));
   a[16] = vmul(vmul(nso, m[16]), S(kInvNorm<16>));
   a[17] = vmul(vmul(nso, m[17]), S(kInvNorm<17>));
   a[18] = vmul(vmul(nso, m[18]), S(kInvNorm<18>));
